@@ -506,3 +506,51 @@ def test_six_slice_lanes_bitwise(shape, na, absn, vz):
         p.set_tuning({"backward_vz": 0, "backward_table": 1})  # automatic: six / five slices per lane
         assert torch.equal(p.backward_ref(dev(b)), computed)
     assert p.status() == 0
+
+
+@pytest.mark.parametrize("n,nz", [(5, 9), (12, 16), (17, 5), (24, 64), (33, 17), (31, 65), (20, 128), (21, 130),
+                                  (26, 132), (16, 256), (15, 261), (41, 12), (64, 33)])
+@pytest.mark.parametrize("absn", [None, "mask", "ray"])
+def test_forward_strips_at_their_edges(n, nz, absn):
+    """The strip forward against the oracle and the generic kernel: strips past the last detector bin, slice
+    counts around the lanes of one chunk (float4 rows and single slices), paired and unpaired angles, rays along
+    rows, columns and diagonals.  A strip sums batches of at most 32 pixels and then the batches, at most
+    32 + 2.3 n / 25 additions of 2^-24 each: 2.3e-6 at the sizes here.  An infinity and a NaN reach exactly the
+    bins that sample their pixels."""
+    rng = np.random.default_rng(n * nz)
+    ang = np.array([0.0, 30.0, 45.0, 62.5, 90.0, 133.3, 180.0, 210.0, 242.5, 270.0, 301.0])
+    x = rng.uniform(-0.2, 1, (n, n, nz))
+    p = plan_for(x.shape, ang)
+    oabs = None
+    if absn == "mask":
+        m = rng.uniform(0.2, 1.0, (n, n))
+        p.set_absorption("mask", mask=m)
+        oabs = ("mask", m)
+    elif absn == "ray":
+        p.set_absorption("ray", alpha_per_px=0.03, radius_px=n / 2 - 1.5)
+        oabs = ("ray", 0.03, n / 2 - 1.5)
+    ref = O.parallel_forward(x, ang, absorption=oabs)
+    got = p.forward(dev(x)).cpu().numpy()
+    assert np.abs(got - ref).max() <= 2.3e-6 * O.parallel_forward(np.abs(x), ang, absorption=oabs).max()
+    if n < 8:
+        return
+    xi = x.copy()
+    xi[n // 2, n // 3, nz // 2], xi[n // 3, n // 2, 0] = np.inf, np.nan
+    skew = np.delete(ang, [0, 4, 6, 9])  # (a tap of weight 1e-17 on an axis is read or not by rounding)
+    q = plan_for(x.shape, skew)
+    if absn == "mask":
+        q.set_absorption("mask", mask=m)
+    elif absn == "ray":
+        q.set_absorption("ray", alpha_per_px=0.03, radius_px=n / 2 - 1.5)
+    strip = q.forward(dev(xi)).cpu().numpy()
+    q.set_tuning({"forward_vz": 1})
+    plain = q.forward(dev(xi)).cpu().numpy()
+    # an angle's partner 180 degrees away is sampled from the same lattice, mirrored (the generic kernel forms
+    # its coordinates anew, and a weight of one rounding more or less than zero decides about an infinity)
+    mirror = plain.copy()
+    rows = np.arange(2 * (n // 2) - n + 1, n)
+    for a, b in ((0, 4), (2, 5)) if absn != "ray" else ():  # 30 and 210, 62.5 and 242.5 (unpaired with "ray")
+        mirror[2 * (n // 2) - rows, b] = plain[rows, a]
+    assert np.array_equal(np.isnan(strip), np.isnan(mirror)) and np.array_equal(np.isinf(strip), np.isinf(mirror))
+    ok = np.isfinite(plain) & np.isfinite(mirror)
+    assert not ok.all() and np.abs(strip[ok] - plain[ok]).max() <= 4.6e-6 * np.abs(plain[ok]).max()

@@ -4,7 +4,8 @@
 // 32/LZ lanes along the reduction axis; z is the contiguous axis of both the
 // volume [nY][nX][nZ] and the sinogram [nR][nA][nZ], so a warp's tap loads are
 // 128-bit vectors over consecutive z and coalesce into 512-byte requests):
-//   k_forward      R1, rotate-and-sum with skimage-warp bilinear sampling
+//   k_forward_strip (strip.cuh), k_forward
+//                  R1, rotate-and-sum with skimage-warp bilinear sampling
 //                  (vamtoolbox/projector/Projector3DParallel.py:113-156)
 //   k_backward_ref R2, pixel-driven np.interp backprojection + circle clip
 //                  (Projector3DParallel.py:158-207)
@@ -254,36 +255,6 @@ __global__ void __launch_bounds__(256) k_forward(Args a) {
     k_forward_body<VZ, OCC, ABS>(a, blockIdx.x, blockIdx.y);
 }
 
-// ---------------------------------------------------------------------------
-// R1 forward, fast path: 32 lanes along z (VZ floats each), one lattice row
-// (angle, detector) per warp, angle pairs (a, a+180) sampled from one lattice.
-//
-// The sample points of angle a+180 are those of angle a mirrored through the
-// rotation centre: sample (j', k') of a+180 is lattice point (2C-j', 2C-k') of
-// a (the warp matrices of Projector3DParallel.py:137-143 satisfy this
-// identically), so one pass over a's lattice row gives both rays.  For odd N
-// the k ranges coincide; for even N (2C = N) angle a sums k in [0, N-1] and
-// a+180 sums k in [1, N] on the row j in [0, N]; the shared part k in [1, N-1]
-// is accumulated once and the two end samples are added separately.
-// ---------------------------------------------------------------------------
-struct FastArgs {
-    const float* vol;
-    float* sino;
-    const double4* trig;
-    const int2* tasks;
-    int nY, nX, nZ, nA, C;
-    int RS;          // row stride of the volume in floats (nX * nZ)
-    int zchunks;     // ceil(nZ / (32 * VZ))
-    int even;        // N even
-    float alpha, R;  // RAY absorption (tasks are unpaired then)
-};
-
-template <int VZ>
-struct Acc {
-    float v[VZ];
-};
-
-// One bilinear sample (all taps checked), added with weight f into acc.
 // Lane-interleaved z vectors of the fast kernels: with Q = VZ / 4, lane l of
 // a warp owns slices zbase + 4l + 128q + (0..3), q < Q, so every float4 load
 // of the warp covers 512 contiguous bytes (four 128-byte lines).  p points at
@@ -308,35 +279,6 @@ __device__ __forceinline__ void load_vz(const float* __restrict__ p, float* d, i
     for (int q = 0; q < VZ / 4; ++q) {
         float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
         if (q < qn) t = __ldg(reinterpret_cast<const float4*>(p + 128 * q));
-        d[4 * q] = t.x; d[4 * q + 1] = t.y; d[4 * q + 2] = t.z; d[4 * q + 3] = t.w;
-    }
-}
-
-// load_vz with an L1 evict-last priority: the forward's taps, which neighbouring bins and samples of
-// the CTA read again (1.406 -> 1.373 ms at 256^3 x 360, identical results)
-template <int VZ>
-__device__ __forceinline__ void load_vz_keep(const float* __restrict__ p, float* d, int qn = VZ / 4) {
-    if constexpr (VZ == 6 || VZ == 5) {
-        float4 t;
-        asm("ld.global.nc.L1::evict_last.v4.f32 {%0, %1, %2, %3}, [%4];"
-            : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "l"(p));
-        d[0] = t.x; d[1] = t.y; d[2] = t.z; d[3] = t.w;
-        if constexpr (VZ == 6) {
-            float2 u;
-            asm("ld.global.nc.L1::evict_last.v2.f32 {%0, %1}, [%2];"
-                : "=f"(u.x), "=f"(u.y) : "l"(p + 128 - 2 * (int)(threadIdx.x & 31)));
-            d[4] = u.x; d[5] = u.y;
-        } else {
-            asm("ld.global.nc.L1::evict_last.f32 %0, [%1];" : "=f"(d[4]) : "l"(p + 128 - 3 * (int)(threadIdx.x & 31)));
-        }
-        return;
-    }
-#pragma unroll
-    for (int q = 0; q < VZ / 4; ++q) {
-        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (q < qn)
-            asm("ld.global.nc.L1::evict_last.v4.f32 {%0, %1, %2, %3}, [%4];"
-                : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "l"(p + 128 * q));
         d[4 * q] = t.x; d[4 * q + 1] = t.y; d[4 * q + 2] = t.z; d[4 * q + 3] = t.w;
     }
 }
@@ -370,139 +312,13 @@ __device__ __forceinline__ void lane_z(int zc, int lane, int nZ, int& z0, int& q
     z0 = qn ? base : 0;
 }
 
-template <int VZ>
-__device__ __forceinline__ void sample_checked(const FastArgs& a, const float* __restrict__ volz, double row,
-                                               double col, float f, float (&acc)[VZ], int qn) {
-    const double fr = floor(row), fc = floor(col);
-    const int r0 = (int)fr, c0 = (int)fc;
-    const bool rc = row > fr, cc = col > fc;
-    const float dr = (float)(row - fr), dc = (float)(col - fc);
-    const bool vr0 = (unsigned)r0 < (unsigned)a.nY, vr1 = rc && (unsigned)(r0 + 1) < (unsigned)a.nY;
-    const bool vc0 = (unsigned)c0 < (unsigned)a.nX, vc1 = cc && (unsigned)(c0 + 1) < (unsigned)a.nX;
-    const float w00 = (1.f - dr) * (1.f - dc) * f, w01 = (1.f - dr) * dc * f;
-    const float w10 = dr * (1.f - dc) * f, w11 = dr * dc * f;
-    float t[VZ];
-    if (vr0 && vc0) {
-        load_vz<VZ>(volz + (size_t)r0 * a.RS + (size_t)c0 * a.nZ, t, qn);
-#pragma unroll
-        for (int e = 0; e < VZ; ++e) acc[e] = fmaf(w00, t[e], acc[e]);
-    }
-    if (vr0 && vc1) {
-        load_vz<VZ>(volz + (size_t)r0 * a.RS + (size_t)(c0 + 1) * a.nZ, t, qn);
-#pragma unroll
-        for (int e = 0; e < VZ; ++e) acc[e] = fmaf(w01, t[e], acc[e]);
-    }
-    if (vr1 && vc0) {
-        load_vz<VZ>(volz + (size_t)(r0 + 1) * a.RS + (size_t)c0 * a.nZ, t, qn);
-#pragma unroll
-        for (int e = 0; e < VZ; ++e) acc[e] = fmaf(w10, t[e], acc[e]);
-    }
-    if (vr1 && vc1) {
-        load_vz<VZ>(volz + (size_t)(r0 + 1) * a.RS + (size_t)(c0 + 1) * a.nZ, t, qn);
-#pragma unroll
-        for (int e = 0; e < VZ; ++e) acc[e] = fmaf(w11, t[e], acc[e]);
-    }
-}
+}  // namespace
+}  // namespace vam
 
-template <int VZ, bool RAY>
-__device__ __forceinline__ void k_forward_fast_body(const FastArgs& a, unsigned bx, unsigned by) {
-    const int lane = threadIdx.x & 31;
-    const int item = bx * kWarpsPerBlock + (threadIdx.x >> 5);
-    const int zc = item % a.zchunks;
-    const int j = item / a.zchunks;
-    const int2 task = a.tasks[by];
-    const bool paired = task.y >= 0;
-    const int N = a.nY;
-    const bool ext = paired && a.even;   // lattice row / column N is needed by the partner angle
-    if (j > (ext ? N : N - 1)) return;   // uniform per warp
-    int z0, qn;
-    lane_z<VZ>(zc, lane, a.nZ, z0, qn);
-    const bool zok = qn > 0;
-    const float* __restrict__ volz = a.vol + z0;
+#include "strip.cuh"
 
-    const double4 tr = a.trig[task.x];
-    const double c = tr.x, s = tr.y;
-    const double rowb = fma(-s, (double)j, tr.w);
-    const double colb = fma(c, (double)j, tr.z);
-    const int kmax = ext ? N : N - 1;
-    int klo, khi;
-    sample_range(rowb, colb, c, s, a.nY, a.nX, kmax, klo, khi);
-
-    float s_entry = 0.f;
-    if (RAY) {
-        const float t = (float)(j - a.C);
-        s_entry = fabsf(t) <= a.R ? -sqrtf(a.R * a.R - t * t) : 0.f;
-        if (fabsf(t) > a.R) klo = 1, khi = 0;
-    }
-    float acc[VZ], e0[VZ], eN[VZ];
-#pragma unroll
-    for (int e = 0; e < VZ; ++e) acc[e] = e0[e] = eN[e] = 0.f;
-
-    if (zok) {
-        const int nYm1 = a.nY - 1, nXm1 = a.nX - 1;
-        const int lo = max(klo, 1), hi = min(khi, N - 1);
-        for (int k = lo; k <= hi; ++k) {
-            const double row = fma(c, (double)k, rowb);
-            const double col = fma(s, (double)k, colb);
-            const float f = RAY ? ray_factor((float)(k - a.C), s_entry, a.alpha) : 1.f;
-            const double fr = floor(row), fc = floor(col);
-            const int r0 = (int)fr, c0 = (int)fc;
-            if ((unsigned)r0 < (unsigned)nYm1 && (unsigned)c0 < (unsigned)nXm1) {
-                // interior: all four taps in the image; a zero-weight ceil tap is
-                // redirected to the floor tap so no unrelated value is read
-                const float dr = (float)(row - fr), dc = (float)(col - fc);
-                const int o00 = r0 * a.RS + c0 * a.nZ;
-                const int dcol = (col > fc) ? a.nZ : 0;
-                const int o10 = o00 + ((row > fr) ? a.RS : 0);
-                float w00 = (1.f - dr) * (1.f - dc), w01 = (1.f - dr) * dc;
-                float w10 = dr * (1.f - dc), w11 = dr * dc;
-                if (RAY) { w00 *= f; w01 *= f; w10 *= f; w11 *= f; }
-                float t0[VZ], t1[VZ], t2[VZ], t3[VZ];
-                load_vz_keep<VZ>(volz + o00, t0, qn);
-                load_vz_keep<VZ>(volz + o00 + dcol, t1, qn);
-                load_vz_keep<VZ>(volz + o10, t2, qn);
-                load_vz_keep<VZ>(volz + o10 + dcol, t3, qn);
-#pragma unroll
-                for (int e = 0; e < VZ; ++e) {
-                    acc[e] = fmaf(w00, t0[e], acc[e]);
-                    acc[e] = fmaf(w01, t1[e], acc[e]);
-                    acc[e] = fmaf(w10, t2[e], acc[e]);
-                    acc[e] = fmaf(w11, t3[e], acc[e]);
-                }
-            } else {
-                sample_checked<VZ>(a, volz, row, col, f, acc, qn);
-            }
-        }
-        if (klo <= 0 && khi >= 0) {
-            const float f = RAY ? ray_factor((float)(0 - a.C), s_entry, a.alpha) : 1.f;
-            sample_checked<VZ>(a, volz, rowb, colb, f, e0, qn);
-        }
-        if (ext && klo <= N && khi >= N)
-            sample_checked<VZ>(a, volz, fma(c, (double)N, rowb), fma(s, (double)N, colb), 1.f, eN, qn);
-    }
-    if (!zok) return;
-    if (j <= N - 1) {
-        float o[VZ];
-#pragma unroll
-        for (int e = 0; e < VZ; ++e) o[e] = acc[e] + e0[e];
-        store_vz<VZ>(a.sino + ((size_t)j * a.nA + task.x) * a.nZ + z0, o, qn);
-    }
-    if (paired) {
-        // partner detector j' = 2C - j over lattice k in [2C-N+1, 2C]
-        const int jp = 2 * a.C - j;
-        if (jp >= 0 && jp <= N - 1) {
-            float o[VZ];
-#pragma unroll
-            for (int e = 0; e < VZ; ++e) o[e] = acc[e] + (a.even ? eN[e] : e0[e]);
-            store_vz<VZ>(a.sino + ((size_t)jp * a.nA + task.y) * a.nZ + z0, o, qn);
-        }
-    }
-}
-
-template <int VZ, bool RAY>
-__global__ void __launch_bounds__(256) k_forward_fast(FastArgs a) {
-    k_forward_fast_body<VZ, RAY>(a, blockIdx.x, blockIdx.y);
-}
+namespace vam {
+namespace {
 
 // ---------------------------------------------------------------------------
 // Matched transpose, fast path: 32 lanes along z, one pixel per warp.
@@ -1919,7 +1735,7 @@ enum Kind : int { KF_FAST = 0, KF_GEN, KB_BATCHED, KB_FAST, KB_GEN, KA_TABLE, KA
 
 struct Item {
     int kind;
-    int vz;          // slices per lane of the template instance (1, 4 or 8)
+    int vz;          // slices per lane of the template instance (1, 4 or 8; 5 or 6 of the block table)
     int ray, occ, absm, batch;
     unsigned gx, gy;  // the call's own grid (blocks of kWarpsPerBlock warps)
     unsigned smem;    // dynamic shared memory of the body
@@ -1940,7 +1756,8 @@ struct Item {
     const int4* btab4;  // KB_BTABLE: the plan's 2 x 2 block bin table and its block index
     const int* bcidx;
     int* status;       // the plan's status word (kernels with bounded waits record timeouts there)
-    int tma, tma_pad_;  // KF_2D: 1 when tmap describes a.in and the tiles are staged by TMA loads
+    const void* once;  // storage of the plan that a batch lists at most once (null: none)
+    int tma, vec;      // vec (KF_FAST): 1 when the rows load as float4s.  KF_2D: tma is 1 when tmap describes a.in and the tiles are staged by TMA loads
     CUtensorMap tmap;   // read from parameter space, as a direct launch's __grid_constant__ argument
 };
 static_assert(sizeof(Item) % 8 == 0, "Item is copied to shared memory in 8-byte words");
@@ -1986,11 +1803,13 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
                 it.pre_in = in; it.pre_mask = a.mask; it.pre_out = plan->d_img_pad;
                 it.pre_npix = (long long)plan->nY * plan->nX; it.pre_nz = 1;
                 it.pre_w = plan->nX; it.pre_wp = wp;
+                it.once = it.pre_out;
                 a.in = plan->d_img_pad;
                 a.mask = nullptr;
             } else if (a.mask) {  // stage the masked image once per call instead of per tile
                 it.pre_in = in; it.pre_mask = plan->d_mask; it.pre_out = plan->d_vol_scratch;
                 it.pre_npix = (long long)plan->nY * plan->nX; it.pre_nz = 1;
+                it.once = it.pre_out;
                 a.in = plan->d_vol_scratch;
                 a.mask = nullptr;
             }
@@ -2008,30 +1827,37 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         }
         return VAM_OK;
     }
-    // the forward's slices per lane: also six / five where 192- / 160-slice chunks fill every lane
-    // (tuned to 6 / 5, or automatic when 256-slice chunks would not)
-    int fvz = vzf;
-    if (fast_ok && plan->nZ % 192 == 0 && (want == 6 || (want == 0 && plan->nZ % 256 != 0))) fvz = 6;
-    else if (fast_ok && plan->nZ % 160 == 0 && (want == 5 || (want == 0 && plan->nZ % 256 != 0))) fvz = 5;
-    if (op == Op::Forward && !plan->has_occ && (long)plan->nY * plan->nX * plan->nZ < (1L << 31) && fvz) {
+    // detector strips: every volume (any slice count, any alignment) without occlusion unless the generic
+    // kernel is tuned (1).  Eight slices per lane where one 128-slice chunk does not hold the volume.
+    // 201^2 x 117 x 240 angles: 3.92 -> 0.37 ms against the generic kernel, which evaluates every sample's
+    // coordinates in float64 for one slice per lane.  With few slices the strips' weights are not shared
+    // enough: at 122^2 x 440 angles the generic kernel takes 59 / 88 / 164 us with 4 / 8 / 12 slices (float4
+    // rows) and 70 / 125 / 188 with 2 / 3 / 6 (single floats), the strips 86 / 88 / 88 and 98 / 99 / 102, and
+    // 1.6 times that where no angle has a partner 180 degrees away.
+    const bool strips = plan->nZ > 8 || (plan->nZ > 4 && plan->nZ % 4 != 0);
+    if (op == Op::Forward && !plan->has_occ && strips && want != 1 &&
+        (long)plan->nY * plan->nX * plan->nZ < (1L << 31)) {
         FastArgs& a = it.f;
-        a.vol = in;
-        if (plan->abs_mode == VAM_ABS_MASK) {
-            it.pre_in = in; it.pre_mask = plan->d_mask; it.pre_out = plan->d_vol_scratch;
-            it.pre_npix = (long long)plan->nY * plan->nX; it.pre_nz = plan->nZ;
-            a.vol = plan->d_vol_scratch;
-        }
-        a.sino = out; a.trig = plan->d_trig;
+        a.vol = in; a.sino = out; a.trig = plan->d_trig;
+        a.mask = plan->abs_mode == VAM_ABS_MASK ? plan->d_mask : nullptr;
         a.nY = plan->nY; a.nX = plan->nX; a.nZ = plan->nZ; a.nA = plan->nA; a.C = plan->C;
-        a.RS = plan->nX * plan->nZ;
-        a.zchunks = (plan->nZ + 32 * fvz - 1) / (32 * fvz);
         a.even = (plan->nY % 2) == 0;
         a.alpha = plan->abs_alpha; a.R = plan->abs_R;
         a.tasks = ray ? plan->d_tasks_single : plan->d_tasks_paired;
-        const long items = (long)(plan->nX + 1) * a.zchunks;
-        it.kind = KF_FAST; it.vz = fvz; it.ray = ray;
-        it.gx = (unsigned)((items + kWarpsPerBlock - 1) / kWarpsPerBlock);
-        it.gy = (unsigned)(ray ? plan->nA : plan->n_tasks_paired);
+        a.ntasks = ray ? plan->nA : plan->n_tasks_paired;
+        it.kind = KF_FAST; it.ray = ray;
+        it.vec = plan->nZ % 4 == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
+        it.vz = want == 4 || (want != 8 && plan->nZ <= 128) ? 4 : 8;
+        a.lz_shift = 5;
+        if (it.vz == 4)  // lanes to spare take other pixels
+            while (a.lz_shift > 2 && (4 << (a.lz_shift - 1)) >= plan->nZ) --a.lz_shift;
+        const int per = it.vz << a.lz_shift, bins = strip_bins(it.vz / 4);
+        a.zchunks = (plan->nZ + per - 1) / per;
+        a.ashift = 2;
+        const int strips = (plan->nX + 1 + bins - 1) / bins, sub = kWarpsPerBlock >> a.ashift;
+        it.gx = (unsigned)(((strips + sub - 1) / sub) * a.zchunks);
+        it.gy = (unsigned)((a.ntasks + (1 << a.ashift) - 1) >> a.ashift);
+        it.once = a.mask;
         return VAM_OK;
     }
     // the block-table backprojection serves every nZ % 4 == 0, also where the automatic width of the
@@ -2131,10 +1957,8 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
     if constexpr ((FAM & 1) != 0) {
         if (it.kind == KF_FAST) {
             const FastArgs f = it.f;
-            if (it.vz == 8) k_forward_fast_body<8, RAY>(f, bx, by);
-            else if (it.vz == 6) k_forward_fast_body<6, RAY>(f, bx, by);
-            else if (it.vz == 5) k_forward_fast_body<5, RAY>(f, bx, by);
-            else k_forward_fast_body<4, RAY>(f, bx, by);
+            if (it.vz == 8) { if (it.vec) forward_strip_body<2, true, RAY>(f, bx, by); else forward_strip_body<2, false, RAY>(f, bx, by); }
+            else { if (it.vec) forward_strip_body<1, true, RAY>(f, bx, by); else forward_strip_body<1, false, RAY>(f, bx, by); }
         }
     }
     if constexpr ((FAM & 128) != 0) {
@@ -2275,10 +2099,8 @@ void launch_fast(const Item& it, dim3 grid, cudaStream_t st) {
             break;
         case KB_2D: k_backward_2d<RAY><<<grid, block, it.smem, st>>>(it.a); break;
         case KF_FAST:
-            if (it.vz == 8) k_forward_fast<8, RAY><<<grid, block, 0, st>>>(it.f);
-            else if (it.vz == 6) k_forward_fast<6, RAY><<<grid, block, 0, st>>>(it.f);
-            else if (it.vz == 5) k_forward_fast<5, RAY><<<grid, block, 0, st>>>(it.f);
-            else k_forward_fast<4, RAY><<<grid, block, 0, st>>>(it.f);
+            if (it.vz == 8) { if (it.vec) k_forward_strip<2, true, RAY><<<grid, block, 0, st>>>(it.f); else k_forward_strip<2, false, RAY><<<grid, block, 0, st>>>(it.f); }
+            else { if (it.vec) k_forward_strip<1, true, RAY><<<grid, block, 0, st>>>(it.f); else k_forward_strip<1, false, RAY><<<grid, block, 0, st>>>(it.f); }
             break;
         case KB_BATCHED:
             if (it.vz == 8 && !RAY) k_backward_batched8<<<grid, block, it.smem, st>>>(it.a);
@@ -2401,7 +2223,7 @@ static_assert(sizeof(BatchParams) < 32000, "batch parameters must fit the 32 KB 
 // block-table backprojection (four bodies: 4 or 8 slices, full or partial z
 // chunks) 128 (two).
 template <int FAM>
-__global__ void __launch_bounds__(256, FAM == 64 ? 6 : (FAM == 2 || FAM == 128 ? 5 : (FAM == 1 || FAM == 32 ? 4 : (FAM == 256 ? 2 : 3))))
+__global__ void __launch_bounds__(256, FAM == 64 ? 6 : (FAM == 2 || FAM == 128 ? 5 : (FAM == 32 ? 4 : (FAM == 1 || FAM == 256 ? 2 : 3))))
     k_batch(const __grid_constant__ BatchParams P) {
     __shared__ unsigned s_t[2];
     __shared__ int s_idx[2];
@@ -2596,8 +2418,8 @@ extern "C" int vam_parallel_set_absorption(vam_parallel_plan* p, int mode, const
     if (mode == VAM_ABS_MASK) {
         VAM_REQUIRE(mask_dev, VAM_ERR_ARG, "vam_parallel_set_absorption: MASK needs mask_dev");
         if (!p->d_mask) VAM_TRY_CUDA(cudaMalloc(&p->d_mask, sizeof(float) * (size_t)p->nY * p->nX));
-        if (!p->d_vol_scratch)
-            VAM_TRY_CUDA(cudaMalloc(&p->d_vol_scratch, sizeof(float) * (size_t)p->nY * p->nX * p->nZ));
+        if (!p->d_vol_scratch && p->nZ == 1)  // the masked slice of the plain-load 2-D tiles
+            VAM_TRY_CUDA(cudaMalloc(&p->d_vol_scratch, sizeof(float) * (size_t)p->nY * p->nX));
         VAM_TRY_CUDA(cudaMemcpyAsync(p->d_mask, mask_dev, sizeof(float) * (size_t)p->nY * p->nX,
                                      cudaMemcpyDeviceToDevice, (cudaStream_t)stream));
     }
@@ -3002,9 +2824,9 @@ int batch_prepare(vam_batch* b, const vam_work* work, int32_t n) {
         items[i].cost = (long long)std::llround((double)items[i].cost * time_weight(items[i]));
     }
     // a staged forward writes its plan's scratch: two such calls of one plan would share it
-    std::vector<const float*> staged;
+    std::vector<const void*> staged;
     for (const Item& it : items)
-        if (it.pre_out) staged.push_back(it.pre_out);
+        if (it.once) staged.push_back(it.once);
     std::sort(staged.begin(), staged.end());
     VAM_REQUIRE(std::adjacent_find(staged.begin(), staged.end()) == staged.end(), VAM_ERR_ARG,
                 "vam_batch: two forwards of one plan stage their input into the same scratch");

@@ -1,0 +1,477 @@
+// strip.cuh -- the rotate-and-sum forward by detector strips.
+//
+// One warp owns M neighbouring detector bins (a strip) of one angle, or of an angle and the one 180
+// degrees from it, over the slices of one z chunk.  The forward is linear in the pixels: bin j of an angle
+// gets W(j, p) x(p) from pixel p with
+//     W(j, p) = sum over samples k of hat(row(j, k) - row_p) hat(col(j, k) - col_p),  hat(d) = max(0, 1 - |d|),
+// the bilinear weights of all samples of the bin that touch the pixel (Projector3DParallel.py:137-156 via
+// skimage.warp).  Going through the pixels under the strip instead of through its samples loads every
+// pixel's row of slices once for all M bins and all their samples: 1.33 rows per sample for M = 4 (3.26 / 2
+// for two bins, 2.26 for one), against four taps per sample.  The rows' loads are what bounds the forward
+// (L1 data path), so this is where its time goes down.
+//
+// The warp lists the pixels in batches: the 32 lanes take R rows (or columns, whichever the rays run across)
+// of S candidate pixels, form each pixel's position in the rotated lattice and, from its fractions, its M
+// weights; pixels with any nonzero weight go through a ring in shared memory (pixel, M weights) that the same
+// warp then works off, U pixels at a time, the next U pixels' rows in flight meanwhile.
+//
+// Measured (B200): 256^3 x 360 angles 1.39 -> 0.84 ms, 512^2 x 128 x 720 7.30 -> 4.49 ms, 192^3 x 720 1.34 ->
+// 0.89 ms, 201^2 x 117 x 240 3.92 -> 0.37 ms against the sample kernels before.  At 256^3 the L1 data path is
+// 68 % busy (a pixel is eight cycles of row and three or four of weights, which are written to every lane's
+// registers), issue 54 %, FP32 50 %; the rest is what 16 warps leave uncovered.
+#pragma once
+
+#include "vam_internal.cuh"
+
+namespace vam {
+namespace {
+
+// Bins per strip: two with eight slices per lane, three with four.  A strip's pixel costs its row's loads and
+// one broadcast load of its weights; three bins share the row better (4.30 against 4.86 ms at 512^2 x 128 x 720,
+// four slices per lane) until their accumulators take the registers that keep rows in flight (0.93 against
+// 0.82 ms at 256^3 x 360, eight slices per lane).
+__host__ __device__ constexpr int strip_bins(int q) { return q == 2 ? 2 : 3; }
+constexpr int kStripRing = 128;  // ring entries per warp (the whole groups of them): a group short of one entry and a batch of 32 fit
+
+// The strip's geometry, read back by every batch (registers are what the rows in flight need).  A pixel is
+// (main, other): (row, column) when the rays run across rows, (column, row) otherwise.  Its lattice position
+// is J = jc.x main + jc.y other + j0, K = kc.x main + kc.y other + k0; the fractions come from the same sums
+// in 32-bit fixed point, whose overflow drops the whole part, with the coefficients' rounding added back in
+// float32, so they are good to float32 rounding at any size.
+struct StripGeo {
+    float4 coef;   // J and K per step of main and other
+    float4 res;    // what the fixed-point coefficients leave out
+    int4 fix;      // the coefficients times 2^32, modulo 2^32
+    float4 org;    // J and K at the origin; least other of the strip = slope * main + base
+    int2 fixorg;   // the origin in fixed point
+    float4 cs;     // cos and sin, and what their float32 values leave out
+};
+
+struct StripRing {
+    float4 e[kWarpsPerBlock][kStripRing];  // M weights and the pixel
+    StripGeo geo[kWarpsPerBlock];
+};
+
+__device__ __forceinline__ StripRing& strip_ring() {
+    __shared__ __align__(16) StripRing r;
+    return r;
+}
+
+struct FastArgs {
+    const float* vol;
+    float* sino;
+    const double4* trig;
+    const int2* tasks;
+    const float* mask;  // per-pixel factor of the volume, or null
+    int nY, nX, nZ, nA, C;
+    int ntasks;
+    int zchunks;
+    int lz_shift;    // log2 of the lanes along z (a warp's other lanes take other pixels)
+    int ashift;      // log2 of the angle tasks per block
+    int even;        // N even
+    float alpha, R;  // per-ray absorption (tasks are unpaired then)
+};
+
+// A lane's 4 Q slices of one pixel's row as slice pairs, p pointing at its first.  VEC: float4s 4 LZ apart
+// (LZ = 32 when Q = 2), the first n of them inside the volume.  Otherwise single slices LZ apart, any slice
+// count and any alignment.  Slices past the volume are not read; their values are undefined.
+template <int Q, bool VEC>
+__device__ __forceinline__ void strip_load(const float* __restrict__ p, unsigned long long (&v)[2 * Q], int n, int lz) {
+    if constexpr (VEC) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            asm volatile("{ .reg .pred p; setp.gt.s32 p, %3, %4; @p ld.global.nc.v2.u64 {%0, %1}, [%2]; }"
+                : "=l"(v[2 * q]), "=l"(v[2 * q + 1]) : "l"(p + 128 * q), "r"(n), "r"(q));
+    } else {
+        const int st = Q == 2 ? 32 : lz;
+#pragma unroll
+        for (int e = 0; e < 2 * Q; ++e) {
+            float lo, hi;
+            asm volatile("{ .reg .pred p; setp.gt.s32 p, %2, %3; @p ld.global.nc.f32 %0, [%1]; }"
+                : "=f"(lo) : "l"(p + st * 2 * e), "r"(n), "r"(2 * e));
+            asm volatile("{ .reg .pred p; setp.gt.s32 p, %2, %3; @p ld.global.nc.f32 %0, [%1]; }"
+                : "=f"(hi) : "l"(p + st * (2 * e + 1)), "r"(n), "r"(2 * e + 1));
+            v[e] = pk_pair(lo, hi);
+        }
+    }
+}
+
+__device__ __forceinline__ void fma_pairs(unsigned long long& acc, unsigned long long w2, unsigned long long v2) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(w2), "l"(v2));
+}
+
+template <int Q, bool VEC>
+__device__ __forceinline__ void strip_store(float* __restrict__ p, const unsigned long long (&v)[2 * Q], int n, int lz) {
+    if constexpr (VEC) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            if (q < n) *reinterpret_cast<ulonglong2*>(p + 128 * q) = make_ulonglong2(v[2 * q], v[2 * q + 1]);
+    } else {
+        const int st = Q == 2 ? 32 : lz;
+#pragma unroll
+        for (int e = 0; e < 2 * Q; ++e) {
+            float lo, hi;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v[e]));
+            if (2 * e < n) p[st * 2 * e] = lo;
+            if (2 * e + 1 < n) p[st * (2 * e + 1)] = hi;
+        }
+    }
+}
+
+// One bilinear sample (every tap checked against the image) times f added into acc: the end samples k = 0 and
+// k = N of a paired strip, which belong to one of its two angles only.
+template <int Q, bool VEC>
+__device__ __forceinline__ void strip_sample(const FastArgs& a, const float* __restrict__ volz, double row, double col,
+                                             unsigned long long (&acc)[2 * Q], int n, int lz, float f = 1.f) {
+    const double fr = floor(row), fc = floor(col);
+    const int r0 = (int)fr, c0 = (int)fc;
+    const float dr = (float)(row - fr), dc = (float)(col - fc);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        const int r = r0 + (t >> 1), c = c0 + (t & 1);
+        if ((unsigned)r >= (unsigned)a.nY || (unsigned)c >= (unsigned)a.nX) continue;
+        if (((t >> 1) && !(row > fr)) || ((t & 1) && !(col > fc))) continue;
+        float w = ((t >> 1) ? dr : 1.f - dr) * ((t & 1) ? dc : 1.f - dc) * f;
+        const unsigned p = (unsigned)r * (unsigned)a.nX + (unsigned)c;
+        if (a.mask) w *= __ldg(a.mask + p);
+        unsigned long long v[2 * Q];
+        strip_load<Q, VEC>(volz + (size_t)p * a.nZ, v, n, lz);
+#pragma unroll
+        for (int e = 0; e < 2 * Q; ++e) fma_pairs(acc[e], pk_pair(w, w), v[e]);
+    }
+}
+
+// Blocks: 2^ashift angle tasks times 8 / 2^ashift neighbouring strips, which read the same pixels at about
+// the same time.
+//
+// Stores lattice row j's sum: both angles' bins, for even N with the end sample of each (angle a sums k =
+// 0 .. N - 1 of rows 0 .. N - 1, its partner k = 1 .. N of rows 1 .. N).
+template <int Q, bool VEC>
+__device__ __forceinline__ void strip_finish(const FastArgs& a, int2 task, bool ext, int j, const float* __restrict__ volz,
+                                             int z0, int n, int lz, unsigned long long (&sum)[2 * Q]) {
+    float* const here = a.sino + ((size_t)j * a.nA + task.x) * a.nZ + z0;
+    float* const there = a.sino + ((size_t)(2 * a.C - j) * a.nA + task.y) * a.nZ + z0;
+    if (!ext) {
+        strip_store<Q, VEC>(here, sum, n, lz);
+        if (task.y >= 0) strip_store<Q, VEC>(there, sum, n, lz);
+        return;
+    }
+    const double4 tr = a.trig[task.x];
+    const double rowb = fma(-tr.y, (double)j, tr.w), colb = fma(tr.x, (double)j, tr.z);
+    const int N = a.nY;
+    if (j < N) {
+        unsigned long long o[2 * Q];
+#pragma unroll
+        for (int e = 0; e < 2 * Q; ++e) o[e] = sum[e];
+        strip_sample<Q, VEC>(a, volz, rowb, colb, o, n, lz);
+        strip_store<Q, VEC>(here, o, n, lz);
+    }
+    if (j > 0) {
+        strip_sample<Q, VEC>(a, volz, fma(tr.x, (double)N, rowb), fma(tr.y, (double)N, colb), sum, n, lz);
+        strip_store<Q, VEC>(there, sum, n, lz);
+    }
+}
+
+// The sums run over all M bins of every listed pixel; a zero weight then spreads an infinity or a NaN to
+// bins that do not sample it.  A strip with a non-finite sum is therefore done again sample by sample.
+template <int Q, bool VEC, bool RAY>
+__device__ __noinline__ void forward_strip_samples(const FastArgs& a, unsigned bx, unsigned by);
+
+// The warp's place: angle task, first bin, lane's first slice and number of slices (float4s), false when idle.
+template <int Q, bool VEC>
+__device__ __forceinline__ bool strip_place(const FastArgs& a, unsigned bx, unsigned by, int2& task, bool& ext, int& j0,
+                                            int& z0, int& n) {
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, sshift = 3 - a.ashift, LZ = 1 << a.lz_shift;
+    const int ti = (int)((by << a.ashift) + (wp >> sshift));
+    j0 = (int)(((bx / (unsigned)a.zchunks) << sshift) + (wp & ((1 << sshift) - 1))) * strip_bins(Q);
+    if (ti >= a.ntasks) return false;
+    task = a.tasks[ti];
+    ext = task.y >= 0 && a.even;  // lattice row and sample N belong to the partner angle
+    if (j0 > (ext ? a.nY : a.nY - 1)) return false;
+    constexpr int per = VEC ? 4 : 1;
+    z0 = (int)(bx % (unsigned)a.zchunks) * LZ * 4 * Q + per * (lane & (LZ - 1));
+    n = 0;
+#pragma unroll
+    for (int e = 0; e < 4 * Q / per; ++e) n += z0 + per * LZ * e < a.nZ ? 1 : 0;
+    if (n == 0) z0 = 0;
+    return true;
+}
+
+template <int Q, bool VEC, bool RAY>
+__device__ __forceinline__ void forward_strip_body(const FastArgs& a, unsigned bx, unsigned by) {
+    constexpr int M = strip_bins(Q), U = Q == 2 ? 3 : 4, VZ = 4 * Q;
+    StripRing& ring = strip_ring();
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    int2 task;
+    bool ext;
+    int j0, z0, n;
+    if (!strip_place<Q, VEC>(a, bx, by, task, ext, j0, z0, n)) return;  // uniform per warp
+    const int N = a.nY, jmax = ext ? N : N - 1;
+    const int LZ = 1 << a.lz_shift, g = lane >> a.lz_shift, G = 32 >> a.lz_shift;
+    const float* __restrict__ volz = a.vol + z0;
+
+    const double4 tr = a.trig[task.x];
+    const double c = tr.x, s = tr.y;
+    const double B = fabs(c) + fabs(s);  // a bin touches pixels nearer than this along the detector
+    const bool rmain = fabs(c) >= fabs(s);  // the rays run across rows (else across columns)
+    const bool on_axis = fmin(fabs(c), fabs(s)) < 1e-12;
+    const int kfirst = ext ? 1 : 0, klast = N - 1;
+
+    // rows (columns) the strip's samples inside the image touch
+    int mlo = INT_MAX, mhi = INT_MIN;
+    if (lane < M && j0 + lane <= jmax) {
+        const double rowb = fma(-s, (double)(j0 + lane), tr.w), colb = fma(c, (double)(j0 + lane), tr.z);
+        int klo, khi;
+        sample_range(rowb, colb, c, s, a.nY, a.nX, klast, klo, khi);
+        klo = max(klo, kfirst);
+        if (klo <= khi) {
+            const double p0 = rmain ? fma(c, (double)klo, rowb) : fma(s, (double)klo, colb);
+            const double p1 = rmain ? fma(c, (double)khi, rowb) : fma(s, (double)khi, colb);
+            mlo = (int)floor(fmin(p0, p1));
+            mhi = (int)floor(fmax(p0, p1)) + 1;
+        }
+    }
+    mlo = max(__reduce_min_sync(kFull, mlo), 0);
+    mhi = min(__reduce_max_sync(kFull, mhi), (rmain ? a.nY : a.nX) - 1);
+
+    // sum: the batches finished so far; acc: the current one.  Adding batch by batch keeps the rounding of a
+    // long ray's sum at well below a running sum's (64^2 x 40 x 90: 1.1e-7 -> 6.8e-8 relative to float64; 256^3 x 360: 3.8e-7 -> 1.0e-7).
+    unsigned long long sum[M][VZ / 2], acc[M][VZ / 2];
+    // U * G entries from head on: their rows into flight, and the bins' sums once the rows are there
+    auto entries = [&](const float4* ep, float4 (&t)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) t[u] = ep[u];
+    };
+    auto rows = [&](const float4 (&t)[U], unsigned long long (&v)[U][VZ / 2]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            strip_load<Q, VEC>(volz + (size_t)__float_as_uint(t[u].w) * (unsigned)a.nZ, v[u], n, LZ);
+    };
+    auto add1 = [&](const float4& t, const unsigned long long (&v)[VZ / 2]) {
+        const float w[3] = {t.x, t.y, t.z};
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+            for (int e = 0; e < VZ / 2; ++e) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[m][e]) : "l"(pk_pair(w[m], w[m])), "l"(v[e]));
+    };
+    // one step: the next group's entries, one pixel of the waiting group while they arrive, the next
+    // group's rows into flight, the rest of the waiting group
+    auto step = [&](const float4* ep, float4 (&tn)[U], unsigned long long (&vn)[U][VZ / 2], const float4 (&tc)[U],
+                    const unsigned long long (&vc)[U][VZ / 2]) {
+        entries(ep, tn);
+        add1(tc[0], vc[0]);
+        rows(tn, vn);
+#pragma unroll
+        for (int u = 1; u < U; ++u) add1(tc[u], vc[u]);
+    };
+
+    const bool some = mlo <= mhi;
+    int R = 1, lr = 0, slot = 0;
+    if (some) {
+        const double inv = 1.0 / (rmain ? c : s);
+        const double slack = 1e-3 + 2e-6 * N;  // covers the float32 rounding of the edge
+        const int S = (int)(((double)(M - 1) + 2.0 * B) * fabs(inv) + 2.0 * slack) + 1;  // pixels of one row under the strip
+        R = 32 / S;
+        lr = lane / S;
+        slot = lane - lr * S;
+        if (lane == 0) {
+            StripGeo& q = ring.geo[wp];
+            // the edge of the strip (widened by B) that has its least column (row)
+            const double jlo = (rmain ? c > 0.0 : s < 0.0) ? (double)j0 - B : (double)(j0 + M - 1) + B;
+            const double jo = fma(s, tr.w, -c * tr.z), ko = -fma(c, tr.w, s * tr.z);
+            const double x = rmain ? -s : c, y = rmain ? c : -s, z = rmain ? c : s, w = rmain ? s : c;
+            const double two32 = 4294967296.0, qx = rint(x * two32), qy = rint(y * two32), qz = rint(z * two32),
+                         qw = rint(w * two32);
+            q.coef = make_float4((float)x, (float)y, (float)z, (float)w);
+            q.res = make_float4((float)(x - qx / two32), (float)(y - qy / two32), (float)(z - qz / two32), (float)(w - qw / two32));
+            q.fix = make_int4((int)(long long)qx, (int)(long long)qy, (int)(long long)qz, (int)(long long)qw);
+            q.org = make_float4((float)jo, (float)ko, (float)((rmain ? s : c) * inv),
+                                (float)((rmain ? (jlo - s * tr.w) * inv + tr.z : tr.w - (c * tr.z + jlo) * inv) - slack));
+            q.fixorg = make_int2((int)(long long)rint(jo * two32), (int)(long long)rint(ko * two32));
+            q.cs = make_float4((float)c, (float)s, (float)(c - (double)(float)c), (float)(s - (double)(float)s));
+        }
+        __syncwarp();
+    }
+
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+        for (int e = 0; e < VZ / 2; ++e) sum[m][e] = acc[m][e] = 0ull;
+    auto carry = [&]() {
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+            for (int e = 0; e < VZ / 2; ++e) {
+                asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[m][e]) : "l"(acc[m][e]));
+                acc[m][e] = 0ull;
+            }
+    };
+    if (some) {
+        float4 t0[U], t1[U];
+        unsigned long long v0[U][VZ / 2], v1[U][VZ / 2];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            t0[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int e = 0; e < VZ / 2; ++e) v0[u][e] = 0ull;
+        }
+        // the ring holds whole rounds of two groups, so a group never wraps
+        const int round = 2 * U * G, size = kStripRing - kStripRing % round;
+        const float4* const first = &ring.e[wp][g * U];
+        int head = 0, tail = 0, wait = 0;  // next to work off, next free, number between them
+        for (int m0 = mlo; m0 <= mhi; m0 += R) {
+            const StripGeo& q = ring.geo[wp];
+            const int mi = m0 + lr;
+            const float fm = (float)mi;
+            const int ot = (int)ceilf(fmaf(fm, q.org.z, q.org.w)) + slot;
+            const unsigned pix = rmain ? (unsigned)mi * (unsigned)a.nX + (unsigned)ot : (unsigned)ot * (unsigned)a.nX + (unsigned)mi;
+            float W[3] = {0.f, 0.f, 0.f};
+            bool listed = false;
+            if (lr < R && mi <= mhi && (unsigned)ot < (unsigned)N) {
+                const float fo = (float)ot;
+                // nearest lattice point (Jn, Kn) and the pixel's offset from it
+                const float4 co = q.coef, re = q.res;
+                const int4 fx = q.fix;
+                const float dj = fmaf((float)(fx.x * mi + fx.y * ot + q.fixorg.x), 2.3283064e-10f, fmaf(re.x, fm, re.y * fo));
+                const float dk = fmaf((float)(fx.z * mi + fx.w * ot + q.fixorg.y), 2.3283064e-10f, fmaf(re.z, fm, re.w * fo));
+                const float Jn = rintf(fmaf(co.x, fm, fmaf(co.y, fo, q.org.x)) - dj);
+                const float Kn = rintf(fmaf(co.z, fm, fmaf(co.w, fo, q.org.y)) - dk);
+                // cos and sin to more than float32: their rounding would scale every weight of the angle
+                const float4 cs = q.cs;
+                // samples Kn - 1 .. Kn + 1; one outside the ray is moved away, where its weight is zero
+                float ck[3], sk[3];
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    const float kb = Kn + (float)(b - 1);
+                    const float kk = (kb >= (float)kfirst && kb <= (float)klast) ? (float)(b - 1) - dk : 1e9f;
+                    ck[b] = fmaf(cs.x, kk, cs.z * kk);
+                    sk[b] = fmaf(cs.y, kk, cs.w * kk);
+                }
+                const float jn = (float)j0 - Jn;
+#pragma unroll
+                for (int m = 0; m < M; ++m) {
+                    const float d = (jn + (float)m) - dj;
+                    float sent = 0.f;
+                    bool dark = j0 + m > jmax;
+                    if (RAY) {
+                        const float t = (float)(j0 + m - a.C);
+                        if (fabsf(t) > a.R) dark = true;
+                        else sent = -sqrtf(a.R * a.R - t * t);
+                    }
+                    const float sd = -fmaf(cs.y, d, cs.w * d), cd = fmaf(cs.x, d, cs.z * d);
+                    float w = 0.f;
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) {
+                        float h = __saturatef(1.f - fabsf(ck[b] + sd)) * __saturatef(1.f - fabsf(sk[b] + cd));
+                        if (RAY && h != 0.f) h *= ray_factor(Kn + (float)(b - 1 - a.C), sent, a.alpha);
+                        w += h;
+                    }
+                    W[m] = dark ? 0.f : w;
+                    listed |= W[m] != 0.f;
+                }
+                // on an axis the samples' float64 rounding may touch the next row or column with a weight that is
+                // zero here; listing those pixels too lets an infinity in them through
+                listed |= on_axis;
+                if (a.mask) {
+                    const float f = __ldg(a.mask + pix);
+#pragma unroll
+                    for (int m = 0; m < M; ++m) W[m] *= f;
+                }
+            }
+            const unsigned has = __ballot_sync(kFull, listed);
+            if (listed) {
+                const int at = tail + __popc(has & ((1u << lane) - 1u));
+                ring.e[wp][at < size ? at : at - size] = make_float4(W[0], W[1], W[2], __uint_as_float(pix));
+            }
+            const int cnt = __popc(has);
+            tail = tail + cnt < size ? tail + cnt : tail + cnt - size;
+            wait += cnt;
+            __syncwarp();
+            for (; wait >= round; wait -= round) {
+                step(first + head, t1, v1, t0, v0);
+                step(first + head + U * G, t0, v0, t1, v1);
+                head = head + round < size ? head + round : 0;
+            }
+            carry();
+            __syncwarp();  // the entries worked off are free again
+        }
+        if (wait > 0) {  // the rest, filled up with entries of no weight (and the first pixel's row)
+            for (int k = wait + lane; k < round; k += 32) ring.e[wp][head + k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            __syncwarp();
+            step(first + head, t1, v1, t0, v0);
+            step(first + head + U * G, t0, v0, t1, v1);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) add1(t0[u], v0[u]);
+        carry();
+        __syncwarp();
+        float bad = 0.f;
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+            for (int e = 0; e < VZ / 2; ++e) {
+                float lo, hi;
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(sum[m][e]));
+                // (slices past the volume hold anything)
+                if (VEC ? e / 2 < n : 2 * e < n) bad = fmaf(lo, 0.f, bad);
+                if (VEC ? e / 2 < n : 2 * e + 1 < n) bad = fmaf(hi, 0.f, bad);
+            }
+        if (__any_sync(kFull, bad != 0.f)) {
+            forward_strip_samples<Q, VEC, RAY>(a, bx, by);
+            return;
+        }
+    }
+
+    if constexpr (Q == 1)  // the groups' parts
+        for (int off = LZ; off < 32; off <<= 1)
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+#pragma unroll
+                for (int e = 0; e < VZ / 2; ++e) {
+                    const unsigned long long t = __shfl_xor_sync(kFull, sum[m][e], off);
+                    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[m][e]) : "l"(t));
+                }
+    if (n == 0 || g != 0) return;
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+        if (j0 + m <= jmax) strip_finish<Q, VEC>(a, task, ext, j0 + m, volz, z0, n, LZ, sum[m]);
+}
+
+template <int Q, bool VEC, bool RAY>
+__device__ __noinline__ void forward_strip_samples(const FastArgs& a, unsigned bx, unsigned by) {
+    int2 task;
+    bool ext;
+    int j0, z0, n;
+    if (!strip_place<Q, VEC>(a, bx, by, task, ext, j0, z0, n)) return;
+    const int LZ = 1 << a.lz_shift, N = a.nY;
+    if (n == 0 || (threadIdx.x & 31) >> a.lz_shift) return;
+    const float* __restrict__ volz = a.vol + z0;
+    const double4 tr = a.trig[task.x];
+    for (int m = 0; m < strip_bins(Q) && j0 + m <= (ext ? N : N - 1); ++m) {
+        const int j = j0 + m;
+        const double rowb = fma(-tr.y, (double)j, tr.w), colb = fma(tr.x, (double)j, tr.z);
+        unsigned long long acc[2 * Q] = {};
+        int klo, khi;
+        sample_range(rowb, colb, tr.x, tr.y, a.nY, a.nX, N - 1, klo, khi);
+        float sent = 0.f;
+        if (RAY) {
+            const float t = (float)(j - a.C);
+            if (fabsf(t) > a.R) khi = -1;
+            else sent = -sqrtf(a.R * a.R - t * t);
+        }
+        for (int k = max(klo, ext ? 1 : 0); k <= khi; ++k)
+            strip_sample<Q, VEC>(a, volz, fma(tr.x, (double)k, rowb), fma(tr.y, (double)k, colb), acc, n, LZ,
+                                 RAY ? ray_factor((float)(k - a.C), sent, a.alpha) : 1.f);
+        strip_finish<Q, VEC>(a, task, ext, j, volz, z0, n, LZ, acc);
+    }
+}
+
+// 128 registers, two blocks per SM: rows in flight per warp hide more than a third block does (three at 80
+// registers: 0.88 against 0.82 ms at 256^3 x 360)
+template <int Q, bool VEC, bool RAY>
+__global__ void __launch_bounds__(256, 2) k_forward_strip(FastArgs a) {
+    forward_strip_body<Q, VEC, RAY>(a, blockIdx.x, blockIdx.y);
+}
+
+}  // namespace
+}  // namespace vam
