@@ -151,6 +151,22 @@ int vam_parallel_backward_ref_noclip(vam_parallel_plan* plan, const float* sino_
 int vam_parallel_adjoint(vam_parallel_plan* plan, const float* sino_dev, float* vol_dev,
                          vam_stream_t stream);
 
+/* The projections of a plan whose slice count is not a multiple of four read
+ * single floats; with the input's rows of slices padded they read float4s.
+ * vam_pad_rows copies `rows` rows of nz floats into rows of nz rounded up to a
+ * multiple of four, the padding zero (out: 16-byte aligned).
+ * vam_parallel_apply_padded runs op (VAM_OP_*) of the plan on such an input
+ * (volume rows for the forward, sinogram rows otherwise); the output's rows are
+ * the plan's own.  vam_parallel_prepare_padded builds the bin table that the
+ * padded backprojection reads (allocates: before any stream capture).
+ * VAM_ERR_NOTSUP for what the padded kernels do not serve: an
+ * occlusion, a forward or transpose of few slices or with its generic kernel
+ * selected by the tuning, a single slice. */
+int vam_pad_rows(const float* x_dev, int64_t rows, int32_t nz, float* out_dev, vam_stream_t stream);
+int vam_parallel_prepare_padded(vam_parallel_plan* plan, vam_stream_t stream);
+int vam_parallel_apply_padded(vam_parallel_plan* plan, int32_t op, const float* in_dev, float* out_dev,
+                              vam_stream_t stream);
+
 /* Launch shapes of the parallel-beam kernels, chosen per problem by an
  * autotuner (vamtoolbox_b200/autotune.py times the candidates on the device
  * and caches the winner per device and problem shape).  Vector widths are the
@@ -159,7 +175,7 @@ int vam_parallel_adjoint(vam_parallel_plan* plan, const float* sino_dev, float* 
  * value but 0 and 1 selects the shared-memory tile kernels, which 0 picks from
  * 192 (forward) and 320 (backprojection) pixels up); backward_batch is the
  * number of angles whose detector rows one warp loads together (1, 2 or 4);
- * adjoint_table selects the table-driven transpose once it is prepared.
+ * adjoint_table is accepted and has no effect.
  * No counterpart in the reference. */
 typedef struct {
     int32_t forward_vz, backward_vz, adjoint_vz;
@@ -202,10 +218,11 @@ int vam_parallel_get_tuning(vam_parallel_plan* plan, vam_parallel_tuning* tuning
  * Replaces running the reference's per-target projector calls one target at a
  * time (vamtoolbox/projector/Projector3DParallel.py:113-207 per target). */
 typedef struct vam_batch vam_batch;
-enum { VAM_OP_FORWARD = 0, VAM_OP_BACKWARD_REF = 1, VAM_OP_ADJOINT = 2 };
+enum { VAM_OP_FORWARD = 0, VAM_OP_BACKWARD_REF = 1, VAM_OP_ADJOINT = 2,
+       VAM_OP_PADDED = 16 /* flag: the input's rows are padded as by vam_pad_rows (vam_parallel_apply_padded) */ };
 typedef struct {
     vam_parallel_plan* plan;
-    int32_t op;        /* VAM_OP_* */
+    int32_t op;        /* VAM_OP_*, with VAM_OP_PADDED for padded input rows */
     const float* in;   /* volume (forward) or sinogram, device */
     float* out;        /* sinogram (forward) or volume, device */
 } vam_work;
@@ -217,12 +234,9 @@ int vam_batch_prepare(vam_batch* batch, const vam_work* work, int32_t n, vam_str
 /* blocks (over all calls' grids) of the last submitted list and persistent CTAs of its launch */
 int vam_batch_info(vam_batch* batch, int64_t* virtual_blocks, int32_t* ctas);
 
-/* Builds the plan's matched-transpose weight table (16 bytes per pixel and
- * angle: the detector rows that sample the pixel and their summed forward
- * weights), after which vam_parallel_adjoint is a pure gather.  Allocates;
- * call once before capturing adjoint calls in a graph, and again after
- * vam_parallel_set_absorption.  Without it the adjoint enumerates the
- * sampling lattice on the fly.  No counterpart in the reference. */
+/* Accepted and does nothing: the matched transpose forms its weights as it
+ * goes (it read a table of 16 bytes per pixel and angle before).  No
+ * counterpart in the reference. */
 int vam_parallel_prepare_adjoint(vam_parallel_plan* plan, vam_stream_t stream);
 
 /* ======================================================================= */

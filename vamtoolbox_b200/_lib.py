@@ -66,6 +66,7 @@ class ParallelTuning(ctypes.Structure):
 
 
 OP_FORWARD, OP_BACKWARD_REF, OP_ADJOINT = 0, 1, 2
+OP_PADDED = 16
 
 
 class Work(ctypes.Structure):
@@ -116,6 +117,9 @@ _SIGS = {
     "vam_parallel_adjoint": ([_vp, _vp, _vp, _vp], _c_int),
     "vam_parallel_prepare_adjoint": ([_vp, _vp], _c_int),
     "vam_parallel_prepare_backward": ([_vp, _vp], _c_int),
+    "vam_pad_rows": ([_vp, _c_i64, _c_i32, _vp, _vp], _c_int),
+    "vam_parallel_prepare_padded": ([_vp, _vp], _c_int),
+    "vam_parallel_apply_padded": ([_vp, _c_i32, _vp, _vp, _vp], _c_int),
     "vam_parallel_status": ([_vp, ctypes.POINTER(_c_i32)], _c_int),
     "vam_parallel_set_tuning": ([_vp, ctypes.POINTER(ParallelTuning)], _c_int),
     "vam_parallel_get_tuning": ([_vp, ctypes.POINTER(ParallelTuning)], _c_int),

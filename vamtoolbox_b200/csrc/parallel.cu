@@ -75,7 +75,10 @@ struct Args {
     int nY, nX, nZ, nA, C;
     int lz_shift, zvec, zchunks;
     float alpha, R;  // VAM_ABS_RAY
-    int occ_mode, pad_;
+    int occ_mode;
+    int zs;     // floats from one input row to the next (nZ, or nZ rounded up to four: padded rows)
+    int whole;  // the output's rows take float4 stores
+    int pad_;
 };
 
 template <int VZ>
@@ -321,89 +324,6 @@ namespace vam {
 namespace {
 
 // ---------------------------------------------------------------------------
-// Matched transpose, fast path: 32 lanes along z, one pixel per warp.
-//
-// The forward's tap weight of pixel (i, j) from lattice sample (J, K) is
-// hat(i - row(J,K)) * hat(j - col(J,K)) with hat(d) = max(0, 1 - |d|) (the
-// floor / ceil weights (1-dr), dr are exactly that).  The pixel's offset to
-// its nearest lattice point (J0, K0) is formed once in float64 from the same
-// coordinate expression the forward uses; the offsets to the 3 x 3 candidate
-// lattice points follow in float32 by adding multiples of (s, -c) and
-// (-c, -s), small numbers, so every candidate weight agrees with the
-// forward's to ~1e-7 and the kernel gathers at most 3 detector rows per angle.
-// ---------------------------------------------------------------------------
-template <int VZ, bool RAY>
-__device__ __forceinline__ void k_adjoint_fast_body(const Args& a, unsigned bx, unsigned by) {
-    const int lane = threadIdx.x & 31;
-    const long item = (long)bx * kWarpsPerBlock + (threadIdx.x >> 5);
-    const int zchunks = a.zchunks;
-    const int zc = (int)(item % zchunks);
-    const long p = item / zchunks;
-    if (p >= (long)a.nY * a.nX) return;
-    const int i = (int)(p / a.nX), j = (int)(p % a.nX);
-    int z0, qn;
-    lane_z<VZ>(zc, lane, a.nZ, z0, qn);
-    const bool zok = qn > 0;
-    const size_t rs = (size_t)a.nA * a.nZ;
-    const int N = a.nY;
-    float acc[VZ];
-#pragma unroll
-    for (int e = 0; e < VZ; ++e) acc[e] = 0.f;
-    const float* __restrict__ bz = a.in + z0;
-    for (int th = 0; th < a.nA; ++th) {
-        const double4 tr = a.trig[th];
-        const double c = tr.x, s = tr.y;
-        const double ri = (double)i - tr.w, ci = (double)j - tr.z;
-        const double Jf = fma(-s, ri, c * ci), Kf = fma(c, ri, s * ci);
-        const int J0 = __double2int_rn(Jf), K0 = __double2int_rn(Kf);
-        const double row0 = fma(c, (double)K0, fma(-s, (double)J0, tr.w));
-        const double col0 = fma(s, (double)K0, fma(c, (double)J0, tr.z));
-        const float dr = (float)((double)i - row0), dc = (float)((double)j - col0);
-        const float sf = (float)s, cf = (float)c;
-#pragma unroll
-        for (int da = -1; da <= 1; ++da) {
-            const int J = J0 + da;
-            if ((unsigned)J >= (unsigned)a.nX) continue;
-            float s_entry = 0.f;
-            if (RAY) {
-                const float t = (float)(J - a.C);
-                if (fabsf(t) > a.R) continue;
-                s_entry = -sqrtf(a.R * a.R - t * t);
-            }
-            float W = 0.f;
-#pragma unroll
-            for (int db = -1; db <= 1; ++db) {
-                const int K = K0 + db;
-                if ((unsigned)K >= (unsigned)N) continue;
-                const float er = fmaf((float)da, sf, fmaf(-(float)db, cf, dr));
-                const float ec = fmaf(-(float)da, cf, fmaf(-(float)db, sf, dc));
-                float w = fmaxf(0.f, 1.f - fabsf(er)) * fmaxf(0.f, 1.f - fabsf(ec));
-                if (RAY) w *= ray_factor((float)(K - a.C), s_entry, a.alpha);
-                W += w;
-            }
-            if (W != 0.f && zok) {
-                float bv[VZ];
-                load_vz<VZ>(bz + (size_t)J * rs + (size_t)th * a.nZ, bv, qn);
-#pragma unroll
-                for (int e = 0; e < VZ; ++e) acc[e] = fmaf(W, bv[e], acc[e]);
-            }
-        }
-    }
-    if (!zok) return;
-    if (a.mask) {
-        const float m = __ldg(a.mask + p);
-#pragma unroll
-        for (int e = 0; e < VZ; ++e) acc[e] *= m;
-    }
-    store_vz<VZ>(a.out + (size_t)p * a.nZ + z0, acc, qn);
-}
-
-template <int VZ, bool RAY>
-__global__ void __launch_bounds__(256) k_adjoint_fast(Args a) {
-    k_adjoint_fast_body<VZ, RAY>(a, blockIdx.x, blockIdx.y);
-}
-
-// ---------------------------------------------------------------------------
 // R2 backprojection, fast path: 32 lanes along z with VZ floats each (one
 // pixel per warp, angles in sequence); same arithmetic as k_backward_ref.
 // ---------------------------------------------------------------------------
@@ -466,138 +386,6 @@ __device__ __forceinline__ void k_backward_fast_body(const Args& a, unsigned bx,
 template <int VZ, bool RAY>
 __global__ void __launch_bounds__(256) k_backward_fast(Args a) {
     k_backward_fast_body<VZ, RAY>(a, blockIdx.x, blockIdx.y);
-}
-
-// ---------------------------------------------------------------------------
-// Matched transpose from a weight table.
-//
-// k_adj_table evaluates, once per plan, for every pixel (i, j) and angle the
-// forward's own tap weights: the candidate lattice samples (J, K) around the
-// pixel's rotated position are evaluated with the forward's float64
-// coordinate expression and float32 weights, (1-dr)(1-dc) etc. times the RAY
-// factor, and summed per detector row J.  At most three rows J0-1..J0+1
-// touch a pixel (|J - J*| < |cos| + |sin| <= sqrt 2).  k_adjoint_table is then
-// a gather: per pixel and angle one 16-byte entry (broadcast over the warp)
-// and at most three sinogram rows.
-// ---------------------------------------------------------------------------
-template <bool RAY>
-__global__ void __launch_bounds__(256) k_adj_table(const double4* __restrict__ trig, float4* __restrict__ table, int nY,
-                                                   int nX, int nA, int C, float alpha, float R) {
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;   // over (pixel, angle), angle fastest
-    if (idx >= (long)nY * nX * nA) return;
-    const int th = (int)(idx % nA);
-    const long p = idx / nA;
-    const int i = (int)(p / nX), j = (int)(p % nX);
-    const double4 tr = trig[th];
-    const double c = tr.x, s = tr.y;
-    const double ri = (double)i - tr.w, ci = (double)j - tr.z;
-    const int J0 = __double2int_rn(fma(-s, ri, c * ci)), K0 = __double2int_rn(fma(c, ri, s * ci));
-    float W[3] = {0.f, 0.f, 0.f};
-    for (int da = -1; da <= 1; ++da) {
-        const int J = J0 + da;
-        if ((unsigned)J >= (unsigned)nX) continue;
-        float s_entry = 0.f;
-        if (RAY) {
-            const float t = (float)(J - C);
-            if (fabsf(t) > R) continue;
-            s_entry = -sqrtf(R * R - t * t);
-        }
-        const double rowb = fma(-s, (double)J, tr.w), colb = fma(c, (double)J, tr.z);
-        for (int db = -2; db <= 2; ++db) {
-            const int K = K0 + db;
-            if ((unsigned)K >= (unsigned)nY) continue;
-            const double row = fma(c, (double)K, rowb), col = fma(s, (double)K, colb);
-            const double fr = floor(row), fc = floor(col);
-            const int r0 = (int)fr, c0 = (int)fc;
-            const bool rc = row > fr, cc = col > fc;
-            if (!(i == r0 || (rc && i == r0 + 1))) continue;
-            if (!(j == c0 || (cc && j == c0 + 1))) continue;
-            const float dr = (float)(row - fr), dc = (float)(col - fc);
-            float w = ((i == r0) ? (1.f - dr) : dr) * ((j == c0) ? (1.f - dc) : dc);
-            if (RAY) w *= ray_factor((float)(K - C), s_entry, alpha);
-            W[da + 1] += w;
-        }
-    }
-    table[p * nA + th] = make_float4(__int_as_float(J0 - 1), W[0], W[1], W[2]);
-}
-
-template <int VZ>
-__device__ __forceinline__ void k_adjoint_table_body(const Args& a, const float4* __restrict__ table, unsigned bx, unsigned by) {
-    const int lane = threadIdx.x & 31;
-    const long item = (long)bx * kWarpsPerBlock + (threadIdx.x >> 5);
-    const int zc = (int)(item % a.zchunks);
-    const long p = item / a.zchunks;
-    if (p >= (long)a.nY * a.nX) return;
-    int z0, qn;
-    lane_z<VZ>(zc, lane, a.nZ, z0, qn);
-    if (qn == 0) return;
-    const size_t rs = (size_t)a.nA * a.nZ;
-    const float* __restrict__ bz = a.in + z0;
-    const float4* __restrict__ tp = table + p * a.nA;
-    float acc[VZ];
-#pragma unroll
-    for (int e = 0; e < VZ; ++e) acc[e] = 0.f;
-    if constexpr (VZ == 4) {
-        // four slices per lane: the rows of an angle and the next angle's entry in flight together
-        // (3.44 -> 3.09 ms at 256^3 x 360); with eight slices the extra row registers cost more
-        // occupancy than the overlap gains (2.17 -> 2.33 ms), so that instance reads row by row
-        float4 ent = __ldg(tp);
-#pragma unroll 1
-        for (int th = 0; th < a.nA; ++th) {
-            // the next angle's entry is in flight while this angle's rows are read
-            const float4 nxt = __ldg(tp + min(th + 1, a.nA - 1));
-            const int J = __float_as_int(ent.x);
-            const float w[3] = {ent.y, ent.z, ent.w};
-            const float* __restrict__ row = bz + (size_t)J * rs + (size_t)th * a.nZ;
-            // every row's loads are issued before any is consumed; a row of weight 0 is not read and its
-            // zeros leave the sums unchanged (fma(0, 0, s) == s: the sums are never -0), so the result
-            // equals summing the rows of nonzero weight in order
-            float bv[3][VZ];
-#pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                if (w[t] != 0.f) {
-                    load_vz<VZ>(row + (size_t)t * rs, bv[t], qn);
-                } else {
-#pragma unroll
-                    for (int e = 0; e < VZ; ++e) bv[t][e] = 0.f;
-                }
-            }
-#pragma unroll
-            for (int t = 0; t < 3; ++t)
-#pragma unroll
-                for (int e = 0; e < VZ; ++e) acc[e] = fmaf(w[t], bv[t][e], acc[e]);
-            ent = nxt;
-        }
-    } else {
-#pragma unroll 2
-        for (int th = 0; th < a.nA; ++th) {
-            const float4 ent = __ldg(tp + th);
-            const int J = __float_as_int(ent.x);
-            const float w[3] = {ent.y, ent.z, ent.w};
-#pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                if (w[t] != 0.f) {
-                    float bv[VZ];
-                    load_vz<VZ>(bz + (size_t)(J + t) * rs + (size_t)th * a.nZ, bv, qn);
-#pragma unroll
-                    for (int e = 0; e < VZ; ++e) acc[e] = fmaf(w[t], bv[e], acc[e]);
-                }
-            }
-        }
-    }
-    if (a.mask) {
-        const float m = __ldg(a.mask + p);
-#pragma unroll
-        for (int e = 0; e < VZ; ++e) acc[e] *= m;
-    }
-    store_vz<VZ>(a.out + (size_t)p * a.nZ + z0, acc, qn);
-}
-
-// eight resident CTAs per SM (32 registers, no spills): 2.17 -> 1.91 ms at 256^3 x 360 with eight
-// slices per lane, identical results
-template <int VZ>
-__global__ void __launch_bounds__(256, 8) k_adjoint_table(Args a, const float4* __restrict__ table) {
-    k_adjoint_table_body<VZ>(a, table, blockIdx.x, blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -844,7 +632,7 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
         for (int e = 0; e < NP; ++e) acc[q][e] = 0ull;
     const int pc = bcidx[blk];
     if (pc >= 0) {
-        const int rs = a.nA * a.nZ;
+        const int rs = a.nA * a.zs;
         const float* __restrict__ bz = a.in + z0;
         const int4* __restrict__ e = tab + (size_t)pc * a.nA * 2;
         const int nA = a.nA;
@@ -966,7 +754,10 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
         } else {
 #pragma unroll
             for (int q2 = 0; q2 < VZ / 4; ++q2)
-                if (q2 < qn)
+                if (!FULL && !a.whole) {  // (padded input rows: the output's are any length)
+                    for (int e2 = 0; e2 < 4; ++e2)
+                        if (128 * q2 + e2 < a.nZ - z0 && q2 < qn) __stcs(dst + 128 * q2 + e2, v[4 * q2 + e2]);
+                } else if (q2 < qn)
                     __stcs(reinterpret_cast<float4*>(dst + 128 * q2),
                            make_float4(v[4 * q2], v[4 * q2 + 1], v[4 * q2 + 2], v[4 * q2 + 3]));
         }
@@ -1408,14 +1199,14 @@ __device__ __forceinline__ void k_backward_ref_body(const Args& a, unsigned bx, 
     if (a.circle[p]) {
         const double X = (double)(j - a.C), Y = (double)(i - a.C);
         const double tlo = (double)(-a.C), thi = (double)(a.nY - 1 - a.C);
-        const size_t rs = (size_t)a.nA * a.nZ;  // sinogram row stride
+        const size_t rs = (size_t)a.nA * a.zs;  // sinogram row stride
         for (int th = kl; th < a.nA; th += LK) {
             const double4 tr = a.trig[th];
             const double t = __dsub_rn(__dmul_rn(X, tr.x), __dmul_rn(Y, tr.y));
             if (!(t >= tlo && t <= thi)) continue;  // np.interp left = right = 0
             const double ft = floor(t);
             const int j0 = (int)ft + a.C;
-            const float* b0 = a.in + (size_t)j0 * rs + (size_t)th * a.nZ + z0;
+            const float* b0 = a.in + (size_t)j0 * rs + (size_t)th * a.zs + z0;
             float v[VZ];
             if (zok) {
                 load_vec<VZ>(b0, v);
@@ -1467,7 +1258,15 @@ __device__ __forceinline__ void k_backward_ref_body(const Args& a, unsigned bx, 
 #pragma unroll
         for (int e = 0; e < VZ; ++e) acc[e] = m * acc[e];
     }
-    if (kl == 0 && zok) store_vec<VZ>(a.out + (size_t)p * a.nZ + z0, acc);
+    if (kl != 0 || !zok) return;
+    float* o = a.out + (size_t)p * a.nZ + z0;
+    if (VZ == 1 || a.whole) {
+        store_vec<VZ>(o, acc);
+    } else {  // (padded input rows: the output's are any length)
+#pragma unroll
+        for (int e = 0; e < VZ; ++e)
+            if (z0 + e < a.nZ) o[e] = acc[e];
+    }
 }
 
 template <int VZ, bool OCC, int ABS>
@@ -1731,7 +1530,7 @@ int fast_vz(int nZ, bool aligned, double min_eff) {
 // same body for many calls inside one persistent launch.  Both paths therefore
 // compute bit-identical results.
 // ---------------------------------------------------------------------------
-enum Kind : int { KF_FAST = 0, KF_GEN, KB_BATCHED, KB_FAST, KB_GEN, KA_TABLE, KA_FAST, KA_GEN, KF_2D, KB_2D, KB_BTABLE };
+enum Kind : int { KF_FAST = 0, KF_GEN, KB_BATCHED, KB_FAST, KB_GEN, KA_BLOCK, KA_GEN, KF_2D, KB_2D, KB_BTABLE };
 
 struct Item {
     int kind;
@@ -1752,7 +1551,6 @@ struct Item {
     int pre_w, pre_wp;
     Args a;
     FastArgs f;
-    const float4* table;
     const int4* btab4;  // KB_BTABLE: the plan's 2 x 2 block bin table and its block index
     const int* bcidx;
     int* status;       // the plan's status word (kernels with bounded waits record timeouts there)
@@ -1766,15 +1564,20 @@ bool image_tensor_map(const float* img, int nX, int nY, int row_stride, CUtensor
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 
 int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& it, const char* name,
-             bool noclip = false, bool in_batch = false) {
+             bool noclip = false, bool padded = false) {
     VAM_REQUIRE(plan && in && out, VAM_ERR_ARG, std::string(name) + ": null argument");
+    VAM_REQUIRE(!padded || (plan->nZ > 1 && !noclip), VAM_ERR_NOTSUP, std::string(name) + ": padded rows are not served here");
     VAM_REQUIRE(!noclip || plan->d_ones, VAM_ERR_ARG, std::string(name) + ": no all-ones circle table");
     std::memset(&it, 0, sizeof(it));
     it.cost = (long long)plan->nY * plan->nX * plan->nZ * plan->nA;
     it.family = op == Op::Forward ? 1 : (op == Op::BackwardRef ? 2 : 4);
     it.gy = 1;
+    // rows of the input padded to a multiple of four slices (vam_pad_rows): float4 loads for any slice count
+    const int zs = padded ? (plan->nZ + 3) & ~3 : plan->nZ;
+    const bool aligned16 = (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
+    const bool rows4 = zs % 4 == 0 && (((uintptr_t)in) & 15) == 0;
     // slices per lane: tuned (1 = generic kernel, 4 or 8 = fast kernel) or automatic (0)
-    const bool fast_ok = (((uintptr_t)in | (uintptr_t)out) & 31) == 0 && plan->nZ % 4 == 0;
+    const bool fast_ok = (((uintptr_t)in | (padded ? (uintptr_t)0 : (uintptr_t)out)) & 31) == 0 && zs % 4 == 0;
     const int want = op == Op::Forward ? plan->tune_fwd_vz : (op == Op::BackwardRef ? plan->tune_bwd_vz : plan->tune_adj_vz);
     int vzf = 0;
     if (fast_ok) {
@@ -1829,7 +1632,7 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     }
     // detector strips: every volume (any slice count, any alignment) without occlusion unless the generic
     // kernel is tuned (1).  Eight slices per lane where one 128-slice chunk does not hold the volume.
-    // 201^2 x 117 x 240 angles: 3.92 -> 0.37 ms against the generic kernel, which evaluates every sample's
+    // 201^2 x 117 x 240 angles: 3.92 -> 0.38 ms against the generic kernel, which evaluates every sample's
     // coordinates in float64 for one slice per lane.  With few slices the strips' weights are not shared
     // enough: at 122^2 x 440 angles the generic kernel takes 59 / 88 / 164 us with 4 / 8 / 12 slices (float4
     // rows) and 70 / 125 / 188 with 2 / 3 / 6 (single floats), the strips 86 / 88 / 88 and 98 / 99 / 102, and
@@ -1841,12 +1644,13 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         a.vol = in; a.sino = out; a.trig = plan->d_trig;
         a.mask = plan->abs_mode == VAM_ABS_MASK ? plan->d_mask : nullptr;
         a.nY = plan->nY; a.nX = plan->nX; a.nZ = plan->nZ; a.nA = plan->nA; a.C = plan->C;
+        a.vs = zs; a.whole = aligned16 && plan->nZ % 4 == 0;
         a.even = (plan->nY % 2) == 0;
         a.alpha = plan->abs_alpha; a.R = plan->abs_R;
         a.tasks = ray ? plan->d_tasks_single : plan->d_tasks_paired;
         a.ntasks = ray ? plan->nA : plan->n_tasks_paired;
         it.kind = KF_FAST; it.ray = ray;
-        it.vec = plan->nZ % 4 == 0 && (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
+        it.vec = rows4 && (padded || aligned16);
         it.vz = want == 4 || (want != 8 && plan->nZ <= 128) ? 4 : 8;
         a.lz_shift = 5;
         if (it.vz == 4)  // lanes to spare take other pixels
@@ -1860,12 +1664,34 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         it.once = a.mask;
         return VAM_OK;
     }
+    // pixel blocks for the matched transpose: as the strips
+    if (op == Op::Adjoint && !plan->has_occ && strips && want != 1 && (long)plan->nY * plan->nA < (1L << 32)) {
+        Args& a = it.a;
+        a.in = in; a.out = out; a.trig = plan->d_trig;
+        a.mask = plan->abs_mode == VAM_ABS_MASK ? plan->d_mask : nullptr;
+        a.nY = plan->nY; a.nX = plan->nX; a.nZ = plan->nZ; a.nA = plan->nA; a.C = plan->C;
+        a.alpha = plan->abs_alpha; a.R = plan->abs_R;
+        a.zs = zs; a.whole = aligned16 && plan->nZ % 4 == 0;
+        it.kind = KA_BLOCK; it.ray = ray;
+        it.vec = rows4 && (padded || aligned16);
+        it.vz = want == 4 || (want != 8 && plan->nZ <= 128) ? 4 : 8;
+        a.lz_shift = 5;
+        if (it.vz == 4)
+            while (a.lz_shift > 2 && (4 << (a.lz_shift - 1)) >= plan->nZ) --a.lz_shift;
+        const int per = it.vz << a.lz_shift;
+        a.zchunks = (plan->nZ + per - 1) / per;
+        it.gx = (unsigned)((long)((plan->nX + 7) / 8) * ((plan->nY + 3) / 4) * a.zchunks);
+        return VAM_OK;
+    }
     // the block-table backprojection serves every nZ % 4 == 0, also where the automatic width of the
     // computed-bin kernels would fall back to the generic kernel (too many idle lanes)
     const bool blk_ok = op == Op::BackwardRef && fast_ok && !ray && plan->d_bwd_btab && plan->tune_bwd_table;
-    if (op != Op::Forward && !plan->has_occ && (vzf || blk_ok) && !noclip &&
-        (long long)plan->nY * plan->nA * plan->nZ < (1LL << 31)) {
+    VAM_REQUIRE(!padded || (op == Op::BackwardRef && !plan->has_occ), VAM_ERR_NOTSUP,
+                std::string(name) + ": padded rows are not served here");
+    if (op == Op::BackwardRef && !plan->has_occ && (vzf || blk_ok) && !noclip &&
+        (long long)plan->nY * plan->nA * zs < (1LL << 31)) {
         Args& a = it.a;
+        a.zs = zs; a.whole = aligned16 && plan->nZ % 4 == 0;
         a.in = in; a.out = out; a.trig = plan->d_trig; a.circle = plan->d_circle;
         a.mask = plan->abs_mode == VAM_ABS_MASK ? plan->d_mask : nullptr;
         a.nY = plan->nY; a.nX = plan->nX; a.nZ = plan->nZ; a.nA = plan->nA; a.C = plan->C;
@@ -1875,49 +1701,42 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         const long items = (long)plan->nY * plan->nX * a.zchunks;
         it.gx = (unsigned)((items + kWarpsPerBlock - 1) / kWarpsPerBlock);
         it.vz = vzf; it.ray = ray;
-        if (op == Op::BackwardRef) {
-            // the batched kernel stages cos / sin of every angle in shared memory (16 B per angle)
-            const int batch = (size_t)plan->nA * sizeof(double2) <= 48 * 1024 ? plan->tune_bwd_batch : 1;
-            if (blk_ok) {
-                // the 2 x 2 block table: slices per lane as tuned (4 or 8), else eight for full 256-slice
-                // chunks, six / five for full 192- / 160-slice chunks, eight from 160 slices up, four below
-                // (256^3 x 360: 0.92 / 1.41 ms with 8 / 4; 192^3 x 720: 1.46 / 1.94; 96^3 x 720: 0.42 / 0.31)
-                int bvz = 4;
-                if (plan->tune_bwd_vz == 8 || plan->tune_bwd_vz == 4) bvz = plan->tune_bwd_vz;
-                else if (plan->nZ % 256 == 0) bvz = 8;
-                else if (plan->nZ % 192 == 0) bvz = 6;
-                else if (plan->nZ % 160 == 0) bvz = 5;
-                else if (plan->nZ >= 160) bvz = 8;
-                it.kind = KB_BTABLE;
-                it.vz = bvz;
-                a.zchunks = (plan->nZ + 32 * bvz - 1) / (32 * bvz);
-                const long ntx = ((plan->nX + 1) / 2 + 3) / 4, nty = ((plan->nY + 1) / 2 + 1) / 2;
-                it.gx = (unsigned)(ntx * nty * a.zchunks);
-                it.btab4 = plan->d_bwd_btab;
-                it.bcidx = plan->d_bwd_bcidx;
-            } else if (batch >= 2) {
-                it.kind = KB_BATCHED;
-                it.batch = vzf == 8 ? 2 : (batch >= 4 ? 4 : 2);
-                it.smem = (unsigned)(sizeof(double2) * plan->nA);
-            } else {
-                it.kind = KB_FAST;
-            }
-        } else if (plan->d_adj_table && plan->adj_table_abs == plan->abs_mode && plan->tune_adj_table) {
-            it.kind = KA_TABLE;
-            it.table = plan->d_adj_table;
+        // the batched kernel stages cos / sin of every angle in shared memory (16 B per angle)
+        const int batch = (size_t)plan->nA * sizeof(double2) <= 48 * 1024 ? plan->tune_bwd_batch : 1;
+        if (blk_ok) {
+            // the 2 x 2 block table: slices per lane as tuned (4 or 8), else eight for full 256-slice
+            // chunks, six / five for full 192- / 160-slice chunks, eight from 160 slices up, four below
+            // (256^3 x 360: 0.92 / 1.41 ms with 8 / 4; 192^3 x 720: 1.46 / 1.94; 96^3 x 720: 0.42 / 0.31)
+            int bvz = 4;
+            if (plan->tune_bwd_vz == 8 || plan->tune_bwd_vz == 4) bvz = plan->tune_bwd_vz;
+            else if (plan->nZ % 256 == 0) bvz = 8;
+            else if (plan->nZ % 192 == 0) bvz = 6;
+            else if (plan->nZ % 160 == 0) bvz = 5;
+            else if (plan->nZ >= 160) bvz = 8;
+            it.kind = KB_BTABLE;
+            it.vz = bvz;
+            a.zchunks = (plan->nZ + 32 * bvz - 1) / (32 * bvz);
+            const long ntx = ((plan->nX + 1) / 2 + 3) / 4, nty = ((plan->nY + 1) / 2 + 1) / 2;
+            it.gx = (unsigned)(ntx * nty * a.zchunks);
+            it.btab4 = plan->d_bwd_btab;
+            it.bcidx = plan->d_bwd_bcidx;
+        } else if (batch >= 2) {
+            it.kind = KB_BATCHED;
+            it.batch = vzf == 8 ? 2 : (batch >= 4 ? 4 : 2);
+            it.smem = (unsigned)(sizeof(double2) * plan->nA);
         } else {
-            it.kind = KA_FAST;
+            it.kind = KB_FAST;
         }
         return VAM_OK;
     }
-    const bool aligned = (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
-    Layout L = choose_layout(plan->nZ, aligned);
+    Layout L = choose_layout(zs, padded ? rows4 : aligned16);
     Args& a = it.a;
     a.in = in; a.out = out; a.trig = plan->d_trig; a.circle = noclip ? plan->d_ones : plan->d_circle;
     a.mask = plan->d_mask; a.occ = plan->d_occ; a.occ_flag = plan->d_occ_flag;
     a.occ64 = plan->d_occ64; a.occ_mode = plan->has_occ ? plan->occ_mode : 0;
     a.nY = plan->nY; a.nX = plan->nX; a.nZ = plan->nZ; a.nA = plan->nA; a.C = plan->C;
     a.lz_shift = L.lz_shift; a.zvec = L.zvec; a.zchunks = L.zchunks;
+    a.zs = zs; a.whole = aligned16 && plan->nZ % 4 == 0;
     a.alpha = plan->abs_alpha; a.R = plan->abs_R;
     const long items = (op == Op::Forward) ? (long)plan->nX * L.zchunks : (long)plan->nY * plan->nX * L.zchunks;
     it.kind = op == Op::Forward ? KF_GEN : (op == Op::BackwardRef ? KB_GEN : KA_GEN);
@@ -1994,10 +1813,10 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
         }
     }
     if constexpr ((FAM & 4) != 0) {
-        if (it.kind == KA_FAST) {
+        if (it.kind == KA_BLOCK) {
             const Args a = it.a;
-            if (it.vz == 8) k_adjoint_fast_body<8, RAY>(a, bx, by);
-            else k_adjoint_fast_body<4, RAY>(a, bx, by);
+            if (it.vz == 8) { if (it.vec) adjoint_block_body<2, true, RAY>(a, bx); else adjoint_block_body<2, false, RAY>(a, bx); }
+            else { if (it.vec) adjoint_block_body<1, true, RAY>(a, bx); else adjoint_block_body<1, false, RAY>(a, bx); }
         }
     }
 }
@@ -2027,12 +1846,6 @@ __device__ __forceinline__ void item_body(const Item& it, unsigned bx, unsigned 
         } else if constexpr ((FAM & (4 | 8 | 16)) != 0) {
             if (it.vz == 4) { if (it.occ) gen_body_fam<FAM, 4, true>(it, bx, by); else gen_body_fam<FAM, 4, false>(it, bx, by); }
             else { if (it.occ) gen_body_fam<FAM, 1, true>(it, bx, by); else gen_body_fam<FAM, 1, false>(it, bx, by); }
-        }
-    } else if (it.kind == KA_TABLE) {
-        if constexpr ((FAM & 4) != 0) {
-            const Args a = it.a;
-            if (it.vz == 8) k_adjoint_table_body<8>(a, it.table, bx, by);
-            else k_adjoint_table_body<4>(a, it.table, bx, by);
         }
     } else if (it.ray) {
         if constexpr (FAM != 2) fast_body<FAM, true>(it, bx, by);   // nor a per-ray absorption body
@@ -2112,9 +1925,9 @@ void launch_fast(const Item& it, dim3 grid, cudaStream_t st) {
             if (it.vz == 8) k_backward_fast<8, RAY><<<grid, block, 0, st>>>(it.a);
             else k_backward_fast<4, RAY><<<grid, block, 0, st>>>(it.a);
             break;
-        case KA_FAST:
-            if (it.vz == 8) k_adjoint_fast<8, RAY><<<grid, block, 0, st>>>(it.a);
-            else k_adjoint_fast<4, RAY><<<grid, block, 0, st>>>(it.a);
+        case KA_BLOCK:
+            if (it.vz == 8) { if (it.vec) k_adjoint_block<2, true, RAY><<<grid, block, 0, st>>>(it.a); else k_adjoint_block<2, false, RAY><<<grid, block, 0, st>>>(it.a); }
+            else { if (it.vec) k_adjoint_block<1, true, RAY><<<grid, block, 0, st>>>(it.a); else k_adjoint_block<1, false, RAY><<<grid, block, 0, st>>>(it.a); }
             break;
         default: break;
     }
@@ -2135,10 +1948,6 @@ int launch_item(const Item& it, cudaStream_t st, const char* name) {
     if (it.kind == KF_GEN || it.kind == KB_GEN || it.kind == KA_GEN) {
         if (it.vz == 4) { if (it.occ) launch_gen2<4, true>(it, grid, st); else launch_gen2<4, false>(it, grid, st); }
         else { if (it.occ) launch_gen2<1, true>(it, grid, st); else launch_gen2<1, false>(it, grid, st); }
-    } else if (it.kind == KA_TABLE) {
-        const dim3 block(kWarpsPerBlock * kWarp);
-        if (it.vz == 8) k_adjoint_table<8><<<grid, block, 0, st>>>(it.a, it.table);
-        else k_adjoint_table<4><<<grid, block, 0, st>>>(it.a, it.table);
     } else if (it.kind == KB_BTABLE) {
         const dim3 block(kWarpsPerBlock * kWarp);
         const bool full = it.a.nZ % (32 * it.vz) == 0;
@@ -2163,12 +1972,12 @@ int launch_item(const Item& it, cudaStream_t st, const char* name) {
 }
 
 int run(vam_parallel_plan* plan, Op op, const float* in, float* out, cudaStream_t st, const char* name,
-        bool noclip = false) {
+        bool noclip = false, bool padded = false) {
     VAM_REQUIRE(plan, VAM_ERR_ARG, std::string(name) + ": null argument");
     DeviceGuard g(plan->device);
     VAM_REQUIRE(g.ok, VAM_ERR_CUDA, std::string(name) + ": cannot select device");
     Item it;
-    const int rc = describe(plan, op, in, out, it, name, noclip);
+    const int rc = describe(plan, op, in, out, it, name, noclip, padded);
     if (rc != VAM_OK) return rc;
     return launch_item(it, st, name);
 }
@@ -2319,7 +2128,6 @@ extern "C" int vam_parallel_plan_create(const vam_parallel_geom* geom, vam_paral
     p->nY = geom->n_y; p->nX = geom->n_x; p->nZ = geom->n_z; p->nA = geom->n_angles;
     p->C = geom->n_y / 2;
     p->device = geom->device;
-    p->adj_table_abs = -1;
     p->tune_bwd_batch = 2;
     p->tune_adj_table = 1;
     p->tune_bwd_table = 1;
@@ -2398,7 +2206,6 @@ extern "C" int vam_parallel_plan_destroy(vam_parallel_plan* p) {
     cudaFree(p->d_tasks_paired);
     cudaFree(p->d_tasks_single);
     cudaFree(p->d_vol_scratch);
-    cudaFree(p->d_adj_table);
     cudaFree(p->d_bwd_cidx);
     cudaFree(p->d_status);
     cudaFree(p->d_img_pad);
@@ -2556,18 +2363,8 @@ extern "C" int vam_parallel_get_tuning(vam_parallel_plan* p, vam_parallel_tuning
 
 extern "C" int vam_parallel_prepare_adjoint(vam_parallel_plan* p, vam_stream_t stream) {
     clear_error();
+    (void)stream;
     VAM_REQUIRE(p, VAM_ERR_ARG, "vam_parallel_prepare_adjoint: null plan");
-    DeviceGuard g(p->device);
-    const size_t n = (size_t)p->nY * p->nX * p->nA;
-    if (!p->d_adj_table) VAM_TRY_CUDA(cudaMalloc(&p->d_adj_table, sizeof(float4) * n));
-    cudaStream_t st = (cudaStream_t)stream;
-    const unsigned nb = (unsigned)((n + 255) / 256);
-    if (p->abs_mode == VAM_ABS_RAY)
-        k_adj_table<true><<<nb, 256, 0, st>>>(p->d_trig, p->d_adj_table, p->nY, p->nX, p->nA, p->C, p->abs_alpha, p->abs_R);
-    else
-        k_adj_table<false><<<nb, 256, 0, st>>>(p->d_trig, p->d_adj_table, p->nY, p->nX, p->nA, p->C, 0.f, 0.f);
-    VAM_CHECK_LAUNCH("k_adj_table");
-    p->adj_table_abs = p->abs_mode;
     return VAM_OK;
 }
 
@@ -2582,6 +2379,8 @@ extern "C" int vam_parallel_status(vam_parallel_plan* p, int32_t* status) {
     return VAM_OK;
 }
 
+static int prepare_backward(vam_parallel_plan* p, int zs, cudaStream_t st);
+
 extern "C" int vam_parallel_prepare_backward(vam_parallel_plan* p, vam_stream_t stream) {
     clear_error();
     VAM_REQUIRE(p, VAM_ERR_ARG, "vam_parallel_prepare_backward: null plan");
@@ -2589,6 +2388,20 @@ extern "C" int vam_parallel_prepare_backward(vam_parallel_plan* p, vam_stream_t 
                 "vam_parallel_prepare_backward: the table holds 32-bit sinogram offsets (sinogram below 2^31 elements)");
     VAM_REQUIRE(p->nZ % 4 == 0, VAM_ERR_NOTSUP,
                 "vam_parallel_prepare_backward: the table kernel runs four-slice vectors (nZ % 4 == 0)");
+    return prepare_backward(p, p->nZ, (cudaStream_t)stream);
+}
+
+extern "C" int vam_parallel_prepare_padded(vam_parallel_plan* p, vam_stream_t stream) {
+    clear_error();
+    VAM_REQUIRE(p, VAM_ERR_ARG, "vam_parallel_prepare_padded: null plan");
+    const int zs = (p->nZ + 3) & ~3;
+    VAM_REQUIRE(p->nZ > 1 && (long long)p->nY * p->nA * zs < (1LL << 31), VAM_ERR_NOTSUP,
+                "vam_parallel_prepare_padded: a single slice, or a sinogram of 2^31 elements or more");
+    return prepare_backward(p, zs, (cudaStream_t)stream);
+}
+
+// the block table for sinogram rows zs floats apart
+static int prepare_backward(vam_parallel_plan* p, int zs, cudaStream_t st) {
     DeviceGuard g(p->device);
     const int n = p->nY * p->nX;
     // the clip circle exactly as the plan's table (linspace(-1, 1) semantics)
@@ -2615,7 +2428,6 @@ extern "C" int vam_parallel_prepare_backward(vam_parallel_plan* p, vam_stream_t 
             if (any) { bcidx[(size_t)bi * nbx + bj] = (int)blist.size(); blist.push_back(bi * nbx + bj); }
         }
     const int nbc = (int)blist.size();
-    cudaStream_t st = (cudaStream_t)stream;
     if (!p->d_bwd_cidx) VAM_TRY_CUDA(cudaMalloc(&p->d_bwd_cidx, sizeof(int) * n));
     if (!p->d_bwd_bcidx) VAM_TRY_CUDA(cudaMalloc(&p->d_bwd_bcidx, sizeof(int) * bcidx.size()));
     if (!p->d_bwd_btab) VAM_TRY_CUDA(cudaMalloc(&p->d_bwd_btab, sizeof(int4) * 2 * (size_t)std::max(nbc, 1) * p->nA));
@@ -2628,7 +2440,7 @@ extern "C" int vam_parallel_prepare_backward(vam_parallel_plan* p, vam_stream_t 
     if (e == cudaSuccess && nbc) {
         const long tot = (long)nbc * p->nA;
         k_bwd_btable<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(p->d_trig, d_blist, p->d_bwd_cidx, p->d_bwd_btab,
-                                                                    nbc, p->nA, p->nY, p->nX, p->nZ, p->C);
+                                                                    nbc, p->nA, p->nY, p->nX, zs, p->C);
         e = cudaGetLastError();
     }
     // the host vectors and the block list are released after the copies and the build complete
@@ -2637,6 +2449,48 @@ extern "C" int vam_parallel_prepare_backward(vam_parallel_plan* p, vam_stream_t 
     if (e != cudaSuccess)
         return set_error(VAM_ERR_CUDA, std::string("vam_parallel_prepare_backward: ") + cudaGetErrorString(e));
     return VAM_OK;
+}
+
+// out[row] = x[row] and zeros up to the next multiple of four.  A thread per float4 of the output; bound by
+// memory: 201^2 rows of 117 floats (38 MB in and out) 13 us.
+namespace vam {
+namespace {
+__global__ void __launch_bounds__(256) k_pad_rows(const float* __restrict__ x, float4* __restrict__ out, long long n4,
+                                                  int nz, int nz4) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+        const long long row = i / nz4;
+        const int z = 4 * (int)(i - row * nz4);
+        const float* p = x + row * nz + z;
+        float4 v;
+        v.x = __ldg(p);
+        v.y = z + 1 < nz ? __ldg(p + 1) : 0.f;
+        v.z = z + 2 < nz ? __ldg(p + 2) : 0.f;
+        v.w = z + 3 < nz ? __ldg(p + 3) : 0.f;
+        out[i] = v;
+    }
+}
+}  // namespace
+}  // namespace vam
+
+extern "C" int vam_pad_rows(const float* x, int64_t rows, int32_t nz, float* out, vam_stream_t stream) {
+    clear_error();
+    VAM_REQUIRE(x && out, VAM_ERR_ARG, "vam_pad_rows: null argument");
+    VAM_REQUIRE(rows > 0 && nz > 0, VAM_ERR_SHAPE, "vam_pad_rows: rows and nz must be positive");
+    VAM_REQUIRE((((uintptr_t)out) & 15) == 0, VAM_ERR_ARG, "vam_pad_rows: out must be 16-byte aligned");
+    const int nz4 = (nz + 3) / 4;
+    const long long n4 = (long long)rows * nz4;
+    k_pad_rows<<<(unsigned)std::min<long long>((n4 + 255) / 256, 148LL * 32), 256, 0, (cudaStream_t)stream>>>(
+        x, reinterpret_cast<float4*>(out), n4, nz, nz4);
+    VAM_CHECK_LAUNCH("vam_pad_rows");
+    return VAM_OK;
+}
+
+extern "C" int vam_parallel_apply_padded(vam_parallel_plan* p, int32_t op, const float* in, float* out,
+                                         vam_stream_t stream) {
+    clear_error();
+    VAM_REQUIRE(op >= VAM_OP_FORWARD && op <= VAM_OP_ADJOINT, VAM_ERR_ARG, "vam_parallel_apply_padded: unknown op");
+    const Op o = op == VAM_OP_FORWARD ? Op::Forward : (op == VAM_OP_BACKWARD_REF ? Op::BackwardRef : Op::Adjoint);
+    return run(p, o, in, out, (cudaStream_t)stream, "vam_parallel_apply_padded", false, true);
 }
 
 extern "C" int vam_parallel_forward(vam_parallel_plan* p, const float* vol, float* sino, vam_stream_t stream) {
@@ -2788,8 +2642,7 @@ double time_weight(const Item& it) {
         case KB_BATCHED: case KB_FAST: return 1.2;
         case KB_BTABLE: return 0.7;
         case KB_GEN: return slice ? 10.0 : 2.0;
-        case KA_TABLE: return 1.5;
-        case KA_FAST: return 3.5;
+        case KA_BLOCK: return 1.2;
         case KF_2D: return 4.0;
         case KB_2D: return 2.0;
         default: return slice ? 27.0 : 4.0;
@@ -2804,9 +2657,10 @@ int batch_prepare(vam_batch* b, const vam_work* work, int32_t n) {
         const vam_work& w = work[i];
         VAM_REQUIRE(w.plan, VAM_ERR_ARG, "vam_batch: work item without a plan");
         VAM_REQUIRE(w.plan->device == b->device, VAM_ERR_ARG, "vam_batch: plan on another device than the batch");
-        VAM_REQUIRE(w.op >= VAM_OP_FORWARD && w.op <= VAM_OP_ADJOINT, VAM_ERR_ARG, "vam_batch: unknown op");
-        const Op op = w.op == VAM_OP_FORWARD ? Op::Forward : (w.op == VAM_OP_BACKWARD_REF ? Op::BackwardRef : Op::Adjoint);
-        const int rc = describe(w.plan, op, w.in, w.out, items[i], "vam_batch", false, true);
+        const int wop = w.op & ~VAM_OP_PADDED;
+        VAM_REQUIRE(wop >= VAM_OP_FORWARD && wop <= VAM_OP_ADJOINT, VAM_ERR_ARG, "vam_batch: unknown op");
+        const Op op = wop == VAM_OP_FORWARD ? Op::Forward : (wop == VAM_OP_BACKWARD_REF ? Op::BackwardRef : Op::Adjoint);
+        const int rc = describe(w.plan, op, w.in, w.out, items[i], "vam_batch", false, (w.op & VAM_OP_PADDED) != 0);
         if (rc != VAM_OK) return rc;
         const Item& d = items[i];
         // generic bodies with occlusion or per-ray absorption, and per-ray fast backprojections, go

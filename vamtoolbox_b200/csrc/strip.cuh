@@ -64,6 +64,8 @@ struct FastArgs {
     const int2* tasks;
     const float* mask;  // per-pixel factor of the volume, or null
     int nY, nX, nZ, nA, C;
+    int vs;          // floats from one pixel's row to the next (nZ, or nZ rounded up to four: padded rows)
+    int whole;       // the output's rows take float4 stores
     int ntasks;
     int zchunks;
     int lz_shift;    // log2 of the lanes along z (a warp's other lanes take other pixels)
@@ -100,12 +102,26 @@ __device__ __forceinline__ void fma_pairs(unsigned long long& acc, unsigned long
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(w2), "l"(v2));
 }
 
+// whole: the float4s may be stored as such; otherwise slice by slice, the first `left` of them (those the
+// output has: a padded row holds up to three more)
 template <int Q, bool VEC>
-__device__ __forceinline__ void strip_store(float* __restrict__ p, const unsigned long long (&v)[2 * Q], int n, int lz) {
+__device__ __forceinline__ void strip_store(float* __restrict__ p, const unsigned long long (&v)[2 * Q], int n, int lz,
+                                            int whole, int left) {
     if constexpr (VEC) {
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
-            if (q < n) *reinterpret_cast<ulonglong2*>(p + 128 * q) = make_ulonglong2(v[2 * q], v[2 * q + 1]);
+        for (int q = 0; q < Q; ++q) {
+            if (q >= n) break;
+            if (whole) {
+                *reinterpret_cast<ulonglong2*>(p + 128 * q) = make_ulonglong2(v[2 * q], v[2 * q + 1]);
+                continue;
+            }
+            float x[4];
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(x[0]), "=f"(x[1]) : "l"(v[2 * q]));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(x[2]), "=f"(x[3]) : "l"(v[2 * q + 1]));
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (128 * q + e < left) p[128 * q + e] = x[e];
+        }
     } else {
         const int st = Q == 2 ? 32 : lz;
 #pragma unroll
@@ -135,7 +151,7 @@ __device__ __forceinline__ void strip_sample(const FastArgs& a, const float* __r
         const unsigned p = (unsigned)r * (unsigned)a.nX + (unsigned)c;
         if (a.mask) w *= __ldg(a.mask + p);
         unsigned long long v[2 * Q];
-        strip_load<Q, VEC>(volz + (size_t)p * a.nZ, v, n, lz);
+        strip_load<Q, VEC>(volz + (size_t)p * a.vs, v, n, lz);
 #pragma unroll
         for (int e = 0; e < 2 * Q; ++e) fma_pairs(acc[e], pk_pair(w, w), v[e]);
     }
@@ -152,8 +168,8 @@ __device__ __forceinline__ void strip_finish(const FastArgs& a, int2 task, bool 
     float* const here = a.sino + ((size_t)j * a.nA + task.x) * a.nZ + z0;
     float* const there = a.sino + ((size_t)(2 * a.C - j) * a.nA + task.y) * a.nZ + z0;
     if (!ext) {
-        strip_store<Q, VEC>(here, sum, n, lz);
-        if (task.y >= 0) strip_store<Q, VEC>(there, sum, n, lz);
+        strip_store<Q, VEC>(here, sum, n, lz, a.whole, a.nZ - z0);
+        if (task.y >= 0) strip_store<Q, VEC>(there, sum, n, lz, a.whole, a.nZ - z0);
         return;
     }
     const double4 tr = a.trig[task.x];
@@ -164,11 +180,11 @@ __device__ __forceinline__ void strip_finish(const FastArgs& a, int2 task, bool 
 #pragma unroll
         for (int e = 0; e < 2 * Q; ++e) o[e] = sum[e];
         strip_sample<Q, VEC>(a, volz, rowb, colb, o, n, lz);
-        strip_store<Q, VEC>(here, o, n, lz);
+        strip_store<Q, VEC>(here, o, n, lz, a.whole, a.nZ - z0);
     }
     if (j > 0) {
         strip_sample<Q, VEC>(a, volz, fma(tr.x, (double)N, rowb), fma(tr.y, (double)N, colb), sum, n, lz);
-        strip_store<Q, VEC>(there, sum, n, lz);
+        strip_store<Q, VEC>(there, sum, n, lz, a.whole, a.nZ - z0);
     }
 }
 
@@ -245,7 +261,7 @@ __device__ __forceinline__ void forward_strip_body(const FastArgs& a, unsigned b
     auto rows = [&](const float4 (&t)[U], unsigned long long (&v)[U][VZ / 2]) {
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            strip_load<Q, VEC>(volz + (size_t)__float_as_uint(t[u].w) * (unsigned)a.nZ, v[u], n, LZ);
+            strip_load<Q, VEC>(volz + (size_t)__float_as_uint(t[u].w) * (unsigned)a.vs, v[u], n, LZ);
     };
     auto add1 = [&](const float4& t, const unsigned long long (&v)[VZ / 2]) {
         const float w[3] = {t.x, t.y, t.z};
@@ -471,6 +487,274 @@ __device__ __noinline__ void forward_strip_samples(const FastArgs& a, unsigned b
 template <int Q, bool VEC, bool RAY>
 __global__ void __launch_bounds__(256, 2) k_forward_strip(FastArgs a) {
     forward_strip_body<Q, VEC, RAY>(a, blockIdx.x, blockIdx.y);
+}
+
+// ---------------------------------------------------------------------------
+// Matched transpose by pixel blocks.
+//
+// One warp owns a 2 x 2 block of pixels over the slices of one z chunk.  Detector bin j of an angle gives
+// pixel p W(j, p) times its row, W the strip forward's weights (every sample k of the bin with the pixel under
+// its bilinear kernel), so the block needs the at most five bins within 1.5 (|cos| + |sin|) of its centre, 3.6
+// on average, where a pixel alone needs 2.3: 0.9 rows per pixel and angle.  The warp lists the rows of six
+// angles at a time (lanes: angle x bin), weights for the four pixels, and works the ring off like the strips.
+// ---------------------------------------------------------------------------
+constexpr int kBlockBins = 5;
+
+struct BlockRing {
+    float4 w[kWarpsPerBlock][kStripRing];    // the four pixels' weights
+    unsigned o[kWarpsPerBlock][kStripRing];  // the row: bin * angles + angle
+};
+
+__device__ __forceinline__ BlockRing& block_ring() {
+    __shared__ __align__(16) BlockRing r;
+    return r;
+}
+
+// The warp's block (its first pixel), lane's first slice and number of slices (float4s), false when idle.  A
+// thread block covers 4 x 2 blocks of one z chunk, whose warps read the same rows at about the same time.
+template <int Q, bool VEC>
+__device__ __forceinline__ bool block_place(const Args& a, unsigned bx, int& i, int& j, int& z0, int& n) {
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, LZ = 1 << a.lz_shift;
+    const unsigned tile = bx / (unsigned)a.zchunks, ntx = (unsigned)((a.nX + 7) >> 3);
+    i = 2 * (int)(tile / ntx * 2 + (wp >> 2));
+    j = 2 * (int)(tile % ntx * 4 + (wp & 3));
+    if (i >= a.nY || j >= a.nX) return false;
+    constexpr int per = VEC ? 4 : 1;
+    z0 = (int)(bx % (unsigned)a.zchunks) * LZ * 4 * Q + per * (lane & (LZ - 1));
+    n = 0;
+#pragma unroll
+    for (int e = 0; e < 4 * Q / per; ++e) n += z0 + per * LZ * e < a.nZ ? 1 : 0;
+    if (n == 0) z0 = 0;
+    return true;
+}
+
+// Weight of bin J for the pixel at lattice position (J0 + dj, K0 + dk): its samples within one pixel of it.
+template <bool RAY>
+__device__ __forceinline__ float bin_weight(const Args& a, float cf, float sf, float d, float dk, float K0, float sent) {
+    const float kc = rintf(dk);
+    float w = 0.f;
+#pragma unroll
+    for (int b = -1; b <= 1; ++b) {
+        const float k = K0 + (kc + (float)b);
+        const float kk = (k >= 0.f && k <= (float)(a.nY - 1)) ? (kc + (float)b) - dk : 1e9f;  // outside: no weight
+        float h = __saturatef(1.f - fabsf(fmaf(cf, kk, -sf * d))) * __saturatef(1.f - fabsf(fmaf(sf, kk, cf * d)));
+        if (RAY && h != 0.f) h *= ray_factor(k - (float)a.C, sent, a.alpha);
+        w += h;
+    }
+    return w;
+}
+
+template <int Q, bool VEC, bool RAY>
+__device__ __noinline__ void adjoint_block_rows(const Args& a, unsigned bx);
+
+template <int Q, bool VEC, bool RAY>
+__device__ __forceinline__ void adjoint_block_body(const Args& a, unsigned bx) {
+    constexpr int U = Q == 2 ? 2 : 4, VZ = 4 * Q, R = 32 / kBlockBins;
+    BlockRing& ring = block_ring();
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    int i0, j0, z0, n;
+    if (!block_place<Q, VEC>(a, bx, i0, j0, z0, n)) return;  // uniform per warp
+    const int LZ = 1 << a.lz_shift, g = lane >> a.lz_shift, G = 32 >> a.lz_shift;
+    const float* __restrict__ bz = a.in + z0;
+
+    unsigned long long acc[4][VZ / 2];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int e = 0; e < VZ / 2; ++e) acc[q][e] = 0ull;
+    auto entries = [&](int at, float4 (&t)[U], unsigned (&o)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            t[u] = ring.w[wp][at + u];
+            o[u] = ring.o[wp][at + u];
+        }
+    };
+    auto rows = [&](const unsigned (&o)[U], unsigned long long (&v)[U][VZ / 2]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) strip_load<Q, VEC>(bz + (size_t)o[u] * (unsigned)a.zs, v[u], n, LZ);
+    };
+    auto add1 = [&](const float4& t, const unsigned long long (&v)[VZ / 2]) {
+        const float w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int e = 0; e < VZ / 2; ++e) fma_pairs(acc[q][e], pk_pair(w[q], w[q]), v[e]);
+    };
+    auto step = [&](int at, float4 (&tn)[U], unsigned long long (&vn)[U][VZ / 2], const float4 (&tc)[U],
+                    const unsigned long long (&vc)[U][VZ / 2]) {
+        unsigned o[U];
+        entries(at, tn, o);
+        add1(tc[0], vc[0]);
+        rows(o, vn);
+#pragma unroll
+        for (int u = 1; u < U; ++u) add1(tc[u], vc[u]);
+    };
+    float4 t0[U], t1[U];
+    unsigned long long v0[U][VZ / 2], v1[U][VZ / 2];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        t0[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int e = 0; e < VZ / 2; ++e) v0[u][e] = 0ull;
+    }
+    const int round = 2 * U * G, size = kStripRing - kStripRing % round;  // whole rounds: a group never wraps
+    int head = 0, tail = 0, wait = 0;
+    const int la = lane / kBlockBins, slot = lane - la * kBlockBins;
+    for (int th0 = 0; th0 < a.nA; th0 += R) {
+        const int th = th0 + la;
+        float W[4] = {0.f, 0.f, 0.f, 0.f};
+        unsigned row = 0;
+        bool listed = false;
+        if (la < R && th < a.nA) {
+            const double4 tr = a.trig[th];
+            const double ri = (double)i0 - tr.w, ci = (double)j0 - tr.z;
+            const double Jf = fma(-tr.y, ri, tr.x * ci), Kf = fma(tr.x, ri, tr.y * ci);
+            const double Jn = rint(Jf), Kn = rint(Kf);
+            const float cf = (float)tr.x, sf = (float)tr.y, dj = (float)(Jf - Jn), dk = (float)(Kf - Kn);
+            // bins from 1.5 (|cos| + |sin|) below the block's centre on
+            const float lo = dj + 0.5f * (cf - sf) - 1.5f * (fabsf(cf) + fabsf(sf));
+            const float jr = ceilf(lo - 1e-5f) + (float)slot;  // the bin, from Jn
+            const int J = (int)Jn + (int)jr;
+            float sent = 0.f;
+            bool lit = (unsigned)J < (unsigned)a.nX;
+            if (RAY) {
+                const float t = (float)(J - a.C);
+                if (fabsf(t) > a.R) lit = false;
+                else sent = -sqrtf(a.R * a.R - t * t);
+            }
+            if (lit) {
+                row = (unsigned)J * (unsigned)a.nA + (unsigned)th;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float pr = (float)(q >> 1), pc = (float)(q & 1);  // the pixel, from the block's first
+                    const float d = jr - (dj + (pc * cf - pr * sf)), k = dk + (pr * cf + pc * sf);
+                    W[q] = bin_weight<RAY>(a, cf, sf, d, k, (float)Kn, sent);
+                    listed |= W[q] != 0.f;
+                }
+            }
+        }
+        const unsigned has = __ballot_sync(kFull, listed);
+        if (listed) {
+            int at = tail + __popc(has & ((1u << lane) - 1u));
+            at = at < size ? at : at - size;
+            ring.w[wp][at] = make_float4(W[0], W[1], W[2], W[3]);
+            ring.o[wp][at] = row;
+        }
+        const int cnt = __popc(has);
+        tail = tail + cnt < size ? tail + cnt : tail + cnt - size;
+        wait += cnt;
+        __syncwarp();
+        for (; wait >= round; wait -= round) {
+            step(head + g * U, t1, v1, t0, v0);
+            step(head + U * G + g * U, t0, v0, t1, v1);
+            head = head + round < size ? head + round : 0;
+        }
+        __syncwarp();  // the entries worked off are free again
+    }
+    if (wait > 0) {  // the rest, filled up with entries of no weight (and the first row)
+        for (int k = wait + lane; k < round; k += 32) {
+            ring.w[wp][head + k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            ring.o[wp][head + k] = 0u;
+        }
+        __syncwarp();
+        step(head + g * U, t1, v1, t0, v0);
+        step(head + U * G + g * U, t0, v0, t1, v1);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) add1(t0[u], v0[u]);
+    __syncwarp();  // (the next call of a persistent block refills the ring)
+    float bad = 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int e = 0; e < VZ / 2; ++e) {
+            float lo, hi;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[q][e]));
+            if (VEC ? e / 2 < n : 2 * e < n) bad = fmaf(lo, 0.f, bad);
+            if (VEC ? e / 2 < n : 2 * e + 1 < n) bad = fmaf(hi, 0.f, bad);
+        }
+    if (__any_sync(kFull, bad != 0.f)) {  // as in the strips: an infinity only where it is sampled
+        adjoint_block_rows<Q, VEC, RAY>(a, bx);
+        return;
+    }
+    if constexpr (Q == 1)
+        for (int off = LZ; off < 32; off <<= 1)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int e = 0; e < VZ / 2; ++e) {
+                    const unsigned long long t = __shfl_xor_sync(kFull, acc[q][e], off);
+                    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc[q][e]) : "l"(t));
+                }
+    if (n == 0 || g != 0) return;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = i0 + (q >> 1), j = j0 + (q & 1);
+        if (i >= a.nY || j >= a.nX) continue;
+        const size_t p = (size_t)i * a.nX + j;
+        if (a.mask) {
+            const float m = __ldg(a.mask + p);
+            const unsigned long long mm = pk_pair(m, m);
+#pragma unroll
+            for (int e = 0; e < VZ / 2; ++e) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[q][e]) : "l"(mm));
+        }
+        strip_store<Q, VEC>(a.out + p * a.nZ + z0, acc[q], n, LZ, a.whole, a.nZ - z0);
+    }
+}
+
+// The block pixel by pixel, reading only the rows whose samples have the pixel among their taps (decided on
+// the forward's float64 coordinates).
+template <int Q, bool VEC, bool RAY>
+__device__ __noinline__ void adjoint_block_rows(const Args& a, unsigned bx) {
+    int i0, j0, z0, n;
+    if (!block_place<Q, VEC>(a, bx, i0, j0, z0, n)) return;
+    const int LZ = 1 << a.lz_shift;
+    if (n == 0 || (threadIdx.x & 31) >> a.lz_shift) return;
+    const float* __restrict__ bz = a.in + z0;
+    for (int q = 0; q < 4; ++q) {
+        const int i = i0 + (q >> 1), j = j0 + (q & 1);
+        if (i >= a.nY || j >= a.nX) continue;
+        unsigned long long acc[2 * Q] = {};
+        for (int th = 0; th < a.nA; ++th) {
+            const double4 tr = a.trig[th];
+            const double c = tr.x, s = tr.y, ri = (double)i - tr.w, ci = (double)j - tr.z;
+            const int Jn = __double2int_rn(fma(-s, ri, c * ci)), Kn = __double2int_rn(fma(c, ri, s * ci));
+            for (int J = max(Jn - 1, 0); J <= min(Jn + 1, a.nX - 1); ++J) {
+                const float t = (float)(J - a.C);
+                if (RAY && fabsf(t) > a.R) continue;
+                const float sent = RAY ? -sqrtf(a.R * a.R - t * t) : 0.f;
+                const double rowb = fma(-s, (double)J, tr.w), colb = fma(c, (double)J, tr.z);
+                float w = 0.f;
+                for (int K = max(Kn - 2, 0); K <= min(Kn + 2, a.nY - 1); ++K) {
+                    const double row = fma(c, (double)K, rowb), col = fma(s, (double)K, colb);
+                    const double fr = floor(row), fc = floor(col);
+                    const int r0 = (int)fr, c0 = (int)fc;
+                    if (!(i == r0 || (row > fr && i == r0 + 1)) || !(j == c0 || (col > fc && j == c0 + 1))) continue;
+                    const float dr = (float)(row - fr), dc = (float)(col - fc);
+                    float h = (i == r0 ? 1.f - dr : dr) * (j == c0 ? 1.f - dc : dc);
+                    if (RAY) h *= ray_factor((float)(K - a.C), sent, a.alpha);
+                    w += h;
+                }
+                if (w == 0.f) continue;
+                unsigned long long v[2 * Q];
+                strip_load<Q, VEC>(bz + ((size_t)J * a.nA + th) * a.zs, v, n, LZ);
+#pragma unroll
+                for (int e = 0; e < 2 * Q; ++e) fma_pairs(acc[e], pk_pair(w, w), v[e]);
+            }
+        }
+        const size_t p = (size_t)i * a.nX + j;
+        if (a.mask) {
+            const float m = __ldg(a.mask + p);
+#pragma unroll
+            for (int e = 0; e < 2 * Q; ++e) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[e]) : "l"(pk_pair(m, m)));
+        }
+        strip_store<Q, VEC>(a.out + p * a.nZ + z0, acc, n, LZ, a.whole, a.nZ - z0);
+    }
+}
+
+template <int Q, bool VEC, bool RAY>
+__global__ void __launch_bounds__(256, 2) k_adjoint_block(Args a) {
+    adjoint_block_body<Q, VEC, RAY>(a, blockIdx.x);
 }
 
 }  // namespace

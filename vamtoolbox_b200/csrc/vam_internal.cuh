@@ -85,10 +85,6 @@ struct vam_parallel_plan {
     int4* d_bwd_btab;       // [blocks inside][nA][2] 2 x 2 block bin table (k_bwd_btable)
     int* d_bwd_bcidx;       // [(nY + 1) / 2][(nX + 1) / 2] compact block index, -1 outside the circle
     float* d_img_pad;       // nZ == 1: [nY][nX rounded up to 4] staged image of the TMA-tiled 2-D forward
-    // matched-transpose weights: per pixel and angle, the first of <= 3
-    // detector rows (as int bits) and their summed forward tap weights
-    float4* d_adj_table;    // [nY*nX][nA]
-    int adj_table_abs;      // absorption mode the table was built for (-1: none built)
     // reference-parity backprojection bins (k_bwd_btable): the clip circle's compact pixel index
     // (-1 outside) from which the block table is built
     int* d_bwd_cidx;
