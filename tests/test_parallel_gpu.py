@@ -554,3 +554,47 @@ def test_forward_strips_at_their_edges(n, nz, absn):
     assert np.array_equal(np.isnan(strip), np.isnan(mirror)) and np.array_equal(np.isinf(strip), np.isinf(mirror))
     ok = np.isfinite(plain) & np.isfinite(mirror)
     assert not ok.all() and np.abs(strip[ok] - plain[ok]).max() <= 4.6e-6 * np.abs(plain[ok]).max()
+
+
+@pytest.mark.parametrize("n,nz", [(9, 9), (12, 16), (17, 5), (24, 64), (33, 17), (31, 65), (20, 128), (21, 130),
+                                  (26, 132), (16, 256), (15, 261), (40, 70)])
+@pytest.mark.parametrize("absn", [None, "mask", "ray"])
+def test_transpose_blocks_and_padded_rows_at_their_edges(n, nz, absn):
+    """The block kernel of the matched transpose against the oracle: blocks past the image's edge, slice counts
+    around the lanes of one chunk, angle counts around its batches of six.  A pixel sums at most 2.6 rows per
+    angle: 2.6 * 13 additions of 2^-24 each, 2.1e-6.  A slice count that is not a multiple of four is padded to
+    one: forward and transpose equal the same kernels on the unpadded rows bit for bit, the backprojection from
+    its bin table the oracle's.  An infinity reaches exactly the pixels its row touches."""
+    from vamtoolbox_b200 import _lib
+
+    rng = np.random.default_rng(n * nz + 1)
+    ang = np.array([0.0, 17.3, 45.0, 62.5, 90.0, 133.3, 180.0, 197.3, 222.2, 242.5, 270.0, 301.0, 333.3])
+    p = plan_for((n, n, nz), ang)
+    p.pad_from = p.pad_backward_from = 0  # (from any size on)
+    oabs = None
+    if absn == "mask":
+        m = rng.uniform(0.2, 1.0, (n, n))
+        p.set_absorption("mask", mask=m)
+        oabs = ("mask", m)
+    elif absn == "ray":
+        p.set_absorption("ray", alpha_per_px=0.03, radius_px=n / 2 - 1.5)
+        oabs = ("ray", 0.03, n / 2 - 1.5)
+    x, b = rng.uniform(-0.2, 1, (n, n, nz)), rng.uniform(-0.2, 1, (n, ang.size, nz))
+    got = p.adjoint(dev(b))
+    scale = O.parallel_adjoint(np.abs(b), ang, absorption=oabs).max()
+    assert np.abs(got.cpu().numpy() - O.parallel_adjoint(b, ang, absorption=oabs)).max() <= 2.1e-6 * scale
+    if nz % 4:
+        assert p._pads(_lib.OP_FORWARD) and p._pads(_lib.OP_ADJOINT)
+        for op, src, name in (("forward", dev(x), "vam_parallel_forward"), ("adjoint", dev(b), "vam_parallel_adjoint")):
+            padded = getattr(p, op)(src)
+            plain = torch.empty_like(padded)
+            _lib.call(name, p.handle, _lib.ptr(src), _lib.ptr(plain), p._stream())
+            assert torch.equal(padded, plain)
+        back = p.backward_ref(dev(b)).cpu().numpy()
+        assert relL2(back, O.parallel_backward_ref(b, ang, absorption=oabs)) < TOL
+    bi = b.copy()
+    bi[n // 2, 3, nz // 2] = np.inf  # angle 62.5 degrees
+    inf = torch.isinf(p.adjoint(dev(bi))).cpu().numpy()
+    touched = np.zeros((n, ang.size, nz))
+    touched[n // 2, 3, nz // 2] = 1.0
+    assert np.array_equal(inf, O.parallel_adjoint(touched, ang, absorption=oabs) > 1e-6)

@@ -69,7 +69,12 @@ class ProjectionBatch:
                 raise ValueError(f"plan on {plan.device}, batch on {self.device}")
             if OPS[op] == _lib.OP_ADJOINT and not plan._adj_ready and not torch.cuda.is_current_stream_capturing():
                 plan.prepare_adjoint()
-            items.append(_lib.Work(plan.handle.value, OPS[op], x.data_ptr(), y.data_ptr()))
+            code = OPS[op]
+            if plan._pads(code):  # as the plan's own call (bit-identical to it)
+                with torch.cuda.device(self.device):
+                    x = plan._padded(x)
+                code |= _lib.OP_PADDED
+            items.append(_lib.Work(plan.handle.value, code, x.data_ptr(), y.data_ptr()))
             keep.append((plan, x, y))
         arr = (_lib.Work * len(items))(*items)
         return arr, keep
