@@ -598,3 +598,24 @@ def test_transpose_blocks_and_padded_rows_at_their_edges(n, nz, absn):
     touched = np.zeros((n, ang.size, nz))
     touched[n // 2, 3, nz // 2] = 1.0
     assert np.array_equal(inf, O.parallel_adjoint(touched, ang, absorption=oabs) > 1e-6)
+
+
+@pytest.mark.parametrize("n", [31, 32, 33, 64, 65, 100])
+@pytest.mark.parametrize("na", [1, 63, 64, 70])
+def test_slice_backprojection_tiles_at_their_edges(n, na):
+    """The 2-D backprojection tiles (32 x 8 pixels, 64 staged angles, four groups of angles): partial tiles and
+    angle blocks, rays along the axes (coordinates on integers and at the detector's ends), against the oracle.
+    A weight is good to 2^-23 and a group adds at most 18 terms, together below 20 2^-24 of the largest sum:
+    1.2e-6.  An infinity reaches the pixels the generic kernel's does."""
+    rng = np.random.default_rng(n + na)
+    ang = np.concatenate([[0.0, 90.0, 180.0, 270.0, 45.0], rng.uniform(0, 360, 70)])[:na] if na > 1 else np.array([33.3])
+    p = plan_for((n, n, 1), ang)
+    p.set_tuning({"backward_vz": 4})
+    b = rng.uniform(-0.2, 1, (n, ang.size, 1))
+    ref = O.parallel_backward_ref(b, ang)
+    got = p.backward_ref(dev(b)).cpu().numpy()
+    assert np.abs(got - ref).max() <= 1.2e-6 * np.abs(O.parallel_backward_ref(np.abs(b), ang)).max()
+    b[n // 2, ang.size - 1, 0] = np.inf
+    got = p.backward_ref(dev(b))
+    p.set_tuning({"backward_vz": 1})
+    assert torch.equal(torch.isinf(got), torch.isinf(p.backward_ref(dev(b))))

@@ -68,6 +68,7 @@ struct Args {
     float* out;
     const double4* trig;
     const uint8_t* circle;
+    const float4* split;  // nZ == 1: per angle the high and low parts of cos and sin
     const float* mask;
     const float* occ;
     const uint8_t* occ_flag;
@@ -787,10 +788,13 @@ constexpr int k2K = 64;     // forward: samples per bin per tile
 constexpr int k2Box = 96;   // forward: staged box side >= sqrt(2) (k2J + k2K - 2) + 5
 constexpr int k2Stride = k2Box + 1;
 constexpr int k2Smem = (k2Box * k2Stride + 4 * k2J) * 4;  // box + the k-group partial sums
-constexpr int kB2 = 16;     // backprojection: pixel tile side
+constexpr int kB2 = 16;     // backprojection with per-ray absorption: pixel tile side
 constexpr int kB2A = 32;    // backprojection: angles per staged block (one per lane when staging)
-constexpr int kB2W = 30;    // backprojection: window bins per angle >= sqrt(2) (kB2 - 1) + 6
+constexpr int kB2W = 30;    // backprojection with per-ray absorption: window bins per angle >= sqrt(2) (kB2 - 1) + 6
 constexpr int kB2Smem = kB2A * kB2W * 4 + kB2A * 4 + kB2A * 16;
+constexpr int kP2X = 32, kP2Y = 8;  // backprojection: pixel tile, four pixels per thread, four groups of angles
+constexpr int kP2A = 64;    // backprojection: angles per staged block
+constexpr int kP2W = 39;    // backprojection: window bins per angle >= |(kP2X - 1, kP2Y - 1)| + 6, odd (banks)
 
 // grid (ceil(nX / k2J), nA); 256 threads = 64 bins x 4 groups of samples.
 //
@@ -1033,10 +1037,9 @@ __global__ void __launch_bounds__(256) k_forward_2d(Args a) {
     k_forward_2d_body<RAY>(a, blockIdx.x, blockIdx.y);
 }
 
-// grid (ceil(nX / 16) * ceil(nY / 16)); 256 threads = one 16 x 16 pixel tile
-template <bool RAY>
-__device__ __forceinline__ void k_backward_2d_body(const Args& a, unsigned bx, unsigned by) {
-    (void)by;
+// With per-ray absorption: grid (ceil(nX / 16) * ceil(nY / 16)); 256 threads = one 16 x 16 pixel tile
+__device__ __forceinline__ void backward_2d_ray_body(const Args& a, unsigned bx) {
+    constexpr bool RAY = true;
     extern __shared__ float s_b2[];
     float* win = s_b2;                                            // [kB2A][kB2W]
     int* wlo = reinterpret_cast<int*>(s_b2 + kB2A * kB2W);        // [kB2A] first staged detector row
@@ -1107,6 +1110,122 @@ __device__ __forceinline__ void k_backward_2d_body(const Args& a, unsigned bx, u
         if (a.mask) acc = __ldg(a.mask + p) * acc;
         a.out[p] = acc;
     }
+}
+
+// np.interp's bin (from the first staged row) and weight in float64; at the detector's last bin its row alone
+__device__ __noinline__ float2 interp_bin(const double4* tr, float X, float Y, int base, int last) {
+    const double t = __dsub_rn(__dmul_rn((double)X, tr->x), __dmul_rn((double)Y, tr->y));
+    const double ft = floor(t);
+    const int k = (int)fmax(fmin(ft, 1e9), -1e9) + base;
+    return t == ft && k == last ? make_float2(__int_as_float(k - 1), 1.f) : make_float2(__int_as_float(k), (float)(t - ft));
+}
+
+// Grid (ceil(nX / 32) * ceil(nY / 8)), 256 threads = one 32 x 8 pixel tile: warp w sums every fourth angle
+// (w / 2) for four rows of 32 pixels, and the four groups' sums are added at the end.  The small tile and the
+// groups spread a slice over the SMs (a 32 x 16 tile over all angles left 45 % of them idle at 512^2).
+//
+// np.interp's bin and weight without float64 arithmetic in the loop (its conversions and floors are issued at
+// an eighth of the float32 rate and took most of the time): cos and sin are split into a high part of few
+// enough bits that X ch - Y sh is exact in float32 and a low part (the plan's table), so t = A + B with A exact and B below one
+// bin, good to 2^-25 of a bin at any position; the nearest integer comes from adding 1.5 * 2^23.  Fractions
+// within 1e-5 of an integer (where t decides between bins, or whether it is on the detector at all) are
+// formed again in float64 as numpy does, but for an exact integer (the centre pixel's, at every angle).
+// 512^2 x 720: 369 -> 219 us, 600^2 x 800 529 -> 310, 256^2 x 360 95 -> 53; issue is 75 % busy, 34
+// instructions a pixel and angle.
+__device__ __forceinline__ void backward_2d_body(const Args& a, unsigned bx) {
+    __shared__ float win[kP2A * kP2W];
+    __shared__ float4 cs[kP2A];  // ch, cl, sh, sl
+    __shared__ int2 lim[kP2A];   // first staged detector row; last row of the detector from it
+    __shared__ float part[4][kP2Y][kP2X];
+    const int tiles_x = (a.nX + kP2X - 1) / kP2X;
+    const int i0 = (int)(bx / tiles_x) * kP2Y, jx0 = (int)(bx % tiles_x) * kP2X;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, ag = wp >> 1, r0 = 4 * (wp & 1);
+    const float Xf = (float)(jx0 + lane - a.C), Yf = (float)(i0 + r0 - a.C);
+    // the thread's pixel of the output
+    const int oi = i0 + wp, oj = jx0 + lane;
+    const bool inside = oi < a.nY && oj < a.nX;
+    const bool on = inside && a.circle[(long)oi * a.nX + oj];
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const bool any = __syncthreads_or(on);
+    for (int th0 = 0; any && th0 < a.nA; th0 += kP2A) {
+        const int na = min(kP2A, a.nA - th0);
+        if (threadIdx.x < (unsigned)na) {
+            const float4 t4 = a.split[th0 + threadIdx.x];
+            cs[threadIdx.x] = t4;
+            // the tile's least detector coordinate (two rows of margin cover its rounding)
+            const float c = t4.x + t4.y, s = t4.z + t4.w;
+            const float t = (float)(jx0 - a.C) * c - (float)(i0 - a.C) * s;
+            const int lo = max((int)floorf(t + fminf(0.f, (kP2X - 1) * c) + fminf(0.f, -(kP2Y - 1) * s)) + a.C - 2, 0);
+            lim[threadIdx.x] = make_int2(lo, a.nY - 1 - lo);
+        }
+        __syncthreads();
+        // warp w stages window bins w, w + 8, ...; lane = angle (consecutive angles are contiguous)
+#pragma unroll
+        for (int h = 0; h < kP2A; h += 32) {
+            const int sa = lane + h;
+            if (sa < na) {
+                const int lo = lim[sa].x;
+#pragma unroll
+                for (int w = 0; w < kP2W; w += kWarpsPerBlock)
+                    if (w + wp < kP2W)
+                        win[sa * kP2W + w + wp] = lo + w + wp < a.nY ? __ldg(a.in + (size_t)(lo + w + wp) * a.nA + th0 + sa) : 0.f;
+            }
+        }
+        __syncthreads();
+        for (int al = ag; al < na; al += 4) {
+            const float4 t4 = cs[al];
+            const int2 lm = lim[al];
+            const float* wn = win + al * kP2W;
+            const float xh = fmaf(-Yf, t4.z, Xf * t4.x), xl = fmaf(-Yf, t4.w, Xf * t4.y);
+            const int base = a.C - 0x4b400000 - lm.x;
+            float w[4];
+            int k[4];
+            bool near = false;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float A = fmaf(-(float)q, t4.z, xh), B = fmaf(-(float)q, t4.w, xl);
+                const float m = (A + B) + 12582912.f;  // the nearest integer in the low bits
+                const float r = (A - (m - 12582912.f)) + B;
+                w[q] = r < 0.f ? r + 1.f : r;
+                k[q] = __float_as_int(m) + base - (r < 0.f ? 1 : 0);
+                near |= fabsf(r) < 1e-5f && (r != 0.f || k[q] >= lm.y);
+            }
+            if (near) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float2 kw = interp_bin(a.trig + th0 + al, Xf, Yf + (float)q, a.C - lm.x, lm.y);
+                    k[q] = __float_as_int(kw.x);
+                    w[q] = kw.y;
+                }
+            }
+            // np.interp(left = right = 0): nothing off the detector.  (The clamp is for memory safety only:
+            // the window covers the tile.)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float* v = wn + min((unsigned)k[q], (unsigned)(kP2W - 2));
+                const float v0 = v[0], v1 = v[1];
+                const float x = w[q] != 0.f ? fmaf(w[q], v1 - v0, v0) : v0;
+                if ((unsigned)k[q] < (unsigned)lm.y) acc[q] += x;
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) part[ag][r0 + q][lane] = acc[q];
+    __syncthreads();
+    if (inside) {
+        const float x = on ? (part[0][wp][lane] + part[1][wp][lane]) + (part[2][wp][lane] + part[3][wp][lane]) : 0.f;
+        const long p = (long)oi * a.nX + oj;
+        a.out[p] = a.mask ? __ldg(a.mask + p) * x : x;
+    }
+    __syncthreads();  // (a persistent block's next tile reuses the shared memory)
+}
+
+template <bool RAY>
+__device__ __forceinline__ void k_backward_2d_body(const Args& a, unsigned bx, unsigned by) {
+    (void)by;
+    if constexpr (RAY) backward_2d_ray_body(a, bx);
+    else backward_2d_body(a, bx);
 }
 
 template <bool RAY>
@@ -1586,12 +1705,15 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     }
     const bool ray = plan->abs_mode == VAM_ABS_RAY;
     // 2-D slice: shared-memory tiles when tuned to them (any width but 1), or automatically for
-    // slices wide enough to fill the device with tiles (forward from 192, backprojection from 320 px)
-    const bool tiles_2d = want == 0 ? plan->nX >= (op == Op::Forward ? 192 : 320) : want != 1;
+    // slices wide enough to fill the device with tiles: from 192 px (backprojection 29.7 against 31.7 us of the
+    // generic kernel at 192^2 x 180, 31.6 against 23.6 at 160^2 x 180, 53 against 84 at 256^2 x 360; with
+    // per-ray absorption from 320)
+    const bool tiles_2d = want == 0 ? plan->nX >= (op == Op::BackwardRef && ray ? 320 : 192) : want != 1;
     if (plan->nZ == 1 && !plan->has_occ && op != Op::Adjoint && tiles_2d && !noclip) {
         Args& a = it.a;
         a.in = in; a.out = out; a.trig = plan->d_trig; a.circle = plan->d_circle;
         a.mask = plan->abs_mode == VAM_ABS_MASK ? plan->d_mask : nullptr;
+        a.split = plan->d_split;
         a.nY = plan->nY; a.nX = plan->nX; a.nZ = 1; a.nA = plan->nA; a.C = plan->C;
         a.alpha = plan->abs_alpha; a.R = plan->abs_R;
         it.ray = ray;
@@ -1625,8 +1747,9 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
             it.smem = it.tma ? k2SmemTma : k2Smem;
         } else {
             it.kind = KB_2D;
-            it.gx = (unsigned)(((plan->nX + kB2 - 1) / kB2) * ((plan->nY + kB2 - 1) / kB2));
-            it.smem = kB2Smem;
+            it.gx = ray ? (unsigned)(((plan->nX + kB2 - 1) / kB2) * ((plan->nY + kB2 - 1) / kB2))
+                        : (unsigned)(((plan->nX + kP2X - 1) / kP2X) * ((plan->nY + kP2Y - 1) / kP2Y));
+            it.smem = ray ? kB2Smem : 0;
         }
         return VAM_OK;
     }
@@ -1780,11 +1903,11 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
             else { if (it.vec) forward_strip_body<1, true, RAY>(f, bx, by); else forward_strip_body<1, false, RAY>(f, bx, by); }
         }
     }
-    if constexpr ((FAM & 128) != 0) {
+    if constexpr (FAM == 128 || FAM == 512) {
         if (it.kind == KF_2D) {
             const Args a = it.a;
-            if (it.tma) k_forward_2d_tma_body<RAY>(a, &it.tmap, it.status, bx, by);
-            else if constexpr (FAM == 511) k_forward_2d_body<RAY>(a, bx, by);
+            if constexpr (FAM == 128) k_forward_2d_tma_body<RAY>(a, &it.tmap, it.status, bx, by);
+            else k_forward_2d_body<RAY>(a, bx, by);
         }
     }
     if constexpr (FAM == 256 && !RAY) {
@@ -1826,8 +1949,8 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
 // absorption, 4 adjoint, 8 the other backprojections (generic with occlusion
 // or per-ray absorption, fast with per-ray absorption), 16 the generic forward
 // with occlusion or per-ray absorption, 32 / 64 the generic forward /
-// backprojection without either, 256 the block-table backprojection (511: all
-// bodies, for calls of mixed families); a batch launches one instance per family
+// backprojection without either, 256 the block-table backprojection, 512 the 2-D
+// forward with plain staging; a batch launches one instance per family
 // present, so no body is compiled around the registers of rarer ones and each
 // keeps about its direct kernel's occupancy.
 template <int FAM>
@@ -2076,7 +2199,7 @@ BatchKernel batch_kernel(int fam) {
         case 64: return k_batch<64>;
         case 128: return k_batch<128>;
         case 256: return k_batch<256>;
-        default: return k_batch<511>;
+        default: return k_batch<512>;
     }
 }
 
@@ -2181,6 +2304,18 @@ extern "C" int vam_parallel_plan_create(const vam_parallel_geom* geom, vam_paral
     if (e == cudaSuccess) e = cudaMalloc(&p->d_circle, circ.size());
     if (e == cudaSuccess) e = cudaMalloc(&p->d_status, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(p->d_status, 0, sizeof(int));
+    if (e == cudaSuccess && p->nZ == 1) {
+        // cos and sin as a high part whose products with a pixel coordinate (and their difference) are exact in
+        // float32 and the rest: multiples of 2^-bits for coordinates below 2^(22 - bits)
+        const double unit = std::ldexp(1.0, 22 - (ilog2_pow2(p->nX) + 1));
+        std::vector<float4> split(p->nA);
+        for (int i = 0; i < p->nA; ++i) {
+            const double ch = std::rint(trig[i].x * unit) / unit, sh = std::rint(trig[i].y * unit) / unit;
+            split[i] = make_float4((float)ch, (float)(trig[i].x - ch), (float)sh, (float)(trig[i].y - sh));
+        }
+        e = cudaMalloc(&p->d_split, sizeof(float4) * p->nA);
+        if (e == cudaSuccess) e = cudaMemcpy(p->d_split, split.data(), sizeof(float4) * p->nA, cudaMemcpyHostToDevice);
+    }
     if (e == cudaSuccess && p->nZ == 1)
         e = cudaMalloc(&p->d_img_pad, sizeof(float) * (size_t)p->nY * (size_t)((p->nX + 3) & ~3));
     if (e == cudaSuccess) e = cudaMemcpy(p->d_trig, trig.data(), sizeof(double4) * p->nA, cudaMemcpyHostToDevice);
@@ -2209,6 +2344,7 @@ extern "C" int vam_parallel_plan_destroy(vam_parallel_plan* p) {
     cudaFree(p->d_bwd_cidx);
     cudaFree(p->d_status);
     cudaFree(p->d_img_pad);
+    cudaFree(p->d_split);
     cudaFree(p->d_bwd_btab);
     cudaFree(p->d_bwd_bcidx);
     delete p;
@@ -2545,7 +2681,7 @@ struct vam_batch {
     int device;
     unsigned* d_counter;
     int sms;
-    int per_sm[512][4];        // resident CTAs per SM of k_batch<fam> (fam 1 .. 256, 511) per
+    int per_sm[513][4];        // resident CTAs per SM of k_batch<fam> (fam 1 .. 512) per
                                // dynamic shared-memory bucket (kSmemBuckets)
     std::vector<Item> host;    // the described calls of the last list, in queue order
     std::vector<int> group;    // first call of each launch (kBatchMaxItems calls per launch)
@@ -2579,12 +2715,12 @@ extern "C" int vam_batch_create(int32_t device, vam_batch** out) {
     VAM_REQUIRE(g.ok, VAM_ERR_CUDA, "vam_batch_create: cannot select device");
     int sms = 0;
     VAM_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    int per_sm[512][4] = {};
+    int per_sm[513][4] = {};
     // residency for each dynamic shared-memory bucket up to the largest a call may ask for (48 KB,
     // the batched backprojection's trig table), queried once here, so a list never needs a
     // runtime query (which would not be allowed during graph capture); the opt-in limit is
     // raised first, as 48 KB plus the kernel's static shared memory exceeds the default
-    for (int fam : {1, 2, 4, 8, 16, 32, 64, 128, 256, 511}) {
+    for (int fam : {1, 2, 4, 8, 16, 32, 64, 128, 256, 512}) {
         VAM_TRY_CUDA(cudaFuncSetAttribute(batch_kernel(fam), cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
         for (int k = 0; k < 4; ++k) {
             VAM_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[fam][k], batch_kernel(fam),
@@ -2670,8 +2806,8 @@ int batch_prepare(vam_batch* b, const vam_work* work, int32_t n) {
         else if (d.family == 2 && d.ray) items[i].family = 8;
         if (d.kind == KF_GEN) items[i].family = gen_heavy ? 16 : 32;
         // the 2-D forward instance carries the TMA-staged body only; plain staging (no tensor map
-        // encoder) runs in the all-bodies instance
-        if (d.kind == KF_2D && !d.tma) items[i].family = 511;
+        // encoder) has its own
+        if (d.kind == KF_2D && !d.tma) items[i].family = 512;
         if (d.kind == KB_BTABLE) items[i].family = 256;
 
         VAM_REQUIRE((long long)items[i].gx * items[i].gy < (1LL << 31), VAM_ERR_SHAPE, "vam_batch: call grid too large");
@@ -2707,7 +2843,6 @@ int batch_prepare(vam_batch* b, const vam_work* work, int32_t n) {
             b->any_pre |= items[i].pre_in != nullptr;
         }
         b->smem = std::max(b->smem, gsmem);
-        if (fam & (fam - 1)) fam = 511;  // one family per launch; the all-bodies instance otherwise
         // tickets: one per block of each call's grid, the calls one after another
         long long total = 0;
         for (int i = g0; i < g1; ++i) {

@@ -84,6 +84,7 @@ struct vam_parallel_plan {
     int* d_status;          // error bits the kernels record (VAM_STATUS_*), read by vam_parallel_status
     int4* d_bwd_btab;       // [blocks inside][nA][2] 2 x 2 block bin table (k_bwd_btable)
     int* d_bwd_bcidx;       // [(nY + 1) / 2][(nX + 1) / 2] compact block index, -1 outside the circle
+    float4* d_split;        // nZ == 1: [nA] high and low parts of cos and sin (the 2-D backprojection)
     float* d_img_pad;       // nZ == 1: [nY][nX rounded up to 4] staged image of the TMA-tiled 2-D forward
     // reference-parity backprojection bins (k_bwd_btable): the clip circle's compact pixel index
     // (-1 outside) from which the block table is built
