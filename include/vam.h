@@ -323,8 +323,8 @@ int vam_ray_active_at_cap(vam_ray_plan* plan, int64_t* out_count);
 
 /* Trajectory cache of a plan on a 3-D grid medium with the physical path
  * length and the symplectic Euler solver: the rays are traced once (the same
- * steps and exit checks as vam_ray_integrate) and each executed step's
- * position x_ip1 and attenuance are kept, 16 bytes per ray and step
+ * steps and exit checks as vam_ray_integrate) and each step's position x_ip1
+ * and attenuance near the grid are kept, room for 16 bytes per ray and step
  * (max_num_step x num_rays x 16 B: 36 GB at 128^3 x 360 rays x 384 steps).
  * While it is valid, vam_ray_integrate and vam_ray_deposit stream the records
  * instead of re-tracing (bit-identical results); vam_ray_set_medium

@@ -187,3 +187,47 @@ def test_trajectory_cache_bitwise_and_invalidated(golden):
     assert torch.equal(plan.integrate(f), P2.plan.integrate(f))
     assert relL2(plan.deposit(w).cpu().numpy(), P2.plan.deposit(w).cpu().numpy()) < 1e-5
     plan.drop_trajectories()
+
+
+@pytest.mark.parametrize("n,nz", [(5, 3), (16, 33), (31, 40), (64, 2)])
+@pytest.mark.parametrize("curved", [False, True])
+def test_padded_ray_kernels_match_the_recorded_matrix(n, nz, curved):
+    """The tracing and the record-streaming kernels against the propagation matrix (the unpadded kernel's corners,
+    applied in float64): straight rays along voxel centres, where a coordinate is an integer at every step and each
+    such corner counts twice, and curved ones; warps across detector columns; a cache of part of the rays.  The
+    same corners at positions up to 300 roundings of 2^-24 apart (6e-4 voxel at 64 voxels over the grid's width of
+    two), summed over 8 * 300 float32 additions: 1e-3 of the largest sum; a corner counted once where it counts
+    twice is at least 5e-3 of a ray's."""
+    from vamtoolbox_b200 import geometry, medium
+    from vamtoolbox_b200.projector.pyTorchRayTrace import PyTorchRayTracingPropagator
+
+    rng = np.random.default_rng(n + nz)
+    tg = geometry.TargetGeometry(target=np.zeros((n, n, nz)))
+    cv = tg.constructCoordVec()
+    r2 = (np.asarray(cv[0])[:, None] ** 2 + np.asarray(cv[1])[None, :] ** 2)[:, :, None] / np.max(cv[0]) ** 2
+    index = np.full((n, n, nz), 1.5) + (0.02 * r2 + 0.01 * np.linspace(0, 1, nz) if curved else 0.0)
+    im = medium.IndexModel(cv, type="interpolation", form="freeform", n_x=torch.as_tensor(index))
+    am = medium.AttenuationModel(cv, type="interpolation", form="freeform",
+                                 alpha_x=torch.as_tensor(rng.uniform(0.5, 1.0, (n, n, nz))))
+    pg = geometry.ProjectionGeometry(np.array([0.0, 33.0, 45.0, 90.0, 200.0]), "ray_trace", CUDA=True, index_model=im,
+                                     attenuation_model=am, absorption_model=am, ray_trace_method="eikonal",
+                                     eikonal_parametrization="physical_path_length",
+                                     ray_trace_ode_solver="forward_symplectic_euler", ray_trace_ray_config="parallel",
+                                     inclination_angle=0.0, ray_density=1)
+    plan = PyTorchRayTracingPropagator(tg, pg).plan
+    row_ptr, cols, vals = (v.cpu() for v in plan.record())
+    A = torch.sparse_csr_tensor(row_ptr, cols.long(), vals.double(), size=(plan.num_rays, n * n * nz))
+    f = torch.as_tensor(rng.uniform(0.5, 1, n * n * nz))
+    w = torch.as_tensor(rng.uniform(0, 1, plan.num_rays))
+    w[::5] = 0.0
+    g, d = A @ f, A.t() @ w
+    traced = None
+    for rays in (0, plan.num_rays // 2, plan.num_rays):
+        if rays >= 32:
+            assert plan.prepare_trajectories(limit_bytes=plan.trajectory_bytes(rays))
+        got = plan.integrate(f)
+        dep = plan.deposit(w).cpu().double().reshape(-1)
+        traced = got if traced is None else traced
+        assert torch.equal(got, traced)
+        assert (got.cpu().double() - g).abs().max() <= 1e-3 * g.abs().max()
+        assert (dep - d).abs().max() <= 1e-3 * d.abs().max()
