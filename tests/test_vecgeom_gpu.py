@@ -173,3 +173,17 @@ def test_autograd_vec_and_line2d():
     xd = x2.detach().double()
     fd = ((lp.forward((xd + 0.5 * d).float()).double() - lp.forward((xd - 0.5 * d).float()).double()) * w2).sum()
     assert abs(float(fd) - float((x2.grad * d).sum())) / abs(float(fd)) < 1e-4
+
+
+@pytest.mark.parametrize("n,nz", [(5, 33), (17, 96), (9, 200), (6, 300)])
+def test_inclined_blocks_of_several_rows_match_oracle(n, nz):
+    """Blocks that hold several rows of a short axis, the last of them partial, and one row of a long axis, with a
+    detector wider than the volume; the bound of the kernels' other tests (coordinates of 2^-16 of a pixel)."""
+    rng = np.random.default_rng(n + nz)
+    vol, vec = rng.random((n, n, nz)), genVectorsAstra(np.array([3.0, 100.0, 250.0]), 15.0)
+    plan = VecPlan(n, n, nz, vec, n + 2, nz, "cuda")
+    f = plan.forward(torch.as_tensor(vol, dtype=torch.float32, device="cuda")).cpu().numpy()
+    assert relL2(f, V.forward(vol, vec, n + 2, nz)) < 2e-5
+    sino = rng.random((n + 2, 3, nz))
+    b = plan.backward(torch.as_tensor(sino, dtype=torch.float32, device="cuda")).cpu().numpy()
+    assert relL2(b, V.backward(sino, vec, (n, n, nz))) < 2e-5
