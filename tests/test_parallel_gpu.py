@@ -646,3 +646,23 @@ def test_slice_forward_tiles_with_paired_angles_at_their_edges(n, absn):
     assert np.abs(got - ref).max() <= 1e-4 * ref.max()
     p.set_tuning({"forward_tma": 0})
     assert np.array_equal(p.forward(dev(x)).cpu().numpy(), got)
+
+
+@pytest.mark.parametrize("n", [63, 64])
+@pytest.mark.parametrize("absn", [None, "ray"])
+def test_slice_forward_tiles_spread_no_infinity(n, absn):
+    """An infinite pixel reaches the bins of the 2-D forward tiles that it reaches in the generic kernel: those it
+    has a weight for, not those whose zero weight it would turn into NaN (angles off the axes, where the pixel is
+    on no sample's edge to rounding, and 0 and 90 degrees, whose samples are pixels)."""
+    ang = np.array([0.0, 17.3, 90.0, 197.3, 61.9])
+    x = np.random.default_rng(n).uniform(0.5, 1, (n, n, 1))
+    x[n // 3, n // 2, 0] = np.inf
+    p = plan_for((n, n, 1), ang)
+    if absn == "ray":
+        p.set_absorption("ray", alpha_per_px=0.01, radius_px=n / 2.0)
+    p.set_tuning({"forward_vz": 4})
+    got = p.forward(dev(x))
+    p.set_tuning({"forward_vz": 1})
+    ref = p.forward(dev(x))
+    assert torch.equal(torch.isinf(got), torch.isinf(ref)) and torch.equal(torch.isnan(got), torch.isnan(ref))
+    assert 0 < int(torch.isinf(got).sum()) < 20

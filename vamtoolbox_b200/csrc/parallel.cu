@@ -801,7 +801,7 @@ constexpr int kP2W = 39;    // backprojection: window bins per angle >= |(kP2X -
 // bins of its lattice rows, j in [0, N] and k in [1, N - 1] for even N, to which each adds its end sample.
 // The tile is bound by the latency of its single box and by issue (warps of 8 bins x 4 samples, which halve
 // the bank conflicts near 90 degrees, measured the same): half the tiles took 343 -> 189 us at 512^2 x 720
-// angles, 105 -> 67 at 363^2 x 360 and 49 -> 39 at 256^2 x 360.
+// angles, 105 -> 67 at 363^2 x 360 and 49 -> 39 at 256^2 x 360; with Line2d 182, 65 and 37.
 struct Slice2d {
     int theta, partner;  // partner < 0: unpaired
     bool ext;            // even N, paired: lattice row and sample N belong to the partner
@@ -834,9 +834,43 @@ __device__ __forceinline__ float sample_2d(const Args& a, const double4& tr, int
     return v;
 }
 
+// Position in a tile's box, 2^-32 of a pixel: four samples on is an addition, the whole part is the tap and the
+// fraction's first 23 bits the weight.  (The offsets were float32 products, whose floors and conversions run on
+// the quarter-rate unit, good to 4e-6 of a pixel; with sums of every second sample of a tile the error of a 512^2
+// slice's sinogram against 64 bits went from 1.3e-7 to 4.8e-8, at 128^2 from 2e-7 to 4.5e-8, the generic
+// kernel's being 4.2e-8.)
+struct Line2d {
+    long long r, q;
+    __device__ __forceinline__ Line2d(double row, double col) : r(fixed(row)), q(fixed(col)) {}
+    static __device__ __forceinline__ long long fixed(double v) { return __double2ll_rn(v * 4294967296.0); }
+    static __device__ __forceinline__ int split(long long v, float& frac) {
+        frac = __uint_as_float(0x3F800000u + ((((unsigned)v >> 8) + 1u) >> 1)) - 1.f;
+        return (int)(v >> 32);
+    }
+    __device__ __forceinline__ int row(float& frac) const { return split(r, frac); }
+    __device__ __forceinline__ int col(float& frac) const { return split(q, frac); }
+    __device__ __forceinline__ void step(long long dr, long long dq) { r += dr; q += dq; }
+};
+
+// A sum that is not finite again, tap by tap: a tile adds zero weights too, which an infinity turns into NaN.
+template <bool RAY>
+__device__ __forceinline__ float resum_2d(const Args& a, int theta, int j, int k0) {
+    const double4 tr = a.trig[theta];
+    const float t = (float)(j - a.C);
+    if (RAY && fabsf(t) > a.R) return 0.f;
+    float sum = 0.f;
+    for (int k = k0; k < a.nY; ++k) {
+        const float v = sample_2d(a, tr, j, k);
+        sum += RAY ? v * ray_factor((float)(k - a.C), -sqrtf(a.R * a.R - t * t), a.alpha) : v;
+    }
+    return sum;
+}
+
 // Lattice row j's bins from the sum of its samples.
+template <bool RAY>
 __device__ __forceinline__ void store_2d(const Args& a, const Slice2d& t, const double4& tr, int j, float sum) {
     const int N = a.nX;
+    if (!(fabsf(sum) <= 3.402823466e38f)) sum = resum_2d<RAY>(a, t.theta, j, t.kfirst);
     if (j < N) a.out[(size_t)j * a.nA + t.theta] = t.ext ? sum + sample_2d(a, tr, j, 0) : sum;
     const int jp = 2 * a.C - j;
     if (t.partner >= 0 && jp >= 0 && jp < N)
@@ -853,7 +887,7 @@ __device__ __forceinline__ void last_row_2d(const Args& a, const Slice2d& t, con
     if (threadIdx.x == 0) {
         float sum = 0.f;
         for (int w = 0; w < kWarpsPerBlock; ++w) sum += part[w];
-        store_2d(a, t, tr, a.nX, sum);
+        store_2d<false>(a, t, tr, a.nX, sum);
     }
     __syncthreads();
 }
@@ -865,9 +899,8 @@ __device__ __forceinline__ void last_row_2d(const Args& a, const Slice2d& t, con
 // affine in j and k, so the corners bound them); it is staged unclipped, with
 // zeros outside the image, which is exactly the zero padding of the reference's
 // warp, so every tap is an unconditional shared-memory read.  Each bin's
-// coordinates are the reference's float64 values at the tile's first sample;
-// the offsets along the ray are float32 (coordinate error below 2e-5 pixel on
-// a continuous bilinear interpolant).
+// coordinates are the reference's float64 values at the tile's first sample,
+// taken on along the ray in fixed point (Line2d).
 template <bool RAY>
 __device__ __forceinline__ void k_forward_2d_body(const Args& a, unsigned bx, unsigned by) {
     extern __shared__ float s_f2[];
@@ -881,7 +914,7 @@ __device__ __forceinline__ void k_forward_2d_body(const Args& a, unsigned bx, un
     const double4 tr = a.trig[t2.theta];
     if (j0 == a.nX) return last_row_2d(a, t2, tr, part);
     const double c = tr.x, s = tr.y;
-    const float cf = (float)c, sf = (float)s;
+    const long long c4 = Line2d::fixed(4 * c), s4 = Line2d::fixed(4 * s);
     const double rowb = fma(-s, (double)j, tr.w), colb = fma(c, (double)j, tr.z);
     float s_entry = 0.f;
     bool live = j <= t2.jmax;
@@ -924,14 +957,14 @@ __device__ __forceinline__ void k_forward_2d_body(const Args& a, unsigned bx, un
         }
         __syncthreads();
         if (live) {
-            const float rl0 = (float)(fma(c, (double)k0, rowb) - (double)rlo);
-            const float cl0 = (float)(fma(s, (double)k0, colb) - (double)clo);
-            for (int kk = tk; kk <= k1 - k0; kk += 4) {
-                const float row = fmaf(cf, (float)kk, rl0), col = fmaf(sf, (float)kk, cl0);
-                const float fr = floorf(row), fc = floorf(col);
-                const float dr = row - fr, dc = col - fc;
-                // clamped for memory safety only: the margins keep every weighted tap inside the box
-                const int r0 = min(max((int)fr, 0), H - 2), c0 = min(max((int)fc, 0), W - 2);
+            float tile = 0.f, other = 0.f;  // sums of every second sample
+            Line2d l(fma(c, (double)(k0 + tk), rowb) - (double)rlo, fma(s, (double)(k0 + tk), colb) - (double)clo);
+#pragma unroll 2
+            for (int kk = tk; kk <= k1 - k0; kk += 4, l.step(c4, s4)) {
+                float dr, dc;
+                // inside the box: a sample lies between the corners, floor(rmin) to floor(rmax), whose rows are 1 to
+                // H - 3, and 16 steps of 2^-33 move it by less than a row
+                const int r0 = l.row(dr), c0 = l.col(dc);
                 const float* t0 = box + r0 * k2Stride + c0;
                 const float w00 = (1.f - dr) * (1.f - dc), w01 = (1.f - dr) * dc;
                 const float w10 = dr * (1.f - dc), w11 = dr * dc;
@@ -940,15 +973,18 @@ __device__ __forceinline__ void k_forward_2d_body(const Args& a, unsigned bx, un
                 v = fmaf(w10, t0[k2Stride], v);
                 v = fmaf(w11, t0[k2Stride + 1], v);
                 if (RAY) v *= ray_factor((float)(k0 + kk - a.C), s_entry, a.alpha);
-                acc += v;
+                const float sum = tile + v;
+                tile = other;
+                other = sum;
             }
+            acc += tile + other;
         }
         __syncthreads();
     }
     part[tk * k2J + tj] = acc;
     __syncthreads();
     if (tk == 0 && j <= t2.jmax)
-        store_2d(a, t2, tr, j, ((part[tj] + part[k2J + tj]) + part[2 * k2J + tj]) + part[3 * k2J + tj]);
+        store_2d<RAY>(a, t2, tr, j, ((part[tj] + part[k2J + tj]) + part[2 * k2J + tj]) + part[3 * k2J + tj]);
 }
 
 // The same tiles with the footprint box staged by one TMA tensor load per tile.
@@ -1005,7 +1041,7 @@ __device__ __forceinline__ void k_forward_2d_tma_body(const Args& a, const CUten
     const double4 tr = a.trig[t2.theta];
     if (j0 == a.nX) return last_row_2d(a, t2, tr, part);
     const double c = tr.x, s = tr.y;
-    const float cf = (float)c, sf = (float)s;
+    const long long c4 = Line2d::fixed(4 * c), s4 = Line2d::fixed(4 * s);
     const double rowb = fma(-s, (double)j, tr.w), colb = fma(c, (double)j, tr.z);
     float s_entry = 0.f;
     bool live = j <= t2.jmax;
@@ -1054,14 +1090,14 @@ __device__ __forceinline__ void k_forward_2d_tma_body(const Args& a, const CUten
         phase ^= 1u;
         if (failed) break;  // uniform in practice; a block that gives up writes no outputs
         if (live) {
-            const float rl0 = (float)(fma(c, (double)k0, rowb) - (double)rlo);
-            const float cl0 = (float)(fma(s, (double)k0, colb) - (double)clo);
-            for (int kk = tk; kk <= k1 - k0; kk += 4) {
-                const float row = fmaf(cf, (float)kk, rl0), col = fmaf(sf, (float)kk, cl0);
-                const float fr = floorf(row), fc = floorf(col);
-                const float dr = row - fr, dc = col - fc;
-                // clamped for memory safety only: the margins keep every weighted tap inside the box
-                const int r0 = min(max((int)fr, 0), H - 2), c0 = min(max((int)fc, 0), W - 2);
+            float tile = 0.f, other = 0.f;  // sums of every second sample
+            Line2d l(fma(c, (double)(k0 + tk), rowb) - (double)rlo, fma(s, (double)(k0 + tk), colb) - (double)clo);
+#pragma unroll 2
+            for (int kk = tk; kk <= k1 - k0; kk += 4, l.step(c4, s4)) {
+                float dr, dc;
+                // inside the box: a sample lies between the corners, floor(rmin) to floor(rmax), whose rows are 1 to
+                // H - 3, and 16 steps of 2^-33 move it by less than a row
+                const int r0 = l.row(dr), c0 = l.col(dc);
                 const float* t0 = box + r0 * kTmaW + c0 + cofs;
                 const float w00 = (1.f - dr) * (1.f - dc), w01 = (1.f - dr) * dc;
                 const float w10 = dr * (1.f - dc), w11 = dr * dc;
@@ -1070,8 +1106,11 @@ __device__ __forceinline__ void k_forward_2d_tma_body(const Args& a, const CUten
                 v = fmaf(w10, t0[kTmaW], v);
                 v = fmaf(w11, t0[kTmaW + 1], v);
                 if (RAY) v *= ray_factor((float)(k0 + kk - a.C), s_entry, a.alpha);
-                acc += v;
+                const float sum = tile + v;
+                tile = other;
+                other = sum;
             }
+            acc += tile + other;
         }
         __syncthreads();  // every read of this box is done before the next copy overwrites it
     }
@@ -1082,7 +1121,7 @@ __device__ __forceinline__ void k_forward_2d_tma_body(const Args& a, const CUten
         part[tk * k2J + tj] = acc;
         __syncthreads();
         if (tk == 0 && j <= t2.jmax)
-            store_2d(a, t2, tr, j, ((part[tj] + part[k2J + tj]) + part[2 * k2J + tj]) + part[3 * k2J + tj]);
+            store_2d<RAY>(a, t2, tr, j, ((part[tj] + part[k2J + tj]) + part[2 * k2J + tj]) + part[3 * k2J + tj]);
     }
     __syncthreads();
     if (threadIdx.x == 0) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
@@ -1770,7 +1809,8 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     // slices wide enough to fill the device with tiles: from 192 px (backprojection 29.7 against 31.7 us of the
     // generic kernel at 192^2 x 180, 31.6 against 23.6 at 160^2 x 180, 53 against 84 at 256^2 x 360; with
     // per-ray absorption from 320)
-    const bool tiles_2d = want == 0 ? plan->nX >= (op == Op::BackwardRef && ray ? 320 : 192) : want != 1;
+    // forward, 96^2 x 120 angles: tiles 14.4 us, generic 14.4; 128^2 x 180: 16.4 and 26.7
+    const bool tiles_2d = want == 0 ? plan->nX >= (op == Op::Forward ? 112 : ray ? 320 : 192) : want != 1;
     if (plan->nZ == 1 && !plan->has_occ && op != Op::Adjoint && tiles_2d && !noclip) {
         Args& a = it.a;
         a.in = in; a.out = out; a.trig = plan->d_trig; a.circle = plan->d_circle;
