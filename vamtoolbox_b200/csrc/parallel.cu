@@ -1809,8 +1809,11 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     // slices wide enough to fill the device with tiles: from 192 px (backprojection 29.7 against 31.7 us of the
     // generic kernel at 192^2 x 180, 31.6 against 23.6 at 160^2 x 180, 53 against 84 at 256^2 x 360; with
     // per-ray absorption from 320)
-    // forward, 96^2 x 120 angles: tiles 14.4 us, generic 14.4; 128^2 x 180: 16.4 and 26.7
-    const bool tiles_2d = want == 0 ? plan->nX >= (op == Op::Forward ? 112 : ray ? 320 : 192) : want != 1;
+    // forward, 96^2 x 120 angles: tiles 14.4 us, generic 14.4; 112^2 x 150 14.4 and 20.5; 128^2 x 180 16.4 and
+    // 26.7.  Below 192 only images that need no staging: a batch lists a plan whose storage a call uses once.
+    const bool unstaged = plan->nX % 4 == 0 && (((uintptr_t)in) & 15) == 0 && plan->abs_mode != VAM_ABS_MASK;
+    const bool tiles_2d = want != 0 ? want != 1
+                          : op == Op::Forward ? plan->nX >= (unstaged ? 112 : 192) : plan->nX >= (ray ? 320 : 192);
     if (plan->nZ == 1 && !plan->has_occ && op != Op::Adjoint && tiles_2d && !noclip) {
         Args& a = it.a;
         a.in = in; a.out = out; a.trig = plan->d_trig; a.circle = plan->d_circle;

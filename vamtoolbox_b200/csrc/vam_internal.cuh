@@ -75,12 +75,12 @@ struct vam_parallel_plan {
     int occ_mode;
     double* d_occ64;
     uint8_t* d_ones;        // [nY][nX] all ones: the circle table of a backprojection without clipping
-    // angle tasks of the fast forward: (a, b) with b the angle 180 degrees from a
+    // angle tasks of the strip and 2-D tile forwards: (a, b) with b the angle 180 degrees from a
     // (both sampled from a's lattice), or b = -1 for an unpaired angle
     int2* d_tasks_paired;
     int n_tasks_paired;
     int2* d_tasks_single;   // (a, -1) for every angle
-    float* d_vol_scratch;   // [nY][nX][nZ] masked copy of the input (VAM_ABS_MASK)
+    float* d_vol_scratch;   // nZ == 1: [nY][nX] masked copy of the image (VAM_ABS_MASK, plain-load 2-D tiles)
     int* d_status;          // error bits the kernels record (VAM_STATUS_*), read by vam_parallel_status
     int4* d_bwd_btab;       // [blocks inside][nA][2] 2 x 2 block bin table (k_bwd_btable)
     int* d_bwd_bcidx;       // [(nY + 1) / 2][(nX + 1) / 2] compact block index, -1 outside the circle
