@@ -19,7 +19,7 @@ Reported beside the headline:
               arrays (engine="host"), the plain per-call GPU path;
   fwd_adj     forward + reference-parity backprojection pairs per second;
   roofline    of the dominant kernel of the step (the projector with the larger share of the
-              measured kernel time), HBM bytes it must move, and its on-chip gathered taps;
+              measured kernel time), HBM bytes it must move, and the bytes it loads on chip;
   cpu_baseline the reference's algorithm (oracle/vamoracle.c, OpenMP) on a bounded
               z-slab sample on this host's cores, extrapolated to the full volume.
 `--impl reference` prints the CPU reference arm's line instead.
@@ -109,6 +109,45 @@ def bclp_options(n_iter):
     from vamtoolbox_b200.optimize import Options
 
     return Options(method="BCLP", n_iter=n_iter, p=2, q=1, eps=0.1, learning_rate=1e-5, filter="ram-lak")
+
+
+def strip_pixels(n, angles, bins=2):
+    """Image pixels that the forward's strips of ``bins`` detector bins touch, per lattice sample: the distinct
+    taps of a strip over its samples (each is loaded once), averaged over a few of the angles."""
+    c0 = n // 2
+    j, k = np.meshgrid(np.arange(n), np.arange(n), indexing="ij")
+    total = samples = 0
+    for th in np.deg2rad(angles[:: max(len(angles) // 16, 1)]):
+        row = np.cos(th) * (k - c0) - np.sin(th) * (j - c0) + c0
+        col = np.sin(th) * (k - c0) + np.cos(th) * (j - c0) + c0
+        r0, q0 = np.floor(row).astype(np.int64), np.floor(col).astype(np.int64)
+        keys = []
+        for t in range(4):
+            r, q = r0 + (t >> 1), q0 + (t & 1)
+            ok = (r >= 0) & (r < n) & (q >= 0) & (q < n)
+            keys.append((((j // bins) * n + r) * n + q)[ok])
+        total += np.unique(np.concatenate(keys)).size
+        samples += n * n
+    return total / samples
+
+
+def block_rows(n, angles, inside):
+    """Detector rows that a 2 x 2 pixel block's interpolation reads per angle (each loaded once by the block-table
+    kernel), summed over the blocks that have a pixel inside the clip circle, averaged over a few of the angles."""
+    m = n + n % 2
+    x, y = np.meshgrid(np.arange(m) - n // 2, n // 2 - np.arange(m))
+    use = np.zeros((m, m), bool)
+    use[:n, :n] = inside
+    quads = lambda v: v.reshape(m // 2, 2, m // 2, 2).transpose(0, 2, 1, 3).reshape(-1, 4)
+    total = count = 0
+    for th in np.deg2rad(angles[:: max(len(angles) // 16, 1)]):
+        b = quads(np.floor(x * np.cos(th) - y * np.sin(th)).astype(np.int64))
+        u = quads(use)
+        rows = np.sort(np.concatenate([np.where(u, b, 1 << 40), np.where(u, b + 1, 1 << 40)], axis=1), axis=1)
+        new = np.concatenate([np.ones((len(rows), 1), bool), np.diff(rows, axis=1) > 0], axis=1)
+        total += int((new & (rows < 1 << 40)).sum())
+        count += 1
+    return total / count
 
 
 def count_angle_pairs(angles):
@@ -1297,20 +1336,21 @@ def run_ours(args):
     dom_ms = kmean[dom]
     achieved = (vol_bytes + sino_bytes) / (dom_ms * 1e-3) / 1e9
     if dom == "forward":
-        # taps the kernel gathers: 4 x 4 B per lattice sample and slice; angle pairs (a, a+180) share
-        # one lattice of (N+1)^2 samples (even N), unpaired angles use N^2; the reference's warp
-        # samples N^2 points per angle
+        # pixels the kernel loads: a strip of two detector bins loads each pixel it touches once, 4 B a
+        # slice; angle pairs (a, a+180) share one lattice of (N+1)^2 samples (even N), unpaired angles use
+        # N^2; the reference's warp reads four taps at N^2 points per angle
         pairs = count_angle_pairs(np.linspace(0, 360, na, endpoint=False))
         lattice = pairs * (n + 1 - n % 2) ** 2 + (na - 2 * pairs) * n * n
-        tap_bytes, ref_tap_bytes = 16.0 * lattice * n, 16.0 * n * n * na * n
+        per_sample = strip_pixels(n, np.linspace(0, 360, na, endpoint=False))
+        tap_bytes, ref_tap_bytes = 4.0 * per_sample * lattice * n, 16.0 * n * n * na * n
         dom_name = "forward projector (R1)"
     else:
-        # 2 detector rows x 4 B per (pixel, angle, slice): the kernel reads them for the pixels inside
-        # the clip circle, the reference's np.interp for every pixel
+        # 2 detector rows x 4 B per (pixel, angle, slice) in the reference's np.interp; the block-table kernel
+        # loads the distinct rows of each 2 x 2 block inside the clip circle once
         from vamtoolbox_b200.util.data import circle_inside_mask
 
-        inside = int(circle_inside_mask(ny, nx).sum())
-        tap_bytes, ref_tap_bytes = 8.0 * inside * na * n, 8.0 * ny * nx * na * n
+        rows = block_rows(n, np.linspace(0, 360, na, endpoint=False), circle_inside_mask(ny, nx))
+        tap_bytes, ref_tap_bytes = 4.0 * rows * na * n, 8.0 * ny * nx * na * n
         dom_name = "reference-parity backprojection (R2)"
     onchip_peak = 148 * 128 * 1.965e9 / 1e9     # L1/shared load bandwidth, nominal
     traffic = None
