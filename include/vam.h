@@ -191,6 +191,32 @@ typedef struct {
 int vam_parallel_set_tuning(vam_parallel_plan* plan, const vam_parallel_tuning* tuning);
 int vam_parallel_get_tuning(vam_parallel_plan* plan, vam_parallel_tuning* tuning);
 
+/* Which kernel a call would take, decided by the very rule the calls use, on
+ * the host alone (no plan, no device): the call is described by its sizes,
+ * the plan's state and the operands' alignment.  Returns what the call itself
+ * would return (VAM_ERR_ARG / VAM_ERR_NOTSUP for calls that are refused). */
+enum vam_kernel_kind {
+    VAM_KERNEL_FORWARD_STRIP = 0, VAM_KERNEL_FORWARD_GENERIC, VAM_KERNEL_BACKWARD_BATCHED,
+    VAM_KERNEL_BACKWARD_FAST, VAM_KERNEL_BACKWARD_GENERIC, VAM_KERNEL_ADJOINT_BLOCK, VAM_KERNEL_ADJOINT_GENERIC,
+    VAM_KERNEL_FORWARD_TILE, VAM_KERNEL_BACKWARD_TILE, VAM_KERNEL_BACKWARD_TABLE
+};
+typedef struct {
+    int32_t n, n_z, n_angles;   /* slice side, slices, angles */
+    int32_t angle_tasks;        /* angles less one for every pair 180 degrees apart */
+    int32_t absorption;         /* VAM_ABS_* */
+    int32_t occlusion, table;   /* an occlusion is set; the backprojection bin table is built */
+    int32_t op;                 /* VAM_OP_*, with VAM_OP_PADDED for padded input rows */
+    uint64_t in_address, out_address;  /* only their alignment counts (0: refused as null) */
+    vam_parallel_tuning tuning;
+} vam_parallel_call;
+typedef struct {
+    int32_t kernel;             /* vam_kernel_kind */
+    int32_t slices_per_lane;    /* 1, 4 or 8 (5 or 6 of the bin table) */
+    int32_t row_stride;         /* floats between the input's rows that the kernel steps by */
+    int32_t vector_loads, vector_stores;  /* it loads / stores float4s */
+} vam_parallel_route_info;
+int vam_parallel_route(const vam_parallel_call* call, vam_parallel_route_info* route);
+
 /* Batched calls over many plans (targets of uneven size, different angle
  * counts, 2-D slices next to 3-D volumes) in persistent launches fed by
  * device work queues: one launch per kernel-body family present in the list,

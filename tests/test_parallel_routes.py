@@ -1,0 +1,40 @@
+"""Which kernel a parallel-beam call takes (CPU only: the dispatch rule itself, on the host)."""
+import ctypes
+import itertools
+
+import pytest
+
+from vamtoolbox_b200 import _lib
+
+AUTO = dict(forward_vz=0, backward_vz=0, adjoint_vz=0, backward_batch=2, adjoint_table=1, backward_table=1,
+            forward_tma=1)
+ALIGNED = 1 << 20
+
+
+def route(n, nz, na, op, padded=False, absorption=_lib.ABS_NONE, occlusion=0, table=0, tasks=None, src=ALIGNED,
+          dst=ALIGNED, **tuning):
+    """(return code, ParallelRoute) of one call."""
+    t = _lib.ParallelTuning(*({**AUTO, **tuning}[k] for k, _ in _lib.ParallelTuning._fields_))
+    call = _lib.ParallelCall(n, nz, na, tasks or (na + 1) // 2, absorption, occlusion, table,
+                             op | (_lib.OP_PADDED if padded else 0), src, dst, t)
+    out = _lib.ParallelRoute()
+    return _lib.load().vam_parallel_route(ctypes.byref(call), ctypes.byref(out)), out
+
+
+TUNED = [dict(backward_vz=v, backward_batch=b, backward_table=t)
+         for v, b, t in itertools.product((0, 1, 4, 8), (1, 2, 4), (0, 1))]
+
+
+@pytest.mark.parametrize("nz", [5, 9, 33, 63, 65, 117, 130, 191, 193, 201, 255, 257, 318])
+@pytest.mark.parametrize("absorption", [_lib.ABS_NONE, _lib.ABS_MASK, _lib.ABS_RAY])
+def test_padded_backprojection_steps_by_its_padded_rows(nz, absorption):
+    """An input whose rows are padded goes to a body that steps by the padded rows and stores slice by slice where
+    the output's rows are not whole float4s, whatever the tuning, with and without a bin table."""
+    for tuned, table in itertools.product(TUNED, (0, 1)):
+        rc, r = route(201, nz, 240, _lib.OP_BACKWARD_REF, padded=True, absorption=absorption, table=table, **tuned)
+        assert rc == _lib.VAM_OK
+        assert r.kernel in (_lib.KERNEL_BACKWARD_TABLE, _lib.KERNEL_BACKWARD_GENERIC), (tuned, table, r.kernel)
+        assert r.row_stride == (nz + 3) // 4 * 4 and r.vector_loads and not r.vector_stores, (tuned, table)
+        # and what the unpadded call takes is unchanged by any of this: single floats
+        rc, r = route(201, nz, 240, _lib.OP_BACKWARD_REF, absorption=absorption, table=table, **tuned)
+        assert (rc, r.kernel, r.slices_per_lane, r.row_stride) == (_lib.VAM_OK, _lib.KERNEL_BACKWARD_GENERIC, 1, nz)

@@ -65,6 +65,21 @@ class ParallelTuning(ctypes.Structure):
                 ("forward_tma", _c_i32)]
 
 
+class ParallelCall(ctypes.Structure):
+    _fields_ = [("n", _c_i32), ("n_z", _c_i32), ("n_angles", _c_i32), ("angle_tasks", _c_i32),
+                ("absorption", _c_i32), ("occlusion", _c_i32), ("table", _c_i32), ("op", _c_i32),
+                ("in_address", ctypes.c_uint64), ("out_address", ctypes.c_uint64), ("tuning", ParallelTuning)]
+
+
+class ParallelRoute(ctypes.Structure):
+    _fields_ = [("kernel", _c_i32), ("slices_per_lane", _c_i32), ("row_stride", _c_i32), ("vector_loads", _c_i32),
+                ("vector_stores", _c_i32)]
+
+
+(KERNEL_FORWARD_STRIP, KERNEL_FORWARD_GENERIC, KERNEL_BACKWARD_BATCHED, KERNEL_BACKWARD_FAST, KERNEL_BACKWARD_GENERIC,
+ KERNEL_ADJOINT_BLOCK, KERNEL_ADJOINT_GENERIC, KERNEL_FORWARD_TILE, KERNEL_BACKWARD_TILE,
+ KERNEL_BACKWARD_TABLE) = range(10)
+
 OP_FORWARD, OP_BACKWARD_REF, OP_ADJOINT = 0, 1, 2
 OP_PADDED = 16
 
@@ -121,6 +136,7 @@ _SIGS = {
     "vam_parallel_prepare_padded": ([_vp, _vp], _c_int),
     "vam_parallel_apply_padded": ([_vp, _c_i32, _vp, _vp, _vp], _c_int),
     "vam_parallel_status": ([_vp, ctypes.POINTER(_c_i32)], _c_int),
+    "vam_parallel_route": ([ctypes.POINTER(ParallelCall), ctypes.POINTER(ParallelRoute)], _c_int),
     "vam_parallel_set_tuning": ([_vp, ctypes.POINTER(ParallelTuning)], _c_int),
     "vam_parallel_get_tuning": ([_vp, ctypes.POINTER(ParallelTuning)], _c_int),
     "vam_ray_record_count": ([_vp, _vp, _vp], _c_int),

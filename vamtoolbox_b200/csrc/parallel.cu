@@ -1750,7 +1750,12 @@ int fast_vz(int nZ, bool aligned, double min_eff) {
 // same body for many calls inside one persistent launch.  Both paths therefore
 // compute bit-identical results.
 // ---------------------------------------------------------------------------
-enum Kind : int { KF_FAST = 0, KF_GEN, KB_BATCHED, KB_FAST, KB_GEN, KA_BLOCK, KA_GEN, KF_2D, KB_2D, KB_BTABLE };
+enum Kind : int {
+    KF_FAST = VAM_KERNEL_FORWARD_STRIP, KF_GEN = VAM_KERNEL_FORWARD_GENERIC, KB_BATCHED = VAM_KERNEL_BACKWARD_BATCHED,
+    KB_FAST = VAM_KERNEL_BACKWARD_FAST, KB_GEN = VAM_KERNEL_BACKWARD_GENERIC, KA_BLOCK = VAM_KERNEL_ADJOINT_BLOCK,
+    KA_GEN = VAM_KERNEL_ADJOINT_GENERIC, KF_2D = VAM_KERNEL_FORWARD_TILE, KB_2D = VAM_KERNEL_BACKWARD_TILE,
+    KB_BTABLE = VAM_KERNEL_BACKWARD_TABLE
+};
 
 struct Item {
     int kind;
@@ -1796,11 +1801,12 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     const int zs = padded ? (plan->nZ + 3) & ~3 : plan->nZ;
     const bool aligned16 = (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
     const bool rows4 = zs % 4 == 0 && (((uintptr_t)in) & 15) == 0;
-    // slices per lane: tuned (1 = generic kernel, 4 or 8 = fast kernel) or automatic (0)
+    // slices per lane of the computed-bin backprojections (KB_BATCHED, KB_FAST): tuned (1 = generic kernel, 4 or 8)
+    // or automatic (0).  They step by the plan's own rows, so padded rows go to the table's kernel or the generic one.
     const bool fast_ok = (((uintptr_t)in | (padded ? (uintptr_t)0 : (uintptr_t)out)) & 31) == 0 && zs % 4 == 0;
     const int want = op == Op::Forward ? plan->tune_fwd_vz : (op == Op::BackwardRef ? plan->tune_bwd_vz : plan->tune_adj_vz);
     int vzf = 0;
-    if (fast_ok) {
+    if (fast_ok && !padded) {
         if (want == 4 || want == 8) vzf = want;
         else if (want == 0) vzf = fast_vz(plan->nZ, true, op == Op::Forward ? 0.45 : 0.74);
     }
@@ -2601,6 +2607,45 @@ extern "C" int vam_parallel_get_tuning(vam_parallel_plan* p, vam_parallel_tuning
     t->adjoint_table = p->tune_adj_table;
     t->backward_table = p->tune_bwd_table;
     t->forward_tma = p->tune_fwd_tma;
+    return VAM_OK;
+}
+
+// describe() on a plan of these properties; its device pointers are not read, only whether they are there
+extern "C" int vam_parallel_route(const vam_parallel_call* c, vam_parallel_route_info* out) {
+    clear_error();
+    VAM_REQUIRE(c && out, VAM_ERR_ARG, "vam_parallel_route: null argument");
+    VAM_REQUIRE(c->n > 0 && c->n_z > 0 && c->n_angles > 0 && c->angle_tasks > 0 && c->angle_tasks <= c->n_angles,
+                VAM_ERR_SHAPE, "vam_parallel_route: sizes must be positive");
+    const int op = c->op & ~VAM_OP_PADDED;
+    VAM_REQUIRE(op >= VAM_OP_FORWARD && op <= VAM_OP_ADJOINT, VAM_ERR_ARG, "vam_parallel_route: unknown op");
+    alignas(16) static char there[16];
+    vam_parallel_plan p;
+    std::memset(&p, 0, sizeof(p));
+    p.nY = p.nX = c->n; p.nZ = c->n_z; p.nA = c->n_angles; p.C = c->n / 2;
+    p.abs_mode = c->absorption;
+    p.has_occ = c->occlusion;
+    p.n_tasks_paired = c->angle_tasks;
+    p.d_mask = p.d_vol_scratch = reinterpret_cast<float*>(there);
+    if (c->n_z == 1) p.d_img_pad = reinterpret_cast<float*>(there);
+    if (c->table) p.d_bwd_btab = reinterpret_cast<int4*>(there);
+    const int rc = vam_parallel_set_tuning(&p, &c->tuning);
+    if (rc != VAM_OK) return rc;
+    Item it;
+    const Op o = op == VAM_OP_FORWARD ? Op::Forward : (op == VAM_OP_BACKWARD_REF ? Op::BackwardRef : Op::Adjoint);
+    const int rd = describe(&p, o, reinterpret_cast<const float*>((uintptr_t)c->in_address),
+                            reinterpret_cast<float*>((uintptr_t)c->out_address), it, "vam_parallel_route", false,
+                            (c->op & VAM_OP_PADDED) != 0);
+    if (rd != VAM_OK) return rd;
+    out->kernel = it.kind;
+    out->slices_per_lane = it.kind == KF_2D || it.kind == KB_2D ? 1 : it.vz;
+    // the bodies that step by the padded rows (zs, vs); the others step by the plan's slices
+    const bool steps = it.kind == KB_BTABLE || it.kind == KB_GEN || it.kind == KA_BLOCK;
+    out->row_stride = it.kind == KF_FAST ? it.f.vs : steps ? it.a.zs : c->n_z;
+    const bool strip = it.kind == KF_FAST || it.kind == KA_BLOCK;
+    out->vector_loads = strip ? it.vec : it.vz >= 4;
+    out->vector_stores = strip ? it.vec && (it.kind == KF_FAST ? it.f.whole : it.a.whole)
+                         : it.vz >= 4 && (!(it.kind == KB_BTABLE || it.kind == KB_GEN) || it.a.whole ||
+                                          (it.kind == KB_BTABLE && c->n_z % (32 * it.vz) == 0));
     return VAM_OK;
 }
 
