@@ -156,8 +156,8 @@ int vam_parallel_adjoint(vam_parallel_plan* plan, const float* sino_dev, float* 
  * vam_pad_rows copies `rows` rows of nz floats into rows of nz rounded up to a
  * multiple of four, the padding zero (out: 16-byte aligned).
  * vam_parallel_apply_padded runs op (VAM_OP_*) of the plan on such an input
- * (volume rows for the forward, sinogram rows otherwise); the output's rows are
- * the plan's own.  vam_parallel_prepare_padded builds the bin table that the
+ * (volume rows for the forward, sinogram rows otherwise; in: 16-byte aligned,
+ * VAM_ERR_ARG otherwise); the output's rows are the plan's own.  vam_parallel_prepare_padded builds the bin table that the
  * padded backprojection reads (allocates: before any stream capture).
  * VAM_ERR_NOTSUP for what the padded kernels do not serve: an
  * occlusion, a forward or transpose of few slices or with its generic kernel

@@ -38,3 +38,16 @@ def test_padded_backprojection_steps_by_its_padded_rows(nz, absorption):
         # and what the unpadded call takes is unchanged by any of this: single floats
         rc, r = route(201, nz, 240, _lib.OP_BACKWARD_REF, absorption=absorption, table=table, **tuned)
         assert (rc, r.kernel, r.slices_per_lane, r.row_stride) == (_lib.VAM_OK, _lib.KERNEL_BACKWARD_GENERIC, 1, nz)
+
+
+@pytest.mark.parametrize("nz", [8, 33, 64, 67, 130, 256])
+@pytest.mark.parametrize("op", [_lib.OP_FORWARD, _lib.OP_BACKWARD_REF, _lib.OP_ADJOINT])
+def test_padded_rows_are_checked_for_alignment(nz, op):
+    """Padded rows are read as float4s: an input off a 16-byte boundary is refused.  The output may lie anywhere
+    (a multiple of four floats only): where it is off such a boundary it is stored slice by slice."""
+    for off in (4, 8, 12):
+        assert route(96, nz, 90, op, padded=True, table=1, src=ALIGNED + off)[0] == _lib.VAM_ERR_ARG
+    for off, tuned in itertools.product((4, 8, 12), TUNED):
+        rc, r = route(96, nz, 90, op, padded=True, table=1, dst=ALIGNED + off, **tuned)
+        assert rc == _lib.VAM_OK or (nz == 8 and op != _lib.OP_BACKWARD_REF and rc == _lib.VAM_ERR_NOTSUP)
+        assert rc != _lib.VAM_OK or not r.vector_stores, (off, tuned, r.kernel)

@@ -1792,6 +1792,8 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
              bool noclip = false, bool padded = false) {
     VAM_REQUIRE(plan && in && out, VAM_ERR_ARG, std::string(name) + ": null argument");
     VAM_REQUIRE(!padded || (plan->nZ > 1 && !noclip), VAM_ERR_NOTSUP, std::string(name) + ": padded rows are not served here");
+    VAM_REQUIRE(!padded || (((uintptr_t)in) & 15) == 0, VAM_ERR_ARG,
+                std::string(name) + ": padded rows must be 16-byte aligned");
     VAM_REQUIRE(!noclip || plan->d_ones, VAM_ERR_ARG, std::string(name) + ": no all-ones circle table");
     std::memset(&it, 0, sizeof(it));
     it.cost = (long long)plan->nY * plan->nX * plan->nZ * plan->nA;
@@ -1803,7 +1805,8 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     const bool rows4 = zs % 4 == 0 && (((uintptr_t)in) & 15) == 0;
     // slices per lane of the computed-bin backprojections (KB_BATCHED, KB_FAST): tuned (1 = generic kernel, 4 or 8)
     // or automatic (0).  They step by the plan's own rows, so padded rows go to the table's kernel or the generic one.
-    const bool fast_ok = (((uintptr_t)in | (padded ? (uintptr_t)0 : (uintptr_t)out)) & 31) == 0 && zs % 4 == 0;
+    // (an output whose rows are no whole float4s is stored slice by slice and may lie anywhere)
+    const bool fast_ok = (((uintptr_t)in | (plan->nZ % 4 ? (uintptr_t)0 : (uintptr_t)out)) & 31) == 0 && zs % 4 == 0;
     const int want = op == Op::Forward ? plan->tune_fwd_vz : (op == Op::BackwardRef ? plan->tune_bwd_vz : plan->tune_adj_vz);
     int vzf = 0;
     if (fast_ok && !padded) {
