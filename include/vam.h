@@ -157,13 +157,16 @@ int vam_parallel_adjoint(vam_parallel_plan* plan, const float* sino_dev, float* 
  * multiple of four, the padding zero (out: 16-byte aligned).
  * vam_parallel_apply_padded runs op (VAM_OP_*) of the plan on such an input
  * (volume rows for the forward, sinogram rows otherwise; in: 16-byte aligned,
- * VAM_ERR_ARG otherwise); the output's rows are the plan's own.  vam_parallel_prepare_padded builds the bin table that the
- * padded backprojection reads (allocates: before any stream capture).
- * VAM_ERR_NOTSUP for what the padded kernels do not serve: an
- * occlusion, a forward or transpose of few slices or with its generic kernel
- * selected by the tuning, a single slice. */
+ * VAM_ERR_ARG otherwise); the output's rows are the plan's own.
+ * vam_parallel_prepare_padded builds the bin table that the padded
+ * backprojection reads (allocates: before any stream capture).
+ * VAM_ERR_NOTSUP for what the padded kernels do not serve: an occlusion, a
+ * forward or transpose that its generic kernel takes (few slices, 2^31 volume
+ * elements, the tuning), a single slice.  vam_parallel_serves_padded is 1 where
+ * op is served and the padded input stays below 2^31 elements (8 GB), else 0. */
 int vam_pad_rows(const float* x_dev, int64_t rows, int32_t nz, float* out_dev, vam_stream_t stream);
 int vam_parallel_prepare_padded(vam_parallel_plan* plan, vam_stream_t stream);
+int vam_parallel_serves_padded(vam_parallel_plan* plan, int32_t op);
 int vam_parallel_apply_padded(vam_parallel_plan* plan, int32_t op, const float* in_dev, float* out_dev,
                               vam_stream_t stream);
 
@@ -214,6 +217,7 @@ typedef struct {
     int32_t slices_per_lane;    /* 1, 4 or 8 (5 or 6 of the bin table) */
     int32_t row_stride;         /* floats between the input's rows that the kernel steps by */
     int32_t vector_loads, vector_stores;  /* it loads / stores float4s */
+    int32_t pads;               /* vam_parallel_serves_padded of such a plan (also set for refused calls) */
 } vam_parallel_route_info;
 int vam_parallel_route(const vam_parallel_call* call, vam_parallel_route_info* route);
 

@@ -51,3 +51,38 @@ def test_padded_rows_are_checked_for_alignment(nz, op):
         rc, r = route(96, nz, 90, op, padded=True, table=1, dst=ALIGNED + off, **tuned)
         assert rc == _lib.VAM_OK or (nz == 8 and op != _lib.OP_BACKWARD_REF and rc == _lib.VAM_ERR_NOTSUP)
         assert rc != _lib.VAM_OK or not r.vector_stores, (off, tuned, r.kernel)
+
+
+@pytest.mark.parametrize("n,nz,na", [(2048, 513, 8), (1300, 1301, 30), (201, 117, 240), (64, 33, 90), (3000, 31, 30000),
+                                     (96, 9, 90)])
+def test_rows_are_padded_only_where_the_padded_kernels_serve_the_call(n, nz, na, monkeypatch):
+    """Whether a plan pads its input is the dispatch's own answer, so no padded call is refused; a padded copy has
+    fewer than 2^31 elements.  A volume of 2^31 elements or more goes unpadded to the generic forward."""
+    import types
+
+    import numpy as np
+
+    from vamtoolbox_b200.projector import Projector3DParallel as module
+
+    forms = itertools.product((_lib.OP_FORWARD, _lib.OP_BACKWARD_REF, _lib.OP_ADJOINT),
+                              (_lib.ABS_NONE, _lib.ABS_MASK, _lib.ABS_RAY), (0, 1), (0, 1),
+                              (dict(), dict(forward_vz=1, adjoint_vz=1, backward_vz=1), dict(forward_vz=8, adjoint_vz=4)))
+    padded = 0
+    for op, absorption, occlusion, table, tuning in forms:
+        form = dict(absorption=absorption, occlusion=occlusion, table=table, **tuning)
+        plan = module.ParallelPlan.__new__(module.ParallelPlan)
+        plan.shape_vol, plan.angles, plan._h = (n, n, nz), np.zeros(na), None
+        plan.pad_from, plan.pad_backward_from = 0, 0
+        serves = route(n, nz, na, op, **form)[1].pads
+        monkeypatch.setattr(module._lib, "load",
+                            lambda: types.SimpleNamespace(vam_parallel_serves_padded=lambda handle, code: serves))
+        pads = plan._pads(op)
+        monkeypatch.undo()
+        rc, r = route(n, nz, na, op, padded=pads, **form)
+        assert rc == _lib.VAM_OK, (op, form)
+        if pads:
+            padded += 1
+            assert n * (n if op == _lib.OP_FORWARD else na) * ((nz + 3) // 4 * 4) < 2 ** 31, (op, form)
+        elif op == _lib.OP_FORWARD and n * n * nz >= 2 ** 31:
+            assert r.kernel == _lib.KERNEL_FORWARD_GENERIC, form
+    assert padded or n * n * nz >= 2 ** 31 or n * na * nz >= 2 ** 31

@@ -73,7 +73,7 @@ class ParallelCall(ctypes.Structure):
 
 class ParallelRoute(ctypes.Structure):
     _fields_ = [("kernel", _c_i32), ("slices_per_lane", _c_i32), ("row_stride", _c_i32), ("vector_loads", _c_i32),
-                ("vector_stores", _c_i32)]
+                ("vector_stores", _c_i32), ("pads", _c_i32)]
 
 
 (KERNEL_FORWARD_STRIP, KERNEL_FORWARD_GENERIC, KERNEL_BACKWARD_BATCHED, KERNEL_BACKWARD_FAST, KERNEL_BACKWARD_GENERIC,
@@ -134,6 +134,7 @@ _SIGS = {
     "vam_parallel_prepare_backward": ([_vp, _vp], _c_int),
     "vam_pad_rows": ([_vp, _c_i64, _c_i32, _vp, _vp], _c_int),
     "vam_parallel_prepare_padded": ([_vp, _vp], _c_int),
+    "vam_parallel_serves_padded": ([_vp, _c_i32], _c_int),
     "vam_parallel_apply_padded": ([_vp, _c_i32, _vp, _vp, _vp], _c_int),
     "vam_parallel_status": ([_vp, ctypes.POINTER(_c_i32)], _c_int),
     "vam_parallel_route": ([ctypes.POINTER(ParallelCall), ctypes.POINTER(ParallelRoute)], _c_int),

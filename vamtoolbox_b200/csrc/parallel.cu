@@ -2633,6 +2633,7 @@ extern "C" int vam_parallel_route(const vam_parallel_call* c, vam_parallel_route
     if (c->table) p.d_bwd_btab = reinterpret_cast<int4*>(there);
     const int rc = vam_parallel_set_tuning(&p, &c->tuning);
     if (rc != VAM_OK) return rc;
+    out->pads = vam_parallel_serves_padded(&p, op);
     Item it;
     const Op o = op == VAM_OP_FORWARD ? Op::Forward : (op == VAM_OP_BACKWARD_REF ? Op::BackwardRef : Op::Adjoint);
     const int rd = describe(&p, o, reinterpret_cast<const float*>((uintptr_t)c->in_address),
@@ -2774,6 +2775,20 @@ extern "C" int vam_pad_rows(const float* x, int64_t rows, int32_t nz, float* out
         x, reinterpret_cast<float4*>(out), n4, nz, nz4);
     VAM_CHECK_LAUNCH("vam_pad_rows");
     return VAM_OK;
+}
+
+// the dispatch's own answer, so that a caller that pads never meets a refusal
+extern "C" int vam_parallel_serves_padded(vam_parallel_plan* p, int32_t op) {
+    clear_error();
+    if (!p || op < VAM_OP_FORWARD || op > VAM_OP_ADJOINT) return 0;
+    const Op o = op == VAM_OP_FORWARD ? Op::Forward : (op == VAM_OP_BACKWARD_REF ? Op::BackwardRef : Op::Adjoint);
+    const long long row = (p->nZ + 3) & ~3;
+    if (p->nY * (long long)(o == Op::Forward ? p->nX : p->nA) * row >= (1LL << 31)) return 0;
+    alignas(32) static float aligned[8];
+    Item it;
+    const bool ok = describe(p, o, aligned, aligned, it, "vam_parallel_serves_padded", false, true) == VAM_OK;
+    clear_error();
+    return ok;
 }
 
 extern "C" int vam_parallel_apply_padded(vam_parallel_plan* p, int32_t op, const float* in, float* out,

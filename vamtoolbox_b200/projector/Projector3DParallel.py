@@ -126,7 +126,6 @@ class ParallelPlan:
         h = ctypes.c_void_p()
         _lib.call("vam_parallel_plan_create", ctypes.byref(geom), ctypes.byref(h))
         self._h = h
-        self._tuning = dict(_DEFAULT_TUNING)
         if int(n_z) >= 64:
             if int(n_z) % 4 == 0:
                 self.prepare_backward()
@@ -138,7 +137,6 @@ class ParallelPlan:
         with torch.cuda.device(self.device):
             _lib.call("vam_parallel_set_absorption", self._h, _lib.ABS_NONE, None, 0.0, 1.0, self._stream())
             _lib.call("vam_parallel_clear_occlusion", self._h)
-        self._tuning = dict(_DEFAULT_TUNING)
         self.set_tuning(dict(_DEFAULT_TUNING))
 
     @property
@@ -201,14 +199,13 @@ class ParallelPlan:
     def _pads(self, op):
         """Whether ``op`` (OP_*) reads a copy of its input with the rows of slices padded to a multiple of four
         (16-byte loads instead of 4-byte ones; the copy is a pass over the input).  For volumes whose slice
-        count is not one, where the padded kernels serve the call."""
+        count is not one, where the padded kernels serve the call: the C side's dispatch says so itself."""
         ny, nx, nz = self.shape_vol
-        if nz % 4 == 0 or nz < 5 or self.has_occlusion:
+        if nz % 4 == 0 or nz < 5:
             return False
-        size = ny * nx * nz * self.angles.size
-        if op == _lib.OP_BACKWARD_REF:
-            return size >= self.pad_backward_from
-        return size >= self.pad_from and self._tuning["forward_vz" if op == _lib.OP_FORWARD else "adjoint_vz"] != 1
+        if ny * nx * nz * self.angles.size < (self.pad_backward_from if op == _lib.OP_BACKWARD_REF else self.pad_from):
+            return False
+        return bool(_lib.load().vam_parallel_serves_padded(self._h, op))
 
     def _padded(self, t):
         """t ([a, b, nz]) with zero slices up to a multiple of four: a workspace of the current stream."""
@@ -252,7 +249,6 @@ class ParallelPlan:
         cur.update({k: int(v) for k, v in tuning.items()})
         t = _lib.ParallelTuning(*(cur[k] for k in self._TUNING_FIELDS))
         _lib.call("vam_parallel_set_tuning", self._h, ctypes.byref(t))
-        self._tuning = cur
 
     def get_tuning(self):
         t = _lib.ParallelTuning()
