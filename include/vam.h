@@ -228,11 +228,11 @@ int vam_parallel_route(const vam_parallel_call* call, vam_parallel_route_info* r
  * occupancy).  Each work item is one forward / backward_ref / adjoint
  * call exactly as the single-plan entry points describe it, and produces
  * bit-identical results; items run concurrently, so no item may read another
- * item's output or write another item's input or output.  A forward that
- * stages its input in its plan's scratch (mask mode; a 2-D slice whose width
- * is not a multiple of four or whose input is not 16-byte aligned) makes that
- * plan appear at most once per batch with VAM_OP_FORWARD: a list with two
- * such calls of one plan is refused (VAM_ERR_ARG).
+ * item's output or write another item's input or output.  A 2-D tile forward
+ * that stages its image in its plan's scratch (mask mode, a width that is not
+ * a multiple of four, an input that is not 16-byte aligned) makes that plan
+ * appear at most once per batch with VAM_OP_FORWARD: a list with two such
+ * calls of one plan is refused (VAM_ERR_ARG).
  *
  * The calls' descriptions travel by value in the launch's parameters (48
  * calls per launch; longer lists and further families become further

@@ -214,3 +214,16 @@ def test_multi_target_bclp_matches_one_at_a_time(schedule):
         assert np.array_equal(g, g1)
         assert np.array_equal(dose, s.dose)
         assert np.allclose(np.asarray(loss), np.asarray(s.logs.loss), rtol=0, atol=0, equal_nan=True)
+
+
+@pytest.mark.parametrize("nz", [8, 16, 45, 64, 130])
+def test_batch_takes_masked_volume_forwards_of_one_plan_twice(nz):
+    """A masked volume's forward keeps nothing in its plan, so a list may hold a plan's forward more than once."""
+    rng = np.random.default_rng(nz)
+    p = ParallelPlan(40, 40, nz, np.linspace(0, 360, 20, endpoint=False))
+    p.set_absorption("mask", mask=rng.uniform(0.2, 1.0, (40, 40)))
+    x = [torch.as_tensor(rng.uniform(0, 1, p.shape_vol), dtype=torch.float32, device="cuda") for _ in range(2)]
+    out = [torch.full(p.shape_sino, np.nan, device="cuda") for _ in range(2)]
+    ProjectionBatch().submit([(p, "forward", x[0], out[0]), (p, "forward", x[1], out[1])])
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, p.forward(v)) for o, v in zip(out, x))

@@ -28,8 +28,9 @@ class ProjectionBatch:
     ``submit(work)`` runs the calls on the current stream (capturable in a
     CUDA graph: the call descriptions travel in the launch parameters);
     ``prepare(work)`` only validates a list.  Calls of one batch run
-    concurrently: no call may read another's output, and a plan appears at
-    most once as a forward (its mask-mode scratch volume is per plan).
+    concurrently: no call may read another's output, and a single-slice plan
+    whose forward stages its image appears at most once as a forward (the
+    staged image is per plan).
     """
 
     def __init__(self, device=None):

@@ -1767,8 +1767,8 @@ struct Item {
     long long tstart;  // first ticket (virtual block) of the call inside a batch launch
     long long cost;    // estimated time of the call (batch ordering)
     int family;        // body family (k_batch instances): a bit of the FAM mask
-    // pre-pass of the fast forward in mask mode: pre_out = mask * pre_in; of the 2-D tile forward
-    // (pre_wp > 0): rows of pre_w floats of (mask *) pre_in into rows of pre_wp floats of pre_out
+    // pre-pass of the 2-D tile forward: pre_out = mask * pre_in, or (pre_wp > 0) rows of pre_w floats of
+    // (mask *) pre_in into rows of pre_wp floats of pre_out
     const float* pre_in;
     const float* pre_mask;
     float* pre_out;
@@ -1779,7 +1779,6 @@ struct Item {
     const int4* btab4;  // KB_BTABLE: the plan's 2 x 2 block bin table and its block index
     const int* bcidx;
     int* status;       // the plan's status word (kernels with bounded waits record timeouts there)
-    const void* once;  // storage of the plan that a batch lists at most once (null: none)
     int tma, vec;      // vec (KF_FAST): 1 when the rows load as float4s.  KF_2D: tma is 1 when tmap describes a.in and the tiles are staged by TMA loads
     CUtensorMap tmap;   // read from parameter space, as a direct launch's __grid_constant__ argument
 };
@@ -1842,13 +1841,11 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
                 it.pre_in = in; it.pre_mask = a.mask; it.pre_out = plan->d_img_pad;
                 it.pre_npix = (long long)plan->nY * plan->nX; it.pre_nz = 1;
                 it.pre_w = plan->nX; it.pre_wp = wp;
-                it.once = it.pre_out;
                 a.in = plan->d_img_pad;
                 a.mask = nullptr;
             } else if (a.mask) {  // stage the masked image once per call instead of per tile
                 it.pre_in = in; it.pre_mask = plan->d_mask; it.pre_out = plan->d_vol_scratch;
                 it.pre_npix = (long long)plan->nY * plan->nX; it.pre_nz = 1;
-                it.once = it.pre_out;
                 a.in = plan->d_vol_scratch;
                 a.mask = nullptr;
             }
@@ -1900,7 +1897,6 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         const int strips = (plan->nX + 1 + bins - 1) / bins, sub = kWarpsPerBlock >> a.ashift;
         it.gx = (unsigned)(((strips + sub - 1) / sub) * a.zchunks);
         it.gy = (unsigned)((a.ntasks + (1 << a.ashift) - 1) >> a.ashift);
-        it.once = a.mask;
         return VAM_OK;
     }
     // pixel blocks for the matched transpose: as the strips
@@ -2984,9 +2980,9 @@ int batch_prepare(vam_batch* b, const vam_work* work, int32_t n) {
         items[i].cost = (long long)std::llround((double)items[i].cost * time_weight(items[i]));
     }
     // a staged forward writes its plan's scratch: two such calls of one plan would share it
-    std::vector<const void*> staged;
+    std::vector<const float*> staged;
     for (const Item& it : items)
-        if (it.once) staged.push_back(it.once);
+        if (it.pre_out) staged.push_back(it.pre_out);
     std::sort(staged.begin(), staged.end());
     VAM_REQUIRE(std::adjacent_find(staged.begin(), staged.end()) == staged.end(), VAM_ERR_ARG,
                 "vam_batch: two forwards of one plan stage their input into the same scratch");
