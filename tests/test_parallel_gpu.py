@@ -717,3 +717,42 @@ def test_autotune_of_a_padded_slice_count(tmp_path, monkeypatch):
     assert np.abs(p.backward_ref(dev(b)).cpu().numpy() - ref).max() <= 60 * 2.0 ** -24 * ref.max()
     assert relL2(p.forward(dev(x)).cpu().numpy(), O.parallel_forward(x, ang)) < TOL
     assert relL2(p.adjoint(dev(b)).cpu().numpy(), O.parallel_adjoint(b, ang)) < TOL
+
+
+@pytest.mark.parametrize("n,nz", [(24, 65), (33, 67), (40, 117), (21, 130), (31, 165), (26, 201), (17, 261)])
+@pytest.mark.parametrize("absn", [None, "mask"])
+def test_padded_table_backprojection_is_as_exact_as_the_generic_kernel(n, nz, absn):
+    """Padded rows summed from the bin table against the generic kernel, whose lanes share a pixel's angles: bins on
+    integers, the detector's ends (angles on the axes), every slice of the last chunk.  A run adds at most 16 values, each
+    interpolated with three roundings, and the sum of the runs and the mask's product round once: 21 2^-24 of the
+    sum of the magnitudes.  The error's norm is no larger than the generic kernel's but for the last rounding of
+    either (2^-25.5 in the mean).  An infinity and a NaN reach the pixels they reach there (an infinite lower row
+    gives an infinity as in np.interp, where the generic kernel's r0 + w (r1 - r0) gives a NaN)."""
+    from vamtoolbox_b200 import _lib
+
+    rng = np.random.default_rng(n * nz + 3)
+    ang = np.concatenate([np.array([0.0, 45.0, 90.0, 180.0, 270.0, 359.9]), rng.uniform(0, 360, 33)])
+    p = plan_for((n, n, nz), ang)
+    p.pad_backward_from = 0
+    assert p.has_backward_table and p._pads(_lib.OP_BACKWARD_REF)
+    oabs = None
+    if absn == "mask":
+        oabs = ("mask", rng.uniform(0.2, 1.0, (n, n)).astype(np.float32).astype(np.float64))
+        p.set_absorption("mask", mask=oabs[1])
+    b = rng.uniform(-0.3, 1, (n, ang.size, nz)).astype(np.float32)
+    bi = b.copy()
+    bi[n // 2, 0, nz // 2], bi[n // 3, 7, 0], bi[n - 1, 2, nz - 1], bi[n // 2 + 1, 1, 1] = np.inf, np.nan, np.inf, -np.inf
+    ref = O.parallel_backward_ref(b.astype(np.float64), ang, absorption=oabs)
+    size = O.parallel_backward_ref(np.abs(b).astype(np.float64), ang, absorption=oabs)
+
+    def generic(src):
+        out = torch.empty(p.shape_vol, device="cuda")
+        _lib.call("vam_parallel_backward_ref", p.handle, _lib.ptr(src), _lib.ptr(out), p._stream())
+        return out
+
+    for vz in (0, 4, 8):
+        p.set_tuning({"backward_vz": vz})
+        got = p.backward_ref(dev(b)).cpu().numpy()
+        assert (np.abs(got - ref) <= 21 * 2.0 ** -24 * size + 1e-30).all(), vz
+        assert relL2(got, ref) <= relL2(generic(dev(b)).cpu().numpy(), ref) + 2.0 ** -25.5, vz
+        assert torch.equal(p.backward_ref(dev(bi)).isfinite(), generic(dev(bi)).isfinite()), vz

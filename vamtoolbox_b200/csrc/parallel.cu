@@ -500,15 +500,20 @@ __global__ void __launch_bounds__(256, 6) k_backward_batched8(Args a) {
 // weights.  k_backward_blk loads the block's rows once per warp and runs, per
 // pixel, (1 - w) * row j0 then w * row j0 + 1 as packed f32x2 FMAs (two fmaf
 // roundings each), the order of k_backward_batched8, so the sums are
-// bit-identical to it for finite data.  The warp walks the rows in passes
+// bit-identical to it for finite data.  Rows padded to a multiple of four (slice
+// counts that are not one) are summed in runs instead, and a bin on an integer
+// adds its one row there (kBlkSingle).
+// The warp walks the rows in passes
 // d = 0 .. span (rows d and d + 1 live), applying each pixel in the pass of
 // its own j0, so at most three rows are held in registers.  It replaced a
 // per-pixel table kernel (8-byte entries, two rows per pixel and angle, L1
 // bound at 90 %): 1.33 -> 0.92 ms at 256^3 x 360.
 // ---------------------------------------------------------------------------
+constexpr int kBlkSingle = 1 << 14;  // code bit: some pixel's bits are 7, its weight's place holds the one row it adds
+
 __global__ void __launch_bounds__(256) k_bwd_btable(const double4* __restrict__ trig, const int* __restrict__ blist,
                                                     const int* __restrict__ cidx, int4* __restrict__ tab, int nbc,
-                                                    int nA, int nY, int nX, int nZ, int C) {
+                                                    int nA, int nY, int nX, int nZ, int C, int single) {
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;  // over (block, angle), angle fastest
     if (idx >= (long)nbc * nA) return;
     const int th = (int)(idx % nA);
@@ -518,7 +523,7 @@ __global__ void __launch_bounds__(256) k_bwd_btable(const double4* __restrict__ 
     const double4 tr = trig[th];
     int j0s[4];
     float ws[4];
-    bool val[4];
+    bool val[4], last[4];
     int jmin = 1 << 30, jmax = -1;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -526,6 +531,7 @@ __global__ void __launch_bounds__(256) k_bwd_btable(const double4* __restrict__ 
         val[q] = i < nY && j < nX && cidx[(size_t)i * nX + j] >= 0;
         j0s[q] = 0;
         ws[q] = 0.f;
+        last[q] = false;
         if (val[q]) {
             const double X = (double)(j - C), Y = (double)(i - C);
             const double t = __dsub_rn(__dmul_rn(X, tr.x), __dmul_rn(Y, tr.y));
@@ -534,7 +540,7 @@ __global__ void __launch_bounds__(256) k_bwd_btable(const double4* __restrict__ 
             } else {
                 const double ft = floor(t);
                 const int j0 = (int)ft + C;
-                if (j0 == nY - 1) { j0s[q] = nY - 2; ws[q] = 1.f; }
+                if (j0 == nY - 1) { j0s[q] = nY - 2; ws[q] = 1.f; last[q] = true; }
                 else { j0s[q] = j0; ws[q] = (float)(t - ft); }
                 jmin = min(jmin, j0s[q]);
                 jmax = max(jmax, j0s[q]);
@@ -549,7 +555,15 @@ __global__ void __launch_bounds__(256) k_bwd_btable(const double4* __restrict__ 
     int code = jmax - jmin;  // <= 2
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-        if (val[q]) code |= (1 | ((j0s[q] - jmin) << 1)) << (2 + 3 * q);
+        if (val[q]) {
+            int bits = 1 | ((j0s[q] - jmin) << 1);
+            if (single && (ws[q] == 0.f || last[q])) {  // a bin on an integer: the row itself, from the block's first
+                bits = 7;
+                ws[q] = __int_as_float(j0s[q] - jmin + (last[q] ? 1 : 0));
+                code |= kBlkSingle;
+            }
+            code |= bits << (2 + 3 * q);
+        }
     tab[2 * idx] = make_int4(jmin * nA * nZ + th * nZ, code, __float_as_int(ws[0]), __float_as_int(ws[1]));
     tab[2 * idx + 1] = make_int4(__float_as_int(ws[2]), __float_as_int(ws[3]), 0, 0);
 }
@@ -601,18 +615,45 @@ __device__ __forceinline__ void lerp_rows(unsigned long long (&acc)[(VZ + 1) / 2
     if constexpr (VZ == 6 || VZ == 5) fma_pair(acc[2], w1, r1.t.x, r1.t.y);
 }
 
+// acc (slice pairs) += one row
+template <int VZ>
+__device__ __forceinline__ void add_row(unsigned long long (&acc)[(VZ + 1) / 2], const RowV<VZ>& r) {
+#pragma unroll
+    for (int q = 0; q < VZ / 4; ++q) {
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc[2 * q]) : "l"(pk_pair(r.v[q].x, r.v[q].y)));
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc[2 * q + 1]) : "l"(pk_pair(r.v[q].z, r.v[q].w)));
+    }
+}
+
+// sum += acc; with rest, what the rounding drops stays in acc for the next time
+__device__ __forceinline__ void carry_pair(unsigned long long& sum, unsigned long long& acc, bool rest) {
+    unsigned long long t, d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(sum), "l"(acc));
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(t), "l"(sum));
+    asm("sub.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(d));
+    if (!rest) acc = 0ull;
+    sum = t;
+}
+
 // one warp per (2 x 2 block, z chunk of 32 VZ slices); FULL: nZ a multiple of 32 VZ, else the lanes
-// past nZ in the last chunk load and store nothing.  The table entries
+// past nZ in the last chunk load and store nothing; UNEVEN: padded rows of a slice count that is not a multiple of
+// four (sums in runs, slices stored one by one).  The table entries
 // arrive 32 angles at a time (lane l fetches angle k0 + l's 32 bytes, the next chunk in flight while
 // this one is read), so no angle waits for its entry: eight slices per lane by cp.async into the warp's
 // two shared-memory slots (no registers held: the body fits 80 registers, three CTAs per SM; 1.19 ->
 // 0.92 ms at 256^3 x 360 against entries in registers at two CTAs), four slices in registers,
 // broadcast by shuffles (0.21 -> 0.17 ms at 128^3 x 360 against the shared-memory slots).
 constexpr int kBlkEnt = 64;  // int4 per slot: 32 angles x 32 bytes
-template <int VZ, bool FULL>
+
+// a warp's two slots (one array for every instance that a batch kernel holds)
+__device__ __forceinline__ int4* blk_entries(int wp) {
+    __shared__ __align__(16) int4 s_ent[kWarpsPerBlock][2][kBlkEnt];
+    return &s_ent[wp][0][0];
+}
+
+template <int VZ, bool FULL, bool UNEVEN = false>
 __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* __restrict__ tab,
                                                     const int* __restrict__ bcidx, unsigned bx) {
-    __shared__ __align__(16) int4 s_ent[VZ == 8 ? kWarpsPerBlock : 1][2][kBlkEnt];
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     // a CTA: 4 x 2 blocks (8 x 4 pixels, one block per warp) of one z chunk, so the warps of a CTA
     // read overlapping detector rows for the same angle at about the same time
@@ -632,9 +673,25 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
     for (int q = 0; q < 4; ++q)
 #pragma unroll
         for (int e = 0; e < NP; ++e) acc[q][e] = 0ull;
+    // UNEVEN: the runs of angles summed up so far, acc being the current run.  The generic kernel, which these slice
+    // counts took before, spreads a pixel's angles over up to four lanes (two above 128 slices); a running sum over
+    // all angles is less exact (128^2 x 65 x 180 angles, relative to float64: 2.5e-7 against 5.9e-8; 201^2 x 117 x
+    // 240: 2.9e-7 against 2.1e-7).  Runs this long are at or below it (5.8e-8 and 5.6e-8) and cost a fifth of the
+    // time (335 -> 391 us at 201^2 x 117 x 240, 93 -> 113 at 128^2 x 65 x 180; generic 1951 and 364).
+    unsigned long long sum[4][UNEVEN ? NP : 1] = {};
+    const int run = UNEVEN ? min(max(a.nA / (VZ == 8 ? 4 : 6), 4), 32) : 32;
+    bool rest = true;
+    auto carry = [&] {
+        if constexpr (UNEVEN) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int e = 0; e < NP; ++e) carry_pair(sum[q][e], acc[q][e], rest);
+        }
+    };
     const int pc = bcidx[blk];
-    if (pc >= 0) {
-        const int rs = a.nA * a.zs;
+    while (pc >= 0) {
+        const int rs = a.nA * (UNEVEN ? a.zs : a.nZ);
         const float* __restrict__ bz = a.in + z0;
         const int4* __restrict__ e = tab + (size_t)pc * a.nA * 2;
         const int nA = a.nA;
@@ -663,11 +720,18 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
                         if (((code >> (2 + 3 * q)) & 7) == 5) lerp_rows<VZ>(acc[q], w[q], rc, ra);
                 }
             }
+            if (UNEVEN && (code & kBlkSingle)) {
+                for (int q = 0; q < 4; ++q) {
+                    if (((code >> (2 + 3 * q)) & 7) != 7) continue;
+                    load_row<VZ>(ra, pr + __float_as_int(w[q]) * rs, qn);
+                    add_row<VZ>(acc[q], ra);
+                }
+            }
         };
         if constexpr (VZ == 8) {
             // entries by cp.async into the warp's two shared-memory slots: no registers held for them,
             // which lets the eight-slice body fit 80 registers (three CTAs per SM)
-            int4* slot = &s_ent[wp][0][0];
+            int4* slot = blk_entries(wp);
             // chunk of angles k0 .. k0 + 31 into slot sl (one commit group per chunk, empty past the end)
             // the table is read once: evict-first in L2, so it does not push out sinogram lines that other
             // CTAs read again (DRAM 477 -> 459 MB per 256^3 x 360 launch, 0.934 -> 0.922 ms)
@@ -693,10 +757,14 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
                 __syncwarp();
                 const int4* es = slot + sl * kBlkEnt;
 #pragma unroll 1
-                for (int l = 0; l < kn; ++l) {
-                    const int4 e0 = es[2 * l];
-                    if (e0.x < 0) continue;  // uniform: every lane read the same entry
-                    angle(e0, es[2 * l + 1]);
+                for (int l0 = 0; l0 < kn; l0 += run) {
+#pragma unroll 1
+                    for (int l = l0; l < min(l0 + run, kn); ++l) {
+                        const int4 e0 = es[2 * l];
+                        if (e0.x < 0) continue;  // uniform: every lane read the same entry
+                        angle(e0, es[2 * l + 1]);
+                    }
+                    carry();
                 }
                 __syncwarp();  // every lane read the slot before it is refilled
                 fetch(k0 + 64, sl);
@@ -717,18 +785,39 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
             for (int k0 = 0; k0 < nA; k0 += 32) {
                 const int kn = min(32, nA - k0);
 #pragma unroll 1
-                for (int l = 0; l < kn; ++l) {
-                    const int off = __shfl_sync(0xffffffffu, h0.x, l);
-                    if (off < 0) continue;  // uniform: every lane read lane l's entry
-                    const int4 e0 = make_int4(off, __shfl_sync(0xffffffffu, h0.y, l), __shfl_sync(0xffffffffu, h0.z, l),
-                                              __shfl_sync(0xffffffffu, h0.w, l));
-                    const int4 e1 = make_int4(__shfl_sync(0xffffffffu, h1.x, l), __shfl_sync(0xffffffffu, h1.y, l), 0, 0);
-                    angle(e0, e1);
+                for (int l0 = 0; l0 < kn; l0 += run) {
+#pragma unroll 1
+                    for (int l = l0; l < min(l0 + run, kn); ++l) {
+                        const int off = __shfl_sync(0xffffffffu, h0.x, l);
+                        if (off < 0) continue;  // uniform: every lane read lane l's entry
+                        const int4 e0 = make_int4(off, __shfl_sync(0xffffffffu, h0.y, l), __shfl_sync(0xffffffffu, h0.z, l),
+                                                  __shfl_sync(0xffffffffu, h0.w, l));
+                        const int4 e1 = make_int4(__shfl_sync(0xffffffffu, h1.x, l), __shfl_sync(0xffffffffu, h1.y, l), 0, 0);
+                        angle(e0, e1);
+                    }
+                    carry();
                 }
                 h0 = g0; h1 = g1;
                 if (k0 + 64 < nA) chunk(k0 + 64, g0, g1);
             }
         }
+        if (!UNEVEN || !rest) break;
+        // the rest of a sum that is not finite is no number: such a block is summed again without it
+        float bad = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int e2 = 0; e2 < NP; ++e2) {
+                float lo, hi;
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(sum[q][UNEVEN ? e2 : 0]));
+                bad = fmaf(hi, 0.f, fmaf(lo, 0.f, bad));
+            }
+        if (!__any_sync(0xffffffffu, bad != 0.f)) break;
+        rest = false;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int e2 = 0; e2 < NP; ++e2) sum[q][UNEVEN ? e2 : 0] = acc[q][e2] = 0ull;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -738,7 +827,7 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
         float v[2 * NP];
 #pragma unroll
         for (int e2 = 0; e2 < NP; ++e2)
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2 * e2]), "=f"(v[2 * e2 + 1]) : "l"(acc[q][e2]));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2 * e2]), "=f"(v[2 * e2 + 1]) : "l"(UNEVEN ? sum[q][UNEVEN ? e2 : 0] : acc[q][e2]));
         if (a.mask) {
             const float m = __ldg(a.mask + p);
 #pragma unroll
@@ -756,7 +845,7 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
         } else {
 #pragma unroll
             for (int q2 = 0; q2 < VZ / 4; ++q2)
-                if (!FULL && !a.whole) {  // (padded input rows: the output's are any length)
+                if (UNEVEN) {
                     for (int e2 = 0; e2 < 4; ++e2)
                         if (128 * q2 + e2 < a.nZ - z0 && q2 < qn) __stcs(dst + 128 * q2 + e2, v[4 * q2 + e2]);
                 } else if (q2 < qn)
@@ -766,10 +855,10 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
     }
 }
 
-template <int VZ, int MINB, bool FULL>
+template <int VZ, int MINB, bool FULL, bool UNEVEN = false>
 __global__ void __launch_bounds__(256, MINB) k_backward_blk(Args a, const int4* __restrict__ tab,
                                                             const int* __restrict__ bcidx) {
-    k_backward_blk_body<VZ, FULL>(a, tab, bcidx, blockIdx.x);
+    k_backward_blk_body<VZ, FULL, UNEVEN>(a, tab, bcidx, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -2026,7 +2115,8 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
         if (it.kind == KB_BTABLE) {
             const Args a = it.a;
             const bool full = a.nZ % (32 * it.vz) == 0;
-            if (it.vz == 8) { if (full) k_backward_blk_body<8, true>(a, it.btab4, it.bcidx, bx); else k_backward_blk_body<8, false>(a, it.btab4, it.bcidx, bx); }
+            if (a.nZ % 4) { if (it.vz == 8) k_backward_blk_body<8, false, true>(a, it.btab4, it.bcidx, bx); else k_backward_blk_body<4, false, true>(a, it.btab4, it.bcidx, bx); }
+            else if (it.vz == 8) { if (full) k_backward_blk_body<8, true>(a, it.btab4, it.bcidx, bx); else k_backward_blk_body<8, false>(a, it.btab4, it.bcidx, bx); }
             else if (it.vz == 6) k_backward_blk_body<6, true>(a, it.btab4, it.bcidx, bx);
             else if (it.vz == 5) k_backward_blk_body<5, true>(a, it.btab4, it.bcidx, bx);
             else { if (full) k_backward_blk_body<4, true>(a, it.btab4, it.bcidx, bx); else k_backward_blk_body<4, false>(a, it.btab4, it.bcidx, bx); }
@@ -2186,7 +2276,10 @@ int launch_item(const Item& it, cudaStream_t st, const char* name) {
     } else if (it.kind == KB_BTABLE) {
         const dim3 block(kWarpsPerBlock * kWarp);
         const bool full = it.a.nZ % (32 * it.vz) == 0;
-        if (it.vz == 8) {
+        if (it.a.nZ % 4) {
+            if (it.vz == 8) k_backward_blk<8, 3, false, true><<<grid, block, 0, st>>>(it.a, it.btab4, it.bcidx);
+            else k_backward_blk<4, 3, false, true><<<grid, block, 0, st>>>(it.a, it.btab4, it.bcidx);
+        } else if (it.vz == 8) {
             if (full) k_backward_blk<8, 3, true><<<grid, block, 0, st>>>(it.a, it.btab4, it.bcidx);
             else k_backward_blk<8, 3, false><<<grid, block, 0, st>>>(it.a, it.btab4, it.bcidx);
         } else if (it.vz == 6) {
@@ -2728,7 +2821,7 @@ static int prepare_backward(vam_parallel_plan* p, int zs, cudaStream_t st) {
     if (e == cudaSuccess && nbc) {
         const long tot = (long)nbc * p->nA;
         k_bwd_btable<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(p->d_trig, d_blist, p->d_bwd_cidx, p->d_bwd_btab,
-                                                                    nbc, p->nA, p->nY, p->nX, zs, p->C);
+                                                                    nbc, p->nA, p->nY, p->nX, zs, p->C, p->nZ % 4 != 0);
         e = cudaGetLastError();
     }
     // the host vectors and the block list are released after the copies and the build complete
