@@ -68,8 +68,6 @@ struct Args {
     float* out;
     const double4* trig;
     const uint8_t* circle;
-    const float4* split;  // nZ == 1: per angle the high and low parts of cos and sin
-    const int2* tasks;    // 2-D forward tiles: angle, or angle and the one 180 degrees from it
     const float* mask;
     const float* occ;
     const uint8_t* occ_flag;
@@ -78,10 +76,20 @@ struct Args {
     int lz_shift, zvec, zchunks;
     float alpha, R;  // VAM_ABS_RAY
     int occ_mode;
-    int zs;     // floats from one input row to the next (nZ, or nZ rounded up to four: padded rows)
-    int whole;  // the output's rows take float4 stores
-    int pad_;
+    int zs;  // floats from one input row to the next (nZ, or nZ rounded up to four: padded rows)
 };
+// The compiler treats a parameter struct above 128 bytes differently from one up to it.  The generic kernels want the
+// small one (above it the masked forward took 52 registers for 48, one block less per SM, and 5 % more time) ...
+static_assert(sizeof(Args) <= 128, "arguments of the generic kernels");
+
+// ... the 2-D tiles the large one (59 registers for 48 below it: backprojection 209 -> 220 us at 512^2 x 720 angles,
+// forward with per-ray absorption 403 -> 433).
+struct TileArgs : Args {
+    const float4* split;  // backprojection: per angle the high and low parts of cos and sin
+    const int2* tasks;    // forward: angle, or angle and the one 180 degrees from it
+    const void* pad_;
+};
+static_assert(sizeof(TileArgs) > 128, "arguments of the 2-D tiles");
 
 template <int VZ>
 __device__ __forceinline__ void load_vec(const float* p, float (&d)[VZ]) {
@@ -897,7 +905,7 @@ struct Slice2d {
     int jmax, kfirst;
 };
 
-__device__ __forceinline__ Slice2d slice_2d(const Args& a, unsigned by) {
+__device__ __forceinline__ Slice2d slice_2d(const TileArgs& a, unsigned by) {
     const int2 t = a.tasks[by];
     const bool ext = t.y >= 0 && a.nY % 2 == 0;
     return {t.x, t.y, ext, ext ? a.nX : a.nX - 1, ext ? 1 : 0};
@@ -991,7 +999,7 @@ __device__ __forceinline__ void last_row_2d(const Args& a, const Slice2d& t, con
 // coordinates are the reference's float64 values at the tile's first sample,
 // taken on along the ray in fixed point (Line2d).
 template <bool RAY>
-__device__ __forceinline__ void k_forward_2d_body(const Args& a, unsigned bx, unsigned by) {
+__device__ __forceinline__ void k_forward_2d_body(const TileArgs& a, unsigned bx, unsigned by) {
     extern __shared__ float s_f2[];
     float* box = s_f2;
     float* part = s_f2 + k2Box * k2Stride;
@@ -1115,7 +1123,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
 // One block (tile of k2J bins x all samples, one angle) of the TMA-staged forward; tmap points to the
 // image's tensor map in parameter space (a __grid_constant__ argument or a batch item).
 template <bool RAY>
-__device__ __forceinline__ void k_forward_2d_tma_body(const Args& a, const CUtensorMap* tmap, int* status,
+__device__ __forceinline__ void k_forward_2d_tma_body(const TileArgs& a, const CUtensorMap* tmap, int* status,
                                                       unsigned bx, unsigned by) {
     extern __shared__ float s_f2[];
     float* box = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(s_f2) + 127) & ~(uintptr_t)127);
@@ -1217,13 +1225,13 @@ __device__ __forceinline__ void k_forward_2d_tma_body(const Args& a, const CUten
 }
 
 template <bool RAY>
-__global__ void __launch_bounds__(256) k_forward_2d_tma(Args a, const __grid_constant__ CUtensorMap tmap,
+__global__ void __launch_bounds__(256) k_forward_2d_tma(TileArgs a, const __grid_constant__ CUtensorMap tmap,
                                                         int* __restrict__ status) {
     k_forward_2d_tma_body<RAY>(a, &tmap, status, blockIdx.x, blockIdx.y);
 }
 
 template <bool RAY>
-__global__ void __launch_bounds__(256) k_forward_2d(Args a) {
+__global__ void __launch_bounds__(256) k_forward_2d(TileArgs a) {
     k_forward_2d_body<RAY>(a, blockIdx.x, blockIdx.y);
 }
 
@@ -1322,7 +1330,7 @@ __device__ __noinline__ float2 interp_bin(const double4* tr, float X, float Y, i
 // formed again in float64 as numpy does, but for an exact integer (the centre pixel's, at every angle).
 // 512^2 x 720: 369 -> 219 us, 600^2 x 800 529 -> 310, 256^2 x 360 95 -> 53; issue is 75 % busy, 34
 // instructions a pixel and angle.
-__device__ __forceinline__ void backward_2d_body(const Args& a, unsigned bx) {
+__device__ __forceinline__ void backward_2d_body(const TileArgs& a, unsigned bx) {
     __shared__ float win[kP2A * kP2W];
     __shared__ float4 cs[kP2A];  // ch, cl, sh, sl
     __shared__ int2 lim[kP2A];   // first staged detector row; last row of the detector from it
@@ -1412,15 +1420,14 @@ __device__ __forceinline__ void backward_2d_body(const Args& a, unsigned bx) {
 }
 
 template <bool RAY>
-__device__ __forceinline__ void k_backward_2d_body(const Args& a, unsigned bx, unsigned by) {
-    (void)by;
+__device__ __forceinline__ void k_backward_2d_body(const TileArgs& a, unsigned bx) {
     if constexpr (RAY) backward_2d_ray_body(a, bx);
     else backward_2d_body(a, bx);
 }
 
 template <bool RAY>
-__global__ void __launch_bounds__(256) k_backward_2d(Args a) {
-    k_backward_2d_body<RAY>(a, blockIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(256) k_backward_2d(TileArgs a) {
+    k_backward_2d_body<RAY>(a, blockIdx.x);
 }
 
 // out = mask (per pixel, broadcast over z) * x; with nZ % 4 == 0 and aligned buffers four
@@ -1486,7 +1493,10 @@ __device__ __forceinline__ double interp_nan(double t, double ft, int j0, int nY
     return res;
 }
 
-template <int VZ, bool OCC, int ABS>
+// PAD: the input's rows are padded to a multiple of four (the output's are any length).  An instance of its own:
+// with the row length and the stores decided at run time the others took 3 more registers (48 -> 51 with per-ray
+// absorption, one block less per SM) and 3 to 12 % more time.
+template <int VZ, bool OCC, int ABS, bool PAD = false>
 __device__ __forceinline__ void k_backward_ref_body(const Args& a, unsigned bx, unsigned by) {
     const int lane = threadIdx.x & 31;
     const int LZ = 1 << a.lz_shift;
@@ -1508,14 +1518,15 @@ __device__ __forceinline__ void k_backward_ref_body(const Args& a, unsigned bx, 
     if (a.circle[p]) {
         const double X = (double)(j - a.C), Y = (double)(i - a.C);
         const double tlo = (double)(-a.C), thi = (double)(a.nY - 1 - a.C);
-        const size_t rs = (size_t)a.nA * a.zs;  // sinogram row stride
+        const int zs = PAD ? a.zs : a.nZ;
+        const size_t rs = (size_t)a.nA * zs;  // sinogram row stride
         for (int th = kl; th < a.nA; th += LK) {
             const double4 tr = a.trig[th];
             const double t = __dsub_rn(__dmul_rn(X, tr.x), __dmul_rn(Y, tr.y));
             if (!(t >= tlo && t <= thi)) continue;  // np.interp left = right = 0
             const double ft = floor(t);
             const int j0 = (int)ft + a.C;
-            const float* b0 = a.in + (size_t)j0 * rs + (size_t)th * a.zs + z0;
+            const float* b0 = a.in + (size_t)j0 * rs + (size_t)th * zs + z0;
             float v[VZ];
             if (zok) {
                 load_vec<VZ>(b0, v);
@@ -1567,20 +1578,19 @@ __device__ __forceinline__ void k_backward_ref_body(const Args& a, unsigned bx, 
 #pragma unroll
         for (int e = 0; e < VZ; ++e) acc[e] = m * acc[e];
     }
-    if (kl != 0 || !zok) return;
-    float* o = a.out + (size_t)p * a.nZ + z0;
-    if (VZ == 1 || a.whole) {
-        store_vec<VZ>(o, acc);
-    } else {  // (padded input rows: the output's are any length)
+    if constexpr (!PAD) {
+        if (kl == 0 && zok) store_vec<VZ>(a.out + (size_t)p * a.nZ + z0, acc);
+    } else if (kl == 0 && zok) {
+        float* o = a.out + (size_t)p * a.nZ + z0;
 #pragma unroll
         for (int e = 0; e < VZ; ++e)
             if (z0 + e < a.nZ) o[e] = acc[e];
     }
 }
 
-template <int VZ, bool OCC, int ABS>
+template <int VZ, bool OCC, int ABS, bool PAD = false>
 __global__ void __launch_bounds__(256) k_backward_ref(Args a) {
-    k_backward_ref_body<VZ, OCC, ABS>(a, blockIdx.x, blockIdx.y);
+    k_backward_ref_body<VZ, OCC, ABS, PAD>(a, blockIdx.x, blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -1863,7 +1873,7 @@ struct Item {
     float* pre_out;
     long long pre_npix;
     int pre_w, pre_wp;
-    Args a;
+    TileArgs a;
     FastArgs f;
     const int4* btab4;  // KB_BTABLE: the plan's 2 x 2 block bin table and its block index
     const int* bcidx;
@@ -1882,6 +1892,7 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     VAM_REQUIRE(!padded || (plan->nZ > 1 && !noclip), VAM_ERR_NOTSUP, std::string(name) + ": padded rows are not served here");
     VAM_REQUIRE(!padded || (((uintptr_t)in) & 15) == 0, VAM_ERR_ARG,
                 std::string(name) + ": padded rows must be 16-byte aligned");
+    padded = padded && plan->nZ % 4 != 0;  // rows of a multiple of four are the plan's own
     VAM_REQUIRE(!noclip || plan->d_ones, VAM_ERR_ARG, std::string(name) + ": no all-ones circle table");
     std::memset(&it, 0, sizeof(it));
     it.cost = (long long)plan->nY * plan->nX * plan->nZ * plan->nA;
@@ -1915,7 +1926,7 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         Args& a = it.a;
         a.in = in; a.out = out; a.trig = plan->d_trig; a.circle = plan->d_circle;
         a.mask = plan->abs_mode == VAM_ABS_MASK ? plan->d_mask : nullptr;
-        a.split = plan->d_split;
+        it.a.split = plan->d_split;
         a.nY = plan->nY; a.nX = plan->nX; a.nZ = 1; a.nA = plan->nA; a.C = plan->C;
         a.alpha = plan->abs_alpha; a.R = plan->abs_R;
         it.ray = ray;
@@ -1942,7 +1953,7 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
             it.family = 128;
             it.status = plan->d_status;
             it.tma = use_tma && image_tensor_map(a.in, a.nX, a.nY, it.pre_wp ? it.pre_wp : a.nX, it.tmap) ? 1 : 0;
-            a.tasks = ray ? plan->d_tasks_single : plan->d_tasks_paired;
+            it.a.tasks = ray ? plan->d_tasks_single : plan->d_tasks_paired;
             a.zs = it.pre_wp ? it.pre_wp : a.nX;
             it.gx = (unsigned)((plan->nX + (plan->nX % 2 == 0 && !ray) + k2J - 1) / k2J);
             it.gy = (unsigned)(ray ? plan->nA : plan->n_tasks_paired);
@@ -1969,7 +1980,7 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         a.vol = in; a.sino = out; a.trig = plan->d_trig;
         a.mask = plan->abs_mode == VAM_ABS_MASK ? plan->d_mask : nullptr;
         a.nY = plan->nY; a.nX = plan->nX; a.nZ = plan->nZ; a.nA = plan->nA; a.C = plan->C;
-        a.vs = zs; a.whole = aligned16 && plan->nZ % 4 == 0;
+        a.vs = zs;
         a.even = (plan->nY % 2) == 0;
         a.alpha = plan->abs_alpha; a.R = plan->abs_R;
         a.tasks = ray ? plan->d_tasks_single : plan->d_tasks_paired;
@@ -1995,7 +2006,7 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         a.mask = plan->abs_mode == VAM_ABS_MASK ? plan->d_mask : nullptr;
         a.nY = plan->nY; a.nX = plan->nX; a.nZ = plan->nZ; a.nA = plan->nA; a.C = plan->C;
         a.alpha = plan->abs_alpha; a.R = plan->abs_R;
-        a.zs = zs; a.whole = aligned16 && plan->nZ % 4 == 0;
+        a.zs = zs;
         it.kind = KA_BLOCK; it.ray = ray;
         it.vec = rows4 && (padded || aligned16);
         it.vz = want == 4 || (want != 8 && plan->nZ <= 128) ? 4 : 8;
@@ -2015,7 +2026,7 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     if (op == Op::BackwardRef && !plan->has_occ && (vzf || blk_ok) && !noclip &&
         (long long)plan->nY * plan->nA * zs < (1LL << 31)) {
         Args& a = it.a;
-        a.zs = zs; a.whole = aligned16 && plan->nZ % 4 == 0;
+        a.zs = zs;
         a.in = in; a.out = out; a.trig = plan->d_trig; a.circle = plan->d_circle;
         a.mask = plan->abs_mode == VAM_ABS_MASK ? plan->d_mask : nullptr;
         a.nY = plan->nY; a.nX = plan->nX; a.nZ = plan->nZ; a.nA = plan->nA; a.C = plan->C;
@@ -2053,14 +2064,14 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         }
         return VAM_OK;
     }
-    Layout L = choose_layout(zs, padded ? rows4 : aligned16);
+    Layout L = choose_layout(zs, padded || aligned16);
     Args& a = it.a;
     a.in = in; a.out = out; a.trig = plan->d_trig; a.circle = noclip ? plan->d_ones : plan->d_circle;
     a.mask = plan->d_mask; a.occ = plan->d_occ; a.occ_flag = plan->d_occ_flag;
     a.occ64 = plan->d_occ64; a.occ_mode = plan->has_occ ? plan->occ_mode : 0;
     a.nY = plan->nY; a.nX = plan->nX; a.nZ = plan->nZ; a.nA = plan->nA; a.C = plan->C;
     a.lz_shift = L.lz_shift; a.zvec = L.zvec; a.zchunks = L.zchunks;
-    a.zs = zs; a.whole = aligned16 && plan->nZ % 4 == 0;
+    a.zs = zs;
     a.alpha = plan->abs_alpha; a.R = plan->abs_R;
     const long items = (op == Op::Forward) ? (long)plan->nX * L.zchunks : (long)plan->nY * plan->nX * L.zchunks;
     it.kind = op == Op::Forward ? KF_GEN : (op == Op::BackwardRef ? KB_GEN : KA_GEN);
@@ -2074,18 +2085,26 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
 // The bodies receive a local copy of their arguments: read once from the
 // launch's parameter space into registers, instead of an indexed
 // constant-cache load at every use inside the sample loops.
+template <int VZ, bool OCC, int ABS>
+__device__ __forceinline__ void backward_ref_rows(const Args& a, unsigned bx, unsigned by) {
+    if constexpr (VZ == 4 && !OCC) {
+        if (a.zs != a.nZ) return k_backward_ref_body<4, false, ABS, true>(a, bx, by);
+    }
+    k_backward_ref_body<VZ, OCC, ABS>(a, bx, by);
+}
+
 template <int FAM, int VZ, bool OCC, int ABS>
 __device__ __forceinline__ void gen_body(const Item& it, unsigned bx, unsigned by) {
     const Args a = it.a;
     if constexpr ((FAM & 16) != 0) if (it.kind == KF_GEN) k_forward_body<VZ, OCC, ABS>(a, bx, by);
-    if constexpr ((FAM & 8) != 0) if (it.kind == KB_GEN) k_backward_ref_body<VZ, OCC, ABS>(a, bx, by);
+    if constexpr ((FAM & 8) != 0) if (it.kind == KB_GEN) backward_ref_rows<VZ, OCC, ABS>(a, bx, by);
     if constexpr ((FAM & 4) != 0) if (it.kind == KA_GEN) k_adjoint_body<VZ, OCC, ABS>(a, bx, by);
 }
 
 template <int FAM, int VZ, int ABS>
 __device__ __forceinline__ void lean_gen_body(const Item& it, const Args& a, unsigned bx, unsigned by) {
     if constexpr (FAM == 32) if (it.kind == KF_GEN) k_forward_body<VZ, false, ABS>(a, bx, by);
-    if constexpr (FAM == 64) if (it.kind == KB_GEN) k_backward_ref_body<VZ, false, ABS>(a, bx, by);
+    if constexpr (FAM == 64) if (it.kind == KB_GEN) backward_ref_rows<VZ, false, ABS>(a, bx, by);
 }
 
 template <int FAM, int VZ, bool OCC>
@@ -2106,7 +2125,7 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
     }
     if constexpr (FAM == 128 || FAM == 512) {
         if (it.kind == KF_2D) {
-            const Args a = it.a;
+            const TileArgs a = it.a;
             if constexpr (FAM == 128) k_forward_2d_tma_body<RAY>(a, &it.tmap, it.status, bx, by);
             else k_forward_2d_body<RAY>(a, bx, by);
         }
@@ -2124,8 +2143,8 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
     }
     if constexpr ((FAM & 8) != 0 || ((FAM & 2) != 0 && !RAY)) {
         if (it.kind == KB_2D) {
-            const Args a = it.a;
-            k_backward_2d_body<RAY>(a, bx, by);
+            const TileArgs a = it.a;
+            k_backward_2d_body<RAY>(a, bx);
         } else if (it.kind == KB_BATCHED) {
             const Args a = it.a;
             if (it.vz == 8) k_backward_batched_body<8, 2, RAY>(a, bx, by);
@@ -2184,6 +2203,7 @@ template <int VZ, bool OCC, int ABS>
 void launch_gen3(const Item& it, dim3 grid, cudaStream_t st) {
     const dim3 block(kWarpsPerBlock * kWarp);
     if (it.kind == KF_GEN) k_forward<VZ, OCC, ABS><<<grid, block, 0, st>>>(it.a);
+    else if (it.kind == KB_GEN && VZ == 4 && !OCC && it.a.zs != it.a.nZ) k_backward_ref<4, false, ABS, true><<<grid, block, 0, st>>>(it.a);
     else if (it.kind == KB_GEN) k_backward_ref<VZ, OCC, ABS><<<grid, block, 0, st>>>(it.a);
     else k_adjoint<VZ, OCC, ABS><<<grid, block, 0, st>>>(it.a);
 }
@@ -2736,9 +2756,7 @@ extern "C" int vam_parallel_route(const vam_parallel_call* c, vam_parallel_route
     out->row_stride = it.kind == KF_FAST ? it.f.vs : steps ? it.a.zs : c->n_z;
     const bool strip = it.kind == KF_FAST || it.kind == KA_BLOCK;
     out->vector_loads = strip ? it.vec : it.vz >= 4;
-    out->vector_stores = strip ? it.vec && (it.kind == KF_FAST ? it.f.whole : it.a.whole)
-                         : it.vz >= 4 && (!(it.kind == KB_BTABLE || it.kind == KB_GEN) || it.a.whole ||
-                                          (it.kind == KB_BTABLE && c->n_z % (32 * it.vz) == 0));
+    out->vector_stores = out->vector_loads && c->n_z % 4 == 0;
     return VAM_OK;
 }
 

@@ -65,7 +65,6 @@ struct FastArgs {
     const float* mask;  // per-pixel factor of the volume, or null
     int nY, nX, nZ, nA, C;
     int vs;          // floats from one pixel's row to the next (nZ, or nZ rounded up to four: padded rows)
-    int whole;       // the output's rows take float4 stores
     int ntasks;
     int zchunks;
     int lz_shift;    // log2 of the lanes along z (a warp's other lanes take other pixels)
@@ -102,8 +101,8 @@ __device__ __forceinline__ void fma_pairs(unsigned long long& acc, unsigned long
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(w2), "l"(v2));
 }
 
-// whole: the float4s may be stored as such; otherwise slice by slice, the first `left` of them (those the
-// output has: a padded row holds up to three more)
+// whole: the float4s may be stored as such; otherwise (padded rows) slice by slice, the first `left` of them
+// (those the output has: a padded row holds up to three more)
 template <int Q, bool VEC>
 __device__ __forceinline__ void strip_store(float* __restrict__ p, const unsigned long long (&v)[2 * Q], int n, int lz,
                                             int whole, int left) {
@@ -168,8 +167,8 @@ __device__ __forceinline__ void strip_finish(const FastArgs& a, int2 task, bool 
     float* const here = a.sino + ((size_t)j * a.nA + task.x) * a.nZ + z0;
     float* const there = a.sino + ((size_t)(2 * a.C - j) * a.nA + task.y) * a.nZ + z0;
     if (!ext) {
-        strip_store<Q, VEC>(here, sum, n, lz, a.whole, a.nZ - z0);
-        if (task.y >= 0) strip_store<Q, VEC>(there, sum, n, lz, a.whole, a.nZ - z0);
+        strip_store<Q, VEC>(here, sum, n, lz, a.vs == a.nZ, a.nZ - z0);
+        if (task.y >= 0) strip_store<Q, VEC>(there, sum, n, lz, a.vs == a.nZ, a.nZ - z0);
         return;
     }
     const double4 tr = a.trig[task.x];
@@ -180,11 +179,11 @@ __device__ __forceinline__ void strip_finish(const FastArgs& a, int2 task, bool 
 #pragma unroll
         for (int e = 0; e < 2 * Q; ++e) o[e] = sum[e];
         strip_sample<Q, VEC>(a, volz, rowb, colb, o, n, lz);
-        strip_store<Q, VEC>(here, o, n, lz, a.whole, a.nZ - z0);
+        strip_store<Q, VEC>(here, o, n, lz, a.vs == a.nZ, a.nZ - z0);
     }
     if (j > 0) {
         strip_sample<Q, VEC>(a, volz, fma(tr.x, (double)N, rowb), fma(tr.y, (double)N, colb), sum, n, lz);
-        strip_store<Q, VEC>(there, sum, n, lz, a.whole, a.nZ - z0);
+        strip_store<Q, VEC>(there, sum, n, lz, a.vs == a.nZ, a.nZ - z0);
     }
 }
 
@@ -698,7 +697,7 @@ __device__ __forceinline__ void adjoint_block_body(const Args& a, unsigned bx) {
 #pragma unroll
             for (int e = 0; e < VZ / 2; ++e) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[q][e]) : "l"(mm));
         }
-        strip_store<Q, VEC>(a.out + p * a.nZ + z0, acc[q], n, LZ, a.whole, a.nZ - z0);
+        strip_store<Q, VEC>(a.out + p * a.nZ + z0, acc[q], n, LZ, a.zs == a.nZ, a.nZ - z0);
     }
 }
 
@@ -748,7 +747,7 @@ __device__ __noinline__ void adjoint_block_rows(const Args& a, unsigned bx) {
 #pragma unroll
             for (int e = 0; e < 2 * Q; ++e) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[e]) : "l"(pk_pair(m, m)));
         }
-        strip_store<Q, VEC>(a.out + p * a.nZ + z0, acc, n, LZ, a.whole, a.nZ - z0);
+        strip_store<Q, VEC>(a.out + p * a.nZ + z0, acc, n, LZ, a.zs == a.nZ, a.nZ - z0);
     }
 }
 
