@@ -690,6 +690,8 @@ def test_padded_backprojection_under_every_tuning(n, nz, absn):
     b = rng.uniform(0, 1, (n, ang.size, nz))
     ref = O.parallel_backward_ref(b, ang, absorption=oabs)
     bound = 1.6e-6 * ref.max()
+    if nz >= 64:
+        p._prepare_padded()
     bd, guard = dev(b), torch.full((n * n * nz + 64,), -3.0, device="cuda")
     out = guard[32:32 + n * n * nz].view(n, n, nz)
     batch = ProjectionBatch()
@@ -711,6 +713,7 @@ def test_autotune_of_a_padded_slice_count(tmp_path, monkeypatch):
     ang = np.linspace(0, 360, 30, endpoint=False) + 0.3
     p = plan_for((48, 48, 67), ang)
     p.pad_from = p.pad_backward_from = 0
+    p._prepare_padded()
     p.autotune()
     x, b = rng.uniform(0, 1, p.shape_vol), rng.uniform(0, 1, p.shape_sino)
     ref = O.parallel_backward_ref(b, ang)
@@ -734,6 +737,7 @@ def test_padded_table_backprojection_is_as_exact_as_the_generic_kernel(n, nz, ab
     ang = np.concatenate([np.array([0.0, 45.0, 90.0, 180.0, 270.0, 359.9]), rng.uniform(0, 360, 33)])
     p = plan_for((n, n, nz), ang)
     p.pad_backward_from = 0
+    p._prepare_padded()
     assert p.has_backward_table and p._pads(_lib.OP_BACKWARD_REF)
     oabs = None
     if absn == "mask":
@@ -756,3 +760,15 @@ def test_padded_table_backprojection_is_as_exact_as_the_generic_kernel(n, nz, ab
         assert (np.abs(got - ref) <= 21 * 2.0 ** -24 * size + 1e-30).all(), vz
         assert relL2(got, ref) <= relL2(generic(dev(b)).cpu().numpy(), ref) + 2.0 ** -25.5, vz
         assert torch.equal(p.backward_ref(dev(bi)).isfinite(), generic(dev(bi)).isfinite()), vz
+
+
+def test_small_slices_build_no_padded_table():
+    """Slices of few pixels with an odd slice count keep the generic kernel (its rows padded), which their few blocks
+    do not leave waiting as the bin table's kernel."""
+    from vamtoolbox_b200 import _lib
+
+    ang = np.linspace(0, 360, 90, endpoint=False)
+    small, large = plan_for((32, 32, 67), ang), plan_for((96, 96, 101), ang)
+    assert not small.has_backward_table and small._pads(_lib.OP_BACKWARD_REF)
+    assert large.has_backward_table and large._pads(_lib.OP_BACKWARD_REF)
+    assert not plan_for((40, 40, 117), ang)._pads(_lib.OP_BACKWARD_REF)

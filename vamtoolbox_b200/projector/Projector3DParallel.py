@@ -107,9 +107,11 @@ class ParallelPlan:
         self.bwd_table_limit_bytes = 8 << 30
         # pixels x slices x angles from which odd slice counts are padded: below, the copy's launch costs what
         # the wider loads save (forward / transpose 27.6 / 27.6 us padded, 27.8 / 25.6 not, at 64^2 x 33 x 90;
-        # 62.5 / 74.7 against 72.8 / 82.0 at 100^2 x 33 x 180; backprojection 19.5 against 21.5 at 64^2 x 9 x 90,
-        # 246.8 against 497.8 at 200^2 x 33 x 180)
-        self.pad_from, self.pad_backward_from = 25e6, 3e6
+        # 62.5 / 74.7 against 72.8 / 82.0 at 100^2 x 33 x 180; backprojection 12.4 against 13.7 at 64^2 x 9 x 90,
+        # 246.8 against 497.8 at 200^2 x 33 x 180).  Above 112 slices the float4s of one pixel take a warp's lanes,
+        # which leaves its angles to one lane after the other: slices of few pixels then gain nothing (46 against
+        # 42 us at 40^2 x 117 x 90; 47 against 83 at 56^2)
+        self.pad_from, self.pad_backward_from = 25e6, 3e6 if n_y >= 48 or n_z <= 112 else 2e8
         self.has_backward_table = False
         self._key = _pool_key(self.shape_vol, self.angles, self.device)
         reused = _pool_take(self._key)
@@ -129,7 +131,10 @@ class ParallelPlan:
         if int(n_z) >= 64:
             if int(n_z) % 4 == 0:
                 self.prepare_backward()
-            else:
+            elif n_y >= 80 and n_y * n_y * n_z >= 6.5e5:
+                # fewer blocks leave the table's kernel waiting for its rows: 47 us at 32^2 x 65 x 90 angles, 184 at
+                # 80^2 x 65 x 360, 262 at 64^2 x 201 x 360, where the generic kernel on padded rows takes 12, 134 and
+                # 194; at 80^2 x 117 x 360 197 and 213, at 96^2 x 65 x 360 188 and about the same
                 self._prepare_padded()
 
     def _reset(self):
