@@ -227,3 +227,40 @@ def test_batch_takes_masked_volume_forwards_of_one_plan_twice(nz):
     ProjectionBatch().submit([(p, "forward", x[0], out[0]), (p, "forward", x[1], out[1])])
     torch.cuda.synchronize()
     assert all(torch.equal(o, p.forward(v)) for o, v in zip(out, x))
+
+
+@pytest.mark.parametrize("mode", [None, "mask", "ray"])
+def test_batch_of_every_kernel_family_bitwise(mode):
+    """One list with a call of every body family: strips and blocks of four and eight slices per lane on float4 rows
+    and on single slices, generic kernels, bin tables of four, five, six and eight slices per lane and of padded rows,
+    slices by tiles and by the generic kernels.  Each equals the plan's own call bit for bit."""
+    rng = np.random.default_rng(11)
+    work, ref = [], []
+    for n, nz in [(40, 3), (40, 8), (40, 16), (40, 45), (40, 64), (40, 130), (48, 160), (40, 192), (40, 201), (40, 256),
+                  (96, 101), (128, 1), (200, 1)]:
+        p = ParallelPlan(n, n, nz, np.linspace(0, 360, 24, endpoint=False) + 0.4)
+        p.pad_from = 0 if nz % 2 else 1e30
+        if mode == "mask":
+            p.set_absorption("mask", mask=rng.uniform(0.2, 1.0, (n, n)))
+        elif mode == "ray":
+            p.set_absorption("ray", alpha_per_px=0.02, radius_px=n / 2.0)
+        x = torch.as_tensor(rng.uniform(0, 1, p.shape_vol), dtype=torch.float32, device="cuda")
+        b = torch.as_tensor(rng.uniform(0, 1, p.shape_sino), dtype=torch.float32, device="cuda")
+        for vz in (0, 8) if nz > 8 else (0,):  # (a plan's launch shape counts when the list is submitted)
+            q = p if vz == 0 else ParallelPlan(n, n, nz, p.angles)
+            if vz:
+                q.pad_from = p.pad_from
+                if mode == "mask":
+                    q.set_absorption("mask", mask=rng.uniform(0.2, 1.0, (n, n)))
+                elif mode == "ray":
+                    q.set_absorption("ray", alpha_per_px=0.02, radius_px=n / 2.0)
+                q.set_tuning({"forward_vz": vz, "adjoint_vz": vz})
+            work.append((q, "forward", x, torch.full(q.shape_sino, np.nan, device="cuda")))
+            ref.append(q.forward(x))
+            for op, f in (("adjoint", q.adjoint), ("backward_ref", q.backward_ref)):
+                work.append((q, op, b, torch.full(q.shape_vol, np.nan, device="cuda")))
+                ref.append(f(b))
+    ProjectionBatch().submit(work)
+    torch.cuda.synchronize()
+    for (p, op, _, out), r in zip(work, ref):
+        assert torch.equal(out, r), (p.shape_vol, op)

@@ -1856,6 +1856,20 @@ enum Kind : int {
     KB_BTABLE = VAM_KERNEL_BACKWARD_TABLE
 };
 
+// Body families of the batch kernels: a batch launches one instance of k_batch per family present in its list.
+// Where a direct kernel's body fills the registers it has a family of its own: eight strip bodies in one function kept
+// their rows in flight in local memory (transpose of 128^3 x 180 angles 507 us in a batch; 142 so, 124 on its own).
+enum Fam : int {
+    kStrip1 = 0, kStrip1Single, kStrip2, kStrip2Single, kStripRay,  // strips: slices per lane, float4 rows or single
+    kBackFast,                                                      // fast, batched and 2-D backprojections
+    kAdjGen, kBlock1, kBlock1Single, kBlock2, kBlock2Single, kBlockRay,
+    kBackHeavy,  // generic backprojection with occlusion or per-ray absorption, the fast ones with the latter
+    kFwdHeavy,   // generic forward with occlusion or per-ray absorption
+    kFwdGen, kBackGen,
+    kTile, kTable4, kTable8, kTable56, kTableUneven, kTilePlain,
+    kFamilies
+};
+
 struct Item {
     int kind;
     int vz;          // slices per lane of the template instance (1, 4 or 8; 5 or 6 of the block table)
@@ -1865,7 +1879,7 @@ struct Item {
     int pre_nz;
     long long tstart;  // first ticket (virtual block) of the call inside a batch launch
     long long cost;    // estimated time of the call (batch ordering)
-    int family;        // body family (k_batch instances): a bit of the FAM mask
+    int family;        // Fam (set by a batch)
     // pre-pass of the 2-D tile forward: pre_out = mask * pre_in, or (pre_wp > 0) rows of pre_w floats of
     // (mask *) pre_in into rows of pre_wp floats of pre_out
     const float* pre_in;
@@ -1896,7 +1910,6 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     VAM_REQUIRE(!noclip || plan->d_ones, VAM_ERR_ARG, std::string(name) + ": no all-ones circle table");
     std::memset(&it, 0, sizeof(it));
     it.cost = (long long)plan->nY * plan->nX * plan->nZ * plan->nA;
-    it.family = op == Op::Forward ? 1 : (op == Op::BackwardRef ? 2 : 4);
     it.gy = 1;
     // rows of the input padded to a multiple of four slices (vam_pad_rows): float4 loads for any slice count
     const int zs = padded ? (plan->nZ + 3) & ~3 : plan->nZ;
@@ -1950,7 +1963,6 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
                 a.mask = nullptr;
             }
             it.kind = KF_2D;
-            it.family = 128;
             it.status = plan->d_status;
             it.tma = use_tma && image_tensor_map(a.in, a.nX, a.nY, it.pre_wp ? it.pre_wp : a.nX, it.tmap) ? 1 : 0;
             it.a.tasks = ray ? plan->d_tasks_single : plan->d_tasks_paired;
@@ -2096,15 +2108,15 @@ __device__ __forceinline__ void backward_ref_rows(const Args& a, unsigned bx, un
 template <int FAM, int VZ, bool OCC, int ABS>
 __device__ __forceinline__ void gen_body(const Item& it, unsigned bx, unsigned by) {
     const Args a = it.a;
-    if constexpr ((FAM & 16) != 0) if (it.kind == KF_GEN) k_forward_body<VZ, OCC, ABS>(a, bx, by);
-    if constexpr ((FAM & 8) != 0) if (it.kind == KB_GEN) backward_ref_rows<VZ, OCC, ABS>(a, bx, by);
-    if constexpr ((FAM & 4) != 0) if (it.kind == KA_GEN) k_adjoint_body<VZ, OCC, ABS>(a, bx, by);
+    if constexpr (FAM == kFwdHeavy) if (it.kind == KF_GEN) k_forward_body<VZ, OCC, ABS>(a, bx, by);
+    if constexpr (FAM == kBackHeavy) if (it.kind == KB_GEN) backward_ref_rows<VZ, OCC, ABS>(a, bx, by);
+    if constexpr (FAM == kAdjGen) if (it.kind == KA_GEN) k_adjoint_body<VZ, OCC, ABS>(a, bx, by);
 }
 
 template <int FAM, int VZ, int ABS>
 __device__ __forceinline__ void lean_gen_body(const Item& it, const Args& a, unsigned bx, unsigned by) {
-    if constexpr (FAM == 32) if (it.kind == KF_GEN) k_forward_body<VZ, false, ABS>(a, bx, by);
-    if constexpr (FAM == 64) if (it.kind == KB_GEN) backward_ref_rows<VZ, false, ABS>(a, bx, by);
+    if constexpr (FAM == kFwdGen) if (it.kind == KF_GEN) k_forward_body<VZ, false, ABS>(a, bx, by);
+    if constexpr (FAM == kBackGen) if (it.kind == KB_GEN) backward_ref_rows<VZ, false, ABS>(a, bx, by);
 }
 
 template <int FAM, int VZ, bool OCC>
@@ -2116,32 +2128,46 @@ __device__ __forceinline__ void gen_body_fam(const Item& it, unsigned bx, unsign
 
 template <int FAM, bool RAY>
 __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned by) {
-    if constexpr ((FAM & 1) != 0) {
-        if (it.kind == KF_FAST) {
-            const FastArgs f = it.f;
-            if (it.vz == 8) { if (it.vec) forward_strip_body<2, true, RAY>(f, bx, by); else forward_strip_body<2, false, RAY>(f, bx, by); }
-            else { if (it.vec) forward_strip_body<1, true, RAY>(f, bx, by); else forward_strip_body<1, false, RAY>(f, bx, by); }
-        }
+    const FastArgs f = it.f;
+    const Args a0 = it.a;
+    if constexpr (FAM == kStrip1) forward_strip_body<1, true, false>(f, it.f, bx, by);
+    if constexpr (FAM == kStrip1Single) forward_strip_body<1, false, false>(f, it.f, bx, by);
+    if constexpr (FAM == kStrip2) forward_strip_body<2, true, false>(f, it.f, bx, by);
+    if constexpr (FAM == kStrip2Single) forward_strip_body<2, false, false>(f, it.f, bx, by);
+    if constexpr (FAM == kStripRay) {
+        if (it.vz == 8) { if (it.vec) forward_strip_body<2, true, true>(f, it.f, bx, by); else forward_strip_body<2, false, true>(f, it.f, bx, by); }
+        else { if (it.vec) forward_strip_body<1, true, true>(f, it.f, bx, by); else forward_strip_body<1, false, true>(f, it.f, bx, by); }
     }
-    if constexpr (FAM == 128 || FAM == 512) {
-        if (it.kind == KF_2D) {
-            const TileArgs a = it.a;
-            if constexpr (FAM == 128) k_forward_2d_tma_body<RAY>(a, &it.tmap, it.status, bx, by);
-            else k_forward_2d_body<RAY>(a, bx, by);
-        }
+    if constexpr (FAM == kBlock1) adjoint_block_body<1, true, false>(a0, it.a, bx);
+    if constexpr (FAM == kBlock1Single) adjoint_block_body<1, false, false>(a0, it.a, bx);
+    if constexpr (FAM == kBlock2) adjoint_block_body<2, true, false>(a0, it.a, bx);
+    if constexpr (FAM == kBlock2Single) adjoint_block_body<2, false, false>(a0, it.a, bx);
+    if constexpr (FAM == kBlockRay) {
+        if (it.vz == 8) { if (it.vec) adjoint_block_body<2, true, true>(a0, it.a, bx); else adjoint_block_body<2, false, true>(a0, it.a, bx); }
+        else { if (it.vec) adjoint_block_body<1, true, true>(a0, it.a, bx); else adjoint_block_body<1, false, true>(a0, it.a, bx); }
     }
-    if constexpr (FAM == 256 && !RAY) {
-        if (it.kind == KB_BTABLE) {
-            const Args a = it.a;
-            const bool full = a.nZ % (32 * it.vz) == 0;
-            if (a.nZ % 4) { if (it.vz == 8) k_backward_blk_body<8, false, true>(a, it.btab4, it.bcidx, bx); else k_backward_blk_body<4, false, true>(a, it.btab4, it.bcidx, bx); }
-            else if (it.vz == 8) { if (full) k_backward_blk_body<8, true>(a, it.btab4, it.bcidx, bx); else k_backward_blk_body<8, false>(a, it.btab4, it.bcidx, bx); }
-            else if (it.vz == 6) k_backward_blk_body<6, true>(a, it.btab4, it.bcidx, bx);
-            else if (it.vz == 5) k_backward_blk_body<5, true>(a, it.btab4, it.bcidx, bx);
-            else { if (full) k_backward_blk_body<4, true>(a, it.btab4, it.bcidx, bx); else k_backward_blk_body<4, false>(a, it.btab4, it.bcidx, bx); }
-        }
+    if constexpr (FAM == kTile || FAM == kTilePlain) {
+        const TileArgs a = it.a;
+        if constexpr (FAM == kTile) k_forward_2d_tma_body<RAY>(a, &it.tmap, it.status, bx, by);
+        else k_forward_2d_body<RAY>(a, bx, by);
     }
-    if constexpr ((FAM & 8) != 0 || ((FAM & 2) != 0 && !RAY)) {
+    if constexpr (FAM == kTable4 || FAM == kTable8) {
+        constexpr int VZ = FAM == kTable8 ? 8 : 4;
+        const Args a = it.a;
+        if (a.nZ % (32 * VZ) == 0) k_backward_blk_body<VZ, true>(a, it.btab4, it.bcidx, bx);
+        else k_backward_blk_body<VZ, false>(a, it.btab4, it.bcidx, bx);
+    }
+    if constexpr (FAM == kTable56) {
+        const Args a = it.a;
+        if (it.vz == 6) k_backward_blk_body<6, true>(a, it.btab4, it.bcidx, bx);
+        else k_backward_blk_body<5, true>(a, it.btab4, it.bcidx, bx);
+    }
+    if constexpr (FAM == kTableUneven) {
+        const Args a = it.a;
+        if (it.vz == 8) k_backward_blk_body<8, false, true>(a, it.btab4, it.bcidx, bx);
+        else k_backward_blk_body<4, false, true>(a, it.btab4, it.bcidx, bx);
+    }
+    if constexpr (FAM == kBackHeavy || (FAM == kBackFast && !RAY)) {
         if (it.kind == KB_2D) {
             const TileArgs a = it.a;
             k_backward_2d_body<RAY>(a, bx);
@@ -2156,28 +2182,17 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
             else k_backward_fast_body<4, RAY>(a, bx, by);
         }
     }
-    if constexpr ((FAM & 4) != 0) {
-        if (it.kind == KA_BLOCK) {
-            const Args a = it.a;
-            if (it.vz == 8) { if (it.vec) adjoint_block_body<2, true, RAY>(a, bx); else adjoint_block_body<2, false, RAY>(a, bx); }
-            else { if (it.vec) adjoint_block_body<1, true, RAY>(a, bx); else adjoint_block_body<1, false, RAY>(a, bx); }
-        }
-    }
 }
 
-// FAM: the body families this instance carries -- 1 the fast forward, 128
-// the 2-D forward, 2 the fast, batched and 2-D backprojections without per-ray
-// absorption, 4 adjoint, 8 the other backprojections (generic with occlusion
-// or per-ray absorption, fast with per-ray absorption), 16 the generic forward
-// with occlusion or per-ray absorption, 32 / 64 the generic forward /
-// backprojection without either, 256 the block-table backprojection, 512 the 2-D
-// forward with plain staging; a batch launches one instance per family
-// present, so no body is compiled around the registers of rarer ones and each
-// keeps about its direct kernel's occupancy.
+// families whose calls may have per-ray absorption, and those whose calls all have
+constexpr bool ray_family(int fam) { return fam == kStripRay || fam == kBlockRay; }
+constexpr bool both_family(int fam) { return fam == kBackHeavy || fam == kTile || fam == kTilePlain; }
+
+// no body is compiled around the registers of rarer ones, and each keeps about its direct kernel's occupancy
 template <int FAM>
 __device__ __forceinline__ void item_body(const Item& it, unsigned bx, unsigned by) {
     if (it.kind == KF_GEN || it.kind == KB_GEN || it.kind == KA_GEN) {
-        if constexpr (FAM == 32 || FAM == 64) {
+        if constexpr (FAM == kFwdGen || FAM == kBackGen) {
             // the lean generic families: no occlusion, no per-ray absorption
             const Args a = it.a;
             if (it.absm == VAM_ABS_MASK) {
@@ -2187,14 +2202,14 @@ __device__ __forceinline__ void item_body(const Item& it, unsigned bx, unsigned 
                 if (it.vz == 4) lean_gen_body<FAM, 4, VAM_ABS_NONE>(it, a, bx, by);
                 else lean_gen_body<FAM, 1, VAM_ABS_NONE>(it, a, bx, by);
             }
-        } else if constexpr ((FAM & (4 | 8 | 16)) != 0) {
+        } else if constexpr (FAM == kAdjGen || FAM == kBackHeavy || FAM == kFwdHeavy) {
             if (it.vz == 4) { if (it.occ) gen_body_fam<FAM, 4, true>(it, bx, by); else gen_body_fam<FAM, 4, false>(it, bx, by); }
             else { if (it.occ) gen_body_fam<FAM, 1, true>(it, bx, by); else gen_body_fam<FAM, 1, false>(it, bx, by); }
         }
     } else if (it.ray) {
-        if constexpr (FAM != 2) fast_body<FAM, true>(it, bx, by);   // nor a per-ray absorption body
+        if constexpr (ray_family(FAM) || both_family(FAM)) fast_body<FAM, true>(it, bx, by);
     } else {
-        fast_body<FAM, false>(it, bx, by);
+        if constexpr (!ray_family(FAM)) fast_body<FAM, false>(it, bx, by);
     }
 }
 
@@ -2372,15 +2387,17 @@ __device__ __forceinline__ int batch_find(const BatchParams& P, unsigned t) {
 }
 static_assert(sizeof(BatchParams) < 32000, "batch parameters must fit the 32 KB kernel parameter space");
 
-// Resident CTAs per SM each instance asks for, i.e. its register cap: the
-// lean generic backprojection fits 40 registers (six CTAs, as its direct
-// kernel: a 160^3 x 720 call ran 1.36x longer at four), the fast and 2-D
-// backprojections and the 2-D forward 48 (five), the fast forward and the
-// lean generic forward 64 (four); the heavy instances keep 80 (three), the
-// block-table backprojection (four bodies: 4 or 8 slices, full or partial z
-// chunks) 128 (two).
+// Resident CTAs per SM each instance asks for, i.e. its register cap: the lean generic backprojection fits 40
+// registers (six CTAs, as its direct kernel: a 160^3 x 720 call ran 1.36x longer at four), the fast and 2-D
+// backprojections and the 2-D forward 48 (five), the lean generic forward 64 (four), the strips and blocks 128 (two, as
+// their direct kernels), the bin table with eight slices per lane too (256^2 x 256 x 90 angles 320 us, 420 with three);
+// the rest keep 80 (three; the bin table with four slices per lane 156 us at 128^3 x 180, 180 with two).
+constexpr int batch_ctas(int fam) {
+    return fam == kBackGen ? 6 : fam == kBackFast || fam == kTile ? 5 : fam == kFwdGen ? 4
+         : (fam >= kStrip1 && fam <= kStripRay) || (fam >= kBlock1 && fam <= kBlockRay) || fam == kTable8 ? 2 : 3;
+}
 template <int FAM>
-__global__ void __launch_bounds__(256, FAM == 64 ? 6 : (FAM == 2 || FAM == 128 ? 5 : (FAM == 32 ? 4 : (FAM == 1 || FAM == 256 ? 2 : 3))))
+__global__ void __launch_bounds__(256, batch_ctas(FAM))
     k_batch(const __grid_constant__ BatchParams P) {
     __shared__ unsigned s_t[2];
     __shared__ int s_idx[2];
@@ -2413,20 +2430,12 @@ __global__ void __launch_bounds__(256, FAM == 64 ? 6 : (FAM == 2 || FAM == 128 ?
 }
 
 using BatchKernel = void (*)(BatchParams);
-BatchKernel batch_kernel(int fam) {
-    switch (fam) {
-        case 1: return k_batch<1>;
-        case 2: return k_batch<2>;
-        case 4: return k_batch<4>;
-        case 8: return k_batch<8>;
-        case 16: return k_batch<16>;
-        case 32: return k_batch<32>;
-        case 64: return k_batch<64>;
-        case 128: return k_batch<128>;
-        case 256: return k_batch<256>;
-        default: return k_batch<512>;
-    }
+template <int... F>
+BatchKernel batch_kernel_of(int fam, std::integer_sequence<int, F...>) {
+    static const BatchKernel all[] = {k_batch<F>...};
+    return all[fam];
 }
+BatchKernel batch_kernel(int fam) { return batch_kernel_of(fam, std::make_integer_sequence<int, kFamilies>()); }
 
 // mask pre-pass of every fast forward of a batch (blockIdx.y = call)
 __global__ void k_batch_premask(const __grid_constant__ BatchParams P) {
@@ -2958,7 +2967,7 @@ struct vam_batch {
     int device;
     unsigned* d_counter;
     int sms;
-    int per_sm[513][4];        // resident CTAs per SM of k_batch<fam> (fam 1 .. 512) per
+    int per_sm[kFamilies][4];        // resident CTAs per SM of k_batch<fam> per
                                // dynamic shared-memory bucket (kSmemBuckets)
     std::vector<Item> host;    // the described calls of the last list, in queue order
     std::vector<int> group;    // first call of each launch (kBatchMaxItems calls per launch)
@@ -2992,12 +3001,12 @@ extern "C" int vam_batch_create(int32_t device, vam_batch** out) {
     VAM_REQUIRE(g.ok, VAM_ERR_CUDA, "vam_batch_create: cannot select device");
     int sms = 0;
     VAM_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    int per_sm[513][4] = {};
+    int per_sm[kFamilies][4] = {};
     // residency for each dynamic shared-memory bucket up to the largest a call may ask for (48 KB,
     // the batched backprojection's trig table), queried once here, so a list never needs a
     // runtime query (which would not be allowed during graph capture); the opt-in limit is
     // raised first, as 48 KB plus the kernel's static shared memory exceeds the default
-    for (int fam : {1, 2, 4, 8, 16, 32, 64, 128, 256, 512}) {
+    for (int fam = 0; fam < kFamilies; ++fam) {
         VAM_TRY_CUDA(cudaFuncSetAttribute(batch_kernel(fam), cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
         for (int k = 0; k < 4; ++k) {
             VAM_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[fam][k], batch_kernel(fam),
@@ -3062,6 +3071,20 @@ double time_weight(const Item& it) {
     }
 }
 
+int batch_family(const Item& d) {
+    const bool gen_heavy = d.occ || d.absm == VAM_ABS_RAY;
+    switch (d.kind) {
+        case KF_GEN: return gen_heavy ? kFwdHeavy : kFwdGen;
+        case KB_GEN: return gen_heavy ? kBackHeavy : kBackGen;
+        case KF_FAST: return d.ray ? kStripRay : d.vz == 8 ? (d.vec ? kStrip2 : kStrip2Single) : (d.vec ? kStrip1 : kStrip1Single);
+        case KA_BLOCK: return d.ray ? kBlockRay : d.vz == 8 ? (d.vec ? kBlock2 : kBlock2Single) : (d.vec ? kBlock1 : kBlock1Single);
+        case KF_2D: return d.tma ? kTile : kTilePlain;  // (plain staging: no tensor map encoder)
+        case KB_BTABLE: return d.a.nZ % 4 ? kTableUneven : d.vz == 8 ? kTable8 : d.vz == 4 ? kTable4 : kTable56;
+        case KA_GEN: return kAdjGen;
+        default: return d.ray ? kBackHeavy : kBackFast;
+    }
+}
+
 // describe every call, order the queue, number the tickets; no CUDA call
 int batch_prepare(vam_batch* b, const vam_work* work, int32_t n) {
     VAM_REQUIRE(n <= kBatchMaxItems * 64, VAM_ERR_SHAPE, "vam_batch: at most 3072 calls per list");
@@ -3076,17 +3099,7 @@ int batch_prepare(vam_batch* b, const vam_work* work, int32_t n) {
         const int rc = describe(w.plan, op, w.in, w.out, items[i], "vam_batch", false, (w.op & VAM_OP_PADDED) != 0);
         if (rc != VAM_OK) return rc;
         const Item& d = items[i];
-        // generic bodies with occlusion or per-ray absorption, and per-ray fast backprojections, go
-        // to the heavy families (8 backward, 16 forward)
-        const bool gen_heavy = d.occ || d.absm == VAM_ABS_RAY;
-        if (d.kind == KB_GEN) items[i].family = gen_heavy ? 8 : 64;
-        else if (d.family == 2 && d.ray) items[i].family = 8;
-        if (d.kind == KF_GEN) items[i].family = gen_heavy ? 16 : 32;
-        // the 2-D forward instance carries the TMA-staged body only; plain staging (no tensor map
-        // encoder) has its own
-        if (d.kind == KF_2D && !d.tma) items[i].family = 512;
-        if (d.kind == KB_BTABLE) items[i].family = 256;
-
+        items[i].family = batch_family(d);
         VAM_REQUIRE((long long)items[i].gx * items[i].gy < (1LL << 31), VAM_ERR_SHAPE, "vam_batch: call grid too large");
         items[i].cost = (long long)std::llround((double)items[i].cost * time_weight(items[i]));
     }
@@ -3112,10 +3125,9 @@ int batch_prepare(vam_batch* b, const vam_work* work, int32_t n) {
     for (int g0 = 0, g1 = 0; g0 < n; g0 = g1) {
         g1 = g0 + 1;
         while (g1 < n && g1 - g0 < kBatchMaxItems && items[g1].family == items[g0].family) ++g1;
-        int fam = 0;
+        const int fam = items[g0].family;
         unsigned gsmem = 0;
         for (int i = g0; i < g1; ++i) {
-            fam |= items[i].family;
             gsmem = std::max(gsmem, items[i].smem);
             b->any_pre |= items[i].pre_in != nullptr;
         }

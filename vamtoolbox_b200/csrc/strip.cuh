@@ -212,8 +212,9 @@ __device__ __forceinline__ bool strip_place(const FastArgs& a, unsigned bx, unsi
     return true;
 }
 
+// (param: the arguments where the launch left them, for the call at the end; a copy's address would keep it in memory)
 template <int Q, bool VEC, bool RAY>
-__device__ __forceinline__ void forward_strip_body(const FastArgs& a, unsigned bx, unsigned by) {
+__device__ __forceinline__ void forward_strip_body(const FastArgs& a, const FastArgs& param, unsigned bx, unsigned by) {
     constexpr int M = strip_bins(Q), U = Q == 2 ? 3 : 4, VZ = 4 * Q;
     StripRing& ring = strip_ring();
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -432,7 +433,7 @@ __device__ __forceinline__ void forward_strip_body(const FastArgs& a, unsigned b
                 if (VEC ? e / 2 < n : 2 * e + 1 < n) bad = fmaf(hi, 0.f, bad);
             }
         if (__any_sync(kFull, bad != 0.f)) {
-            forward_strip_samples<Q, VEC, RAY>(a, bx, by);
+            forward_strip_samples<Q, VEC, RAY>(param, bx, by);
             return;
         }
     }
@@ -484,8 +485,8 @@ __device__ __noinline__ void forward_strip_samples(const FastArgs& a, unsigned b
 // 128 registers, two blocks per SM: rows in flight per warp hide more than a third block does (three at 80
 // registers: 0.88 against 0.82 ms at 256^3 x 360)
 template <int Q, bool VEC, bool RAY>
-__global__ void __launch_bounds__(256, 2) k_forward_strip(FastArgs a) {
-    forward_strip_body<Q, VEC, RAY>(a, blockIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(256, 2) k_forward_strip(const __grid_constant__ FastArgs a) {
+    forward_strip_body<Q, VEC, RAY>(a, a, blockIdx.x, blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -547,7 +548,7 @@ template <int Q, bool VEC, bool RAY>
 __device__ __noinline__ void adjoint_block_rows(const Args& a, unsigned bx);
 
 template <int Q, bool VEC, bool RAY>
-__device__ __forceinline__ void adjoint_block_body(const Args& a, unsigned bx) {
+__device__ __forceinline__ void adjoint_block_body(const Args& a, const Args& param, unsigned bx) {
     constexpr int U = Q == 2 ? 2 : 4, VZ = 4 * Q, R = 32 / kBlockBins;
     BlockRing& ring = block_ring();
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -673,7 +674,7 @@ __device__ __forceinline__ void adjoint_block_body(const Args& a, unsigned bx) {
             if (VEC ? e / 2 < n : 2 * e + 1 < n) bad = fmaf(hi, 0.f, bad);
         }
     if (__any_sync(kFull, bad != 0.f)) {  // as in the strips: an infinity only where it is sampled
-        adjoint_block_rows<Q, VEC, RAY>(a, bx);
+        adjoint_block_rows<Q, VEC, RAY>(param, bx);
         return;
     }
     if constexpr (Q == 1)
@@ -752,8 +753,8 @@ __device__ __noinline__ void adjoint_block_rows(const Args& a, unsigned bx) {
 }
 
 template <int Q, bool VEC, bool RAY>
-__global__ void __launch_bounds__(256, 2) k_adjoint_block(Args a) {
-    adjoint_block_body<Q, VEC, RAY>(a, blockIdx.x);
+__global__ void __launch_bounds__(256, 2) k_adjoint_block(const __grid_constant__ Args a) {
+    adjoint_block_body<Q, VEC, RAY>(a, a, blockIdx.x);
 }
 
 }  // namespace
