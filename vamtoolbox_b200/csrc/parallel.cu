@@ -1861,8 +1861,9 @@ enum Kind : int {
 // their rows in flight in local memory (transpose of 128^3 x 180 angles 507 us in a batch; 142 so, 124 on its own).
 enum Fam : int {
     kStrip1 = 0, kStrip1Single, kStrip2, kStrip2Single, kStripRay,  // strips: slices per lane, float4 rows or single
+    kStripExact, kStripExactSingle, kStripExactRay,
     kBackFast,                                                      // fast, batched and 2-D backprojections
-    kAdjGen, kBlock1, kBlock1Single, kBlock2, kBlock2Single, kBlockRay,
+    kAdjGen, kBlock1, kBlock1Single, kBlock2, kBlock2Single, kBlockRay, kBlockExact, kBlockExactSingle, kBlockExactRay,
     kBackHeavy,  // generic backprojection with occlusion or per-ray absorption, the fast ones with the latter
     kFwdHeavy,   // generic forward with occlusion or per-ray absorption
     kFwdGen, kBackGen,
@@ -1892,6 +1893,8 @@ struct Item {
     const int4* btab4;  // KB_BTABLE: the plan's 2 x 2 block bin table and its block index
     const int* bcidx;
     int* status;       // the plan's status word (kernels with bounded waits record timeouts there)
+    int exact;         // KF_FAST, KA_BLOCK: sums that keep what their rounding drops
+    int pad_;
     int tma, vec;      // vec (KF_FAST): 1 when the rows load as float4s.  KF_2D: tma is 1 when tmap describes a.in and the tiles are staged by TMA loads
     CUtensorMap tmap;   // read from parameter space, as a direct launch's __grid_constant__ argument
 };
@@ -1985,6 +1988,11 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     // enough: at 122^2 x 440 angles the generic kernel takes 59 / 88 / 164 us with 4 / 8 / 12 slices (float4
     // rows) and 70 / 125 / 188 with 2 / 3 / 6 (single floats), the strips 86 / 88 / 88 and 98 / 99 / 102, and
     // 1.6 times that where no angle has a partner 180 degrees away.
+    // Sums: the lanes among which the generic kernel shares a bin's samples or a pixel's angles, and the groups among
+    // which a strip or block does (four slices per lane).  Where it has more lanes, and no kernel but it served the call
+    // before the strips and blocks, their sums are the exact ones (strip.cuh), so that no slice count is less exact.
+    const int lanes = 32 / choose_layout(plan->nZ, aligned16).LZ;
+    const int groups = plan->nZ <= 16 ? 8 : plan->nZ <= 32 ? 4 : plan->nZ <= 64 ? 2 : 1;
     const bool strips = plan->nZ > 8 || (plan->nZ > 4 && plan->nZ % 4 != 0);
     if (op == Op::Forward && !plan->has_occ && strips && want != 1 &&
         (long)plan->nY * plan->nX * plan->nZ < (1L << 31)) {
@@ -2000,6 +2008,9 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         it.kind = KF_FAST; it.ray = ray;
         it.vec = rows4 && (padded || aligned16);
         it.vz = want == 4 || (want != 8 && plan->nZ <= 128) ? 4 : 8;
+        // (a strip's batches are sums of their own already: as exact as two lanes per bin.  From 58 slices in float4
+        // rows the less exact k_forward_fast served before.)
+        it.exact = it.vz == 4 && lanes >= std::max(4, 2 * groups) && !(aligned16 && fast_vz(plan->nZ, true, 0.45));
         a.lz_shift = 5;
         if (it.vz == 4)  // lanes to spare take other pixels
             while (a.lz_shift > 2 && (4 << (a.lz_shift - 1)) >= plan->nZ) --a.lz_shift;
@@ -2021,7 +2032,9 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         a.zs = zs;
         it.kind = KA_BLOCK; it.ray = ray;
         it.vec = rows4 && (padded || aligned16);
-        it.vz = want == 4 || (want != 8 && plan->nZ <= 128) ? 4 : 8;
+        // (from 96 slices in float4 rows a table of weights served before, its sums as here)
+        it.exact = want != 8 && lanes > groups && !(aligned16 && fast_vz(plan->nZ, true, 0.74));
+        it.vz = want == 4 || it.exact || (want != 8 && plan->nZ <= 128) ? 4 : 8;
         a.lz_shift = 5;
         if (it.vz == 4)
             while (a.lz_shift > 2 && (4 << (a.lz_shift - 1)) >= plan->nZ) --a.lz_shift;
@@ -2138,6 +2151,18 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
         if (it.vz == 8) { if (it.vec) forward_strip_body<2, true, true>(f, it.f, bx, by); else forward_strip_body<2, false, true>(f, it.f, bx, by); }
         else { if (it.vec) forward_strip_body<1, true, true>(f, it.f, bx, by); else forward_strip_body<1, false, true>(f, it.f, bx, by); }
     }
+    if constexpr (FAM == kStripExact) forward_strip_body<1, true, false, true>(f, it.f, bx, by);
+    if constexpr (FAM == kStripExactSingle) forward_strip_body<1, false, false, true>(f, it.f, bx, by);
+    if constexpr (FAM == kStripExactRay) {
+        if (it.vec) forward_strip_body<1, true, true, true>(f, it.f, bx, by);
+        else forward_strip_body<1, false, true, true>(f, it.f, bx, by);
+    }
+    if constexpr (FAM == kBlockExact) adjoint_block_body<1, true, false, true>(a0, it.a, bx);
+    if constexpr (FAM == kBlockExactSingle) adjoint_block_body<1, false, false, true>(a0, it.a, bx);
+    if constexpr (FAM == kBlockExactRay) {
+        if (it.vec) adjoint_block_body<1, true, true, true>(a0, it.a, bx);
+        else adjoint_block_body<1, false, true, true>(a0, it.a, bx);
+    }
     if constexpr (FAM == kBlock1) adjoint_block_body<1, true, false>(a0, it.a, bx);
     if constexpr (FAM == kBlock1Single) adjoint_block_body<1, false, false>(a0, it.a, bx);
     if constexpr (FAM == kBlock2) adjoint_block_body<2, true, false>(a0, it.a, bx);
@@ -2185,7 +2210,7 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
 }
 
 // families whose calls may have per-ray absorption, and those whose calls all have
-constexpr bool ray_family(int fam) { return fam == kStripRay || fam == kBlockRay; }
+constexpr bool ray_family(int fam) { return fam == kStripRay || fam == kStripExactRay || fam == kBlockRay || fam == kBlockExactRay; }
 constexpr bool both_family(int fam) { return fam == kBackHeavy || fam == kTile || fam == kTilePlain; }
 
 // no body is compiled around the registers of rarer ones, and each keeps about its direct kernel's occupancy
@@ -2272,7 +2297,8 @@ void launch_fast(const Item& it, dim3 grid, cudaStream_t st) {
             break;
         case KB_2D: k_backward_2d<RAY><<<grid, block, it.smem, st>>>(it.a); break;
         case KF_FAST:
-            if (it.vz == 8) { if (it.vec) k_forward_strip<2, true, RAY><<<grid, block, 0, st>>>(it.f); else k_forward_strip<2, false, RAY><<<grid, block, 0, st>>>(it.f); }
+            if (it.exact) { if (it.vec) k_forward_strip<1, true, RAY, true><<<grid, block, 0, st>>>(it.f); else k_forward_strip<1, false, RAY, true><<<grid, block, 0, st>>>(it.f); }
+            else if (it.vz == 8) { if (it.vec) k_forward_strip<2, true, RAY><<<grid, block, 0, st>>>(it.f); else k_forward_strip<2, false, RAY><<<grid, block, 0, st>>>(it.f); }
             else { if (it.vec) k_forward_strip<1, true, RAY><<<grid, block, 0, st>>>(it.f); else k_forward_strip<1, false, RAY><<<grid, block, 0, st>>>(it.f); }
             break;
         case KB_BATCHED:
@@ -2286,7 +2312,8 @@ void launch_fast(const Item& it, dim3 grid, cudaStream_t st) {
             else k_backward_fast<4, RAY><<<grid, block, 0, st>>>(it.a);
             break;
         case KA_BLOCK:
-            if (it.vz == 8) { if (it.vec) k_adjoint_block<2, true, RAY><<<grid, block, 0, st>>>(it.a); else k_adjoint_block<2, false, RAY><<<grid, block, 0, st>>>(it.a); }
+            if (it.exact) { if (it.vec) k_adjoint_block<1, true, RAY, true><<<grid, block, 0, st>>>(it.a); else k_adjoint_block<1, false, RAY, true><<<grid, block, 0, st>>>(it.a); }
+            else if (it.vz == 8) { if (it.vec) k_adjoint_block<2, true, RAY><<<grid, block, 0, st>>>(it.a); else k_adjoint_block<2, false, RAY><<<grid, block, 0, st>>>(it.a); }
             else { if (it.vec) k_adjoint_block<1, true, RAY><<<grid, block, 0, st>>>(it.a); else k_adjoint_block<1, false, RAY><<<grid, block, 0, st>>>(it.a); }
             break;
         default: break;
@@ -2394,7 +2421,7 @@ static_assert(sizeof(BatchParams) < 32000, "batch parameters must fit the 32 KB 
 // the rest keep 80 (three; the bin table with four slices per lane 156 us at 128^3 x 180, 180 with two).
 constexpr int batch_ctas(int fam) {
     return fam == kBackGen ? 6 : fam == kBackFast || fam == kTile ? 5 : fam == kFwdGen ? 4
-         : (fam >= kStrip1 && fam <= kStripRay) || (fam >= kBlock1 && fam <= kBlockRay) || fam == kTable8 ? 2 : 3;
+         : (fam >= kStrip1 && fam <= kStripExactRay) || (fam >= kBlock1 && fam <= kBlockExactRay) || fam == kTable8 ? 2 : 3;
 }
 template <int FAM>
 __global__ void __launch_bounds__(256, batch_ctas(FAM))
@@ -3076,8 +3103,10 @@ int batch_family(const Item& d) {
     switch (d.kind) {
         case KF_GEN: return gen_heavy ? kFwdHeavy : kFwdGen;
         case KB_GEN: return gen_heavy ? kBackHeavy : kBackGen;
-        case KF_FAST: return d.ray ? kStripRay : d.vz == 8 ? (d.vec ? kStrip2 : kStrip2Single) : (d.vec ? kStrip1 : kStrip1Single);
-        case KA_BLOCK: return d.ray ? kBlockRay : d.vz == 8 ? (d.vec ? kBlock2 : kBlock2Single) : (d.vec ? kBlock1 : kBlock1Single);
+        case KF_FAST: if (d.exact) return d.ray ? kStripExactRay : d.vec ? kStripExact : kStripExactSingle;
+                      return d.ray ? kStripRay : d.vz == 8 ? (d.vec ? kStrip2 : kStrip2Single) : (d.vec ? kStrip1 : kStrip1Single);
+        case KA_BLOCK: if (d.exact) return d.ray ? kBlockExactRay : d.vec ? kBlockExact : kBlockExactSingle;
+                       return d.ray ? kBlockRay : d.vz == 8 ? (d.vec ? kBlock2 : kBlock2Single) : (d.vec ? kBlock1 : kBlock1Single);
         case KF_2D: return d.tma ? kTile : kTilePlain;  // (plain staging: no tensor map encoder)
         case KB_BTABLE: return d.a.nZ % 4 ? kTableUneven : d.vz == 8 ? kTable8 : d.vz == 4 ? kTable4 : kTable56;
         case KA_GEN: return kAdjGen;

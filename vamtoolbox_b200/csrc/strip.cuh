@@ -101,6 +101,14 @@ __device__ __forceinline__ void fma_pairs(unsigned long long& acc, unsigned long
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(w2), "l"(v2));
 }
 
+// what the rounding of t = s + x drops (s the larger)
+__device__ __forceinline__ unsigned long long dropped(unsigned long long s, unsigned long long t, unsigned long long x) {
+    unsigned long long d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(t), "l"(s));
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(d));
+    return d;
+}
+
 // whole: the float4s may be stored as such; otherwise (padded rows) slice by slice, the first `left` of them
 // (those the output has: a padded row holds up to three more)
 template <int Q, bool VEC>
@@ -174,16 +182,14 @@ __device__ __forceinline__ void strip_finish(const FastArgs& a, int2 task, bool 
     const double4 tr = a.trig[task.x];
     const double rowb = fma(-tr.y, (double)j, tr.w), colb = fma(tr.x, (double)j, tr.z);
     const int N = a.nY;
-    if (j < N) {
-        unsigned long long o[2 * Q];
+    // (an end sample is formed by itself: its four taps would otherwise round the whole sum four times)
+    for (int end = 0; end < 2; ++end) {
+        if (end ? j == 0 : j == N) continue;
+        unsigned long long o[2 * Q] = {};
+        strip_sample<Q, VEC>(a, volz, fma(tr.x, (double)(end * N), rowb), fma(tr.y, (double)(end * N), colb), o, n, lz);
 #pragma unroll
-        for (int e = 0; e < 2 * Q; ++e) o[e] = sum[e];
-        strip_sample<Q, VEC>(a, volz, rowb, colb, o, n, lz);
-        strip_store<Q, VEC>(here, o, n, lz, a.vs == a.nZ, a.nZ - z0);
-    }
-    if (j > 0) {
-        strip_sample<Q, VEC>(a, volz, fma(tr.x, (double)N, rowb), fma(tr.y, (double)N, colb), sum, n, lz);
-        strip_store<Q, VEC>(there, sum, n, lz, a.vs == a.nZ, a.nZ - z0);
+        for (int e = 0; e < 2 * Q; ++e) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(o[e]) : "l"(sum[e]));
+        strip_store<Q, VEC>(end ? there : here, o, n, lz, a.vs == a.nZ, a.nZ - z0);
     }
 }
 
@@ -213,7 +219,11 @@ __device__ __forceinline__ bool strip_place(const FastArgs& a, unsigned bx, unsi
 }
 
 // (param: the arguments where the launch left them, for the call at the end; a copy's address would keep it in memory)
-template <int Q, bool VEC, bool RAY>
+//
+// EXACT: the running sum of the batches keeps what its rounding drops.  For slice counts that the generic kernel gives
+// more lanes per bin than the strips do (Sums in describe()): its lanes' partial sums are otherwise the more exact ones
+// (64^2 x 40 x 90 angles, relative to float64: generic 4.3e-8, strips 5.9e-8, so 4.4e-8; 17.4 -> 18.6 us).
+template <int Q, bool VEC, bool RAY, bool EXACT = false>
 __device__ __forceinline__ void forward_strip_body(const FastArgs& a, const FastArgs& param, unsigned bx, unsigned by) {
     constexpr int M = strip_bins(Q), U = Q == 2 ? 3 : 4, VZ = 4 * Q;
     StripRing& ring = strip_ring();
@@ -318,8 +328,9 @@ __device__ __forceinline__ void forward_strip_body(const FastArgs& a, const Fast
         for (int m = 0; m < M; ++m)
 #pragma unroll
             for (int e = 0; e < VZ / 2; ++e) {
+                const unsigned long long was = sum[m][e];
                 asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[m][e]) : "l"(acc[m][e]));
-                acc[m][e] = 0ull;
+                acc[m][e] = EXACT ? dropped(was, sum[m][e], acc[m][e]) : 0ull;
             }
     };
     if (some) {
@@ -484,9 +495,9 @@ __device__ __noinline__ void forward_strip_samples(const FastArgs& a, unsigned b
 
 // 128 registers, two blocks per SM: rows in flight per warp hide more than a third block does (three at 80
 // registers: 0.88 against 0.82 ms at 256^3 x 360)
-template <int Q, bool VEC, bool RAY>
+template <int Q, bool VEC, bool RAY, bool EXACT = false>
 __global__ void __launch_bounds__(256, 2) k_forward_strip(const __grid_constant__ FastArgs a) {
-    forward_strip_body<Q, VEC, RAY>(a, a, blockIdx.x, blockIdx.y);
+    forward_strip_body<Q, VEC, RAY, EXACT>(a, a, blockIdx.x, blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -529,15 +540,18 @@ __device__ __forceinline__ bool block_place(const Args& a, unsigned bx, int& i, 
 }
 
 // Weight of bin J for the pixel at lattice position (J0 + dj, K0 + dk): its samples within one pixel of it.
-template <bool RAY>
-__device__ __forceinline__ float bin_weight(const Args& a, float cf, float sf, float d, float dk, float K0, float sent) {
+// cs: cos and sin and (EXACT) what their float32 values leave out.
+template <bool RAY, bool EXACT>
+__device__ __forceinline__ float bin_weight(const Args& a, float4 cs, float d, float dk, float K0, float sent) {
     const float kc = rintf(dk);
+    const float sd = EXACT ? fmaf(cs.y, d, cs.w * d) : cs.y * d, cd = EXACT ? fmaf(cs.x, d, cs.z * d) : cs.x * d;
     float w = 0.f;
 #pragma unroll
     for (int b = -1; b <= 1; ++b) {
         const float k = K0 + (kc + (float)b);
         const float kk = (k >= 0.f && k <= (float)(a.nY - 1)) ? (kc + (float)b) - dk : 1e9f;  // outside: no weight
-        float h = __saturatef(1.f - fabsf(fmaf(cf, kk, -sf * d))) * __saturatef(1.f - fabsf(fmaf(sf, kk, cf * d)));
+        float h = __saturatef(1.f - fabsf(fmaf(cs.x, kk, EXACT ? fmaf(cs.z, kk, -sd) : -sd))) *
+                  __saturatef(1.f - fabsf(fmaf(cs.y, kk, EXACT ? fmaf(cs.w, kk, cd) : cd)));
         if (RAY && h != 0.f) h *= ray_factor(k - (float)a.C, sent, a.alpha);
         w += h;
     }
@@ -547,7 +561,9 @@ __device__ __forceinline__ float bin_weight(const Args& a, float cf, float sf, f
 template <int Q, bool VEC, bool RAY>
 __device__ __noinline__ void adjoint_block_rows(const Args& a, unsigned bx);
 
-template <int Q, bool VEC, bool RAY>
+// EXACT: as for the strips, summing every six angles' rows on their own, with cos and sin to more than float32 (the
+// generic kernel forms its weights in float64): 64^2 x 40 x 90 1.0e-7 -> 4.0e-8 (generic 4.2e-8), 18.6 -> 20.4 us.
+template <int Q, bool VEC, bool RAY, bool EXACT = false>
 __device__ __forceinline__ void adjoint_block_body(const Args& a, const Args& param, unsigned bx) {
     constexpr int U = Q == 2 ? 2 : 4, VZ = 4 * Q, R = 32 / kBlockBins;
     BlockRing& ring = block_ring();
@@ -557,11 +573,23 @@ __device__ __forceinline__ void adjoint_block_body(const Args& a, const Args& pa
     const int LZ = 1 << a.lz_shift, g = lane >> a.lz_shift, G = 32 >> a.lz_shift;
     const float* __restrict__ bz = a.in + z0;
 
-    unsigned long long acc[4][VZ / 2];
+    unsigned long long acc[4][VZ / 2], sum[4][EXACT ? VZ / 2 : 1];
 #pragma unroll
     for (int q = 0; q < 4; ++q)
 #pragma unroll
-        for (int e = 0; e < VZ / 2; ++e) acc[q][e] = 0ull;
+        for (int e = 0; e < VZ / 2; ++e) acc[q][e] = sum[q][EXACT ? e : 0] = 0ull;
+    auto carry = [&]() {
+        if constexpr (EXACT) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int e = 0; e < VZ / 2; ++e) {
+                    const unsigned long long was = sum[q][e];
+                    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[q][e]) : "l"(acc[q][e]));
+                    acc[q][e] = dropped(was, sum[q][e], acc[q][e]);
+                }
+        }
+    };
     auto entries = [&](int at, float4 (&t)[U], unsigned (&o)[U]) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -610,7 +638,9 @@ __device__ __forceinline__ void adjoint_block_body(const Args& a, const Args& pa
             const double ri = (double)i0 - tr.w, ci = (double)j0 - tr.z;
             const double Jf = fma(-tr.y, ri, tr.x * ci), Kf = fma(tr.x, ri, tr.y * ci);
             const double Jn = rint(Jf), Kn = rint(Kf);
-            const float cf = (float)tr.x, sf = (float)tr.y, dj = (float)(Jf - Jn), dk = (float)(Kf - Kn);
+            const float cf = (float)tr.x, sf = (float)tr.y;
+            const float4 cs = make_float4(cf, sf, EXACT ? (float)(tr.x - (double)cf) : 0.f, EXACT ? (float)(tr.y - (double)sf) : 0.f);
+            const float dj = (float)(Jf - Jn), dk = (float)(Kf - Kn);
             // bins from 1.5 (|cos| + |sin|) below the block's centre on
             const float lo = dj + 0.5f * (cf - sf) - 1.5f * (fabsf(cf) + fabsf(sf));
             const float jr = ceilf(lo - 1e-5f) + (float)slot;  // the bin, from Jn
@@ -628,7 +658,7 @@ __device__ __forceinline__ void adjoint_block_body(const Args& a, const Args& pa
                 for (int q = 0; q < 4; ++q) {
                     const float pr = (float)(q >> 1), pc = (float)(q & 1);  // the pixel, from the block's first
                     const float d = jr - (dj + (pc * cf - pr * sf)), k = dk + (pr * cf + pc * sf);
-                    W[q] = bin_weight<RAY>(a, cf, sf, d, k, (float)Kn, sent);
+                    W[q] = bin_weight<RAY, EXACT>(a, cs, d, k, (float)Kn, sent);
                     listed |= W[q] != 0.f;
                 }
             }
@@ -649,6 +679,7 @@ __device__ __forceinline__ void adjoint_block_body(const Args& a, const Args& pa
             step(head + U * G + g * U, t0, v0, t1, v1);
             head = head + round < size ? head + round : 0;
         }
+        carry();
         __syncwarp();  // the entries worked off are free again
     }
     if (wait > 0) {  // the rest, filled up with entries of no weight (and the first row)
@@ -662,6 +693,13 @@ __device__ __forceinline__ void adjoint_block_body(const Args& a, const Args& pa
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) add1(t0[u], v0[u]);
+    carry();
+    if constexpr (EXACT) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int e = 0; e < VZ / 2; ++e) acc[q][e] = sum[q][e];
+    }
     __syncwarp();  // (the next call of a persistent block refills the ring)
     float bad = 0.f;
 #pragma unroll
@@ -752,9 +790,9 @@ __device__ __noinline__ void adjoint_block_rows(const Args& a, unsigned bx) {
     }
 }
 
-template <int Q, bool VEC, bool RAY>
+template <int Q, bool VEC, bool RAY, bool EXACT = false>
 __global__ void __launch_bounds__(256, 2) k_adjoint_block(const __grid_constant__ Args a) {
-    adjoint_block_body<Q, VEC, RAY>(a, a, blockIdx.x);
+    adjoint_block_body<Q, VEC, RAY, EXACT>(a, a, blockIdx.x);
 }
 
 }  // namespace
