@@ -86,3 +86,31 @@ def test_rows_are_padded_only_where_the_padded_kernels_serve_the_call(n, nz, na,
         elif op == _lib.OP_FORWARD and n * n * nz >= 2 ** 31:
             assert r.kernel == _lib.KERNEL_FORWARD_GENERIC, form
     assert padded or n * n * nz >= 2 ** 31 or n * na * nz >= 2 ** 31
+
+
+def test_few_slices_take_the_kernel_that_is_faster_there():
+    """Strips and blocks from the slice counts on at which they were measured to beat the generic kernels, which
+    depend on absorption, on angles 180 degrees apart and on the slice's size; a tuning chooses either."""
+    forward, adjoint = _lib.OP_FORWARD, _lib.OP_ADJOINT
+    strip, block = _lib.KERNEL_FORWARD_STRIP, _lib.KERNEL_ADJOINT_BLOCK
+    for n, nz, na, tasks, absorption, strips in [
+            (54, 16, 636, 318, _lib.ABS_RAY, False), (256, 32, 360, 180, _lib.ABS_RAY, False),
+            (256, 56, 360, 180, _lib.ABS_RAY, True), (96, 11, 90, 45, _lib.ABS_RAY, False),
+            (96, 15, 90, 45, _lib.ABS_RAY, True), (96, 16, 91, 91, _lib.ABS_NONE, False),
+            (96, 20, 91, 91, _lib.ABS_NONE, True), (96, 12, 90, 45, _lib.ABS_MASK, True),
+            (54, 16, 90, 45, _lib.ABS_MASK, False), (54, 5, 90, 45, _lib.ABS_NONE, True),
+            (96, 7, 91, 91, _lib.ABS_NONE, False), (32, 32, 90, 45, _lib.ABS_NONE, False),
+            (32, 45, 90, 45, _lib.ABS_NONE, True), (32, 60, 90, 45, _lib.ABS_RAY, True),
+            (64, 36, 30, 15, _lib.ABS_NONE, False), (96, 45, 8, 4, _lib.ABS_NONE, False),
+            (96, 117, 8, 4, _lib.ABS_NONE, True), (96, 128, 8, 4, _lib.ABS_RAY, True),
+            (12, 16, 11, 7, _lib.ABS_NONE, True)]:
+        got = route(n, nz, na, forward, absorption=absorption, tasks=tasks)[1].kernel
+        assert (got == strip) == strips, (n, nz, na, absorption)
+    for n, nz, absorption, blocks in [(32, 12, _lib.ABS_NONE, False), (32, 16, _lib.ABS_NONE, True),
+                                      (32, 24, _lib.ABS_RAY, False), (32, 28, _lib.ABS_RAY, True),
+                                      (32, 6, _lib.ABS_RAY, False), (54, 12, _lib.ABS_RAY, True)]:
+        assert (route(n, nz, 90, adjoint, absorption=absorption)[1].kernel == block) == blocks, (n, nz, absorption)
+    for op, vz, kernel in [(forward, "forward_vz", strip), (adjoint, "adjoint_vz", block)]:
+        assert route(32, 12, 90, op, **{vz: 4})[1].kernel == kernel
+        assert route(128, 128, 90, op, **{vz: 1})[1].kernel == kernel + 1
+    assert block + 1 == _lib.KERNEL_ADJOINT_GENERIC and strip + 1 == _lib.KERNEL_FORWARD_GENERIC

@@ -1842,6 +1842,45 @@ int fast_vz(int nZ, bool aligned, double min_eff) {
     return 0;
 }
 
+// A call of few angles on a small slice takes 5 to 20 us with strips and blocks and 3 to 13 without, about what the host
+// needs to issue it: the rules below leave those to them.
+bool issue_bound(const vam_parallel_plan& p) {
+    return p.nA < 16 && p.nX <= (p.abs_mode == VAM_ABS_RAY ? 40 : 64) && (long long)p.nY * p.nX * p.nZ * p.nA < 1500000;
+}
+
+// The least slice count at which the strips take an automatic forward; below, their weights are shared by too few
+// slices.  Generic / strips in us (four: the generic kernel reads float4s):
+//   four, angles in pairs 180 degrees apart (one strip sums both): 54^2 x 90 angles 10.9 / 12.3 with 16 slices, 20.0 /
+//     13.6 with 20; 96^2 x 90 27.1 / 22.0 with 12
+//   four, no pairs: 96^2 x 91 23.7 / 30.4 with 16 slices, 43.4 / 36.3 with 20
+//   four, per-ray absorption (no pairs, and a factor per weight): 256^2 x 360 454 / 894 with 16 slices, 854 / 971 with
+//     32, 1665 / 1142 with 56
+//   single slices, pairs: 54^2 x 90 15.4 / 14.4 with 5 slices, 96^2 x 90 30.7 / 25.8; no pairs: 96^2 x 91 31.2 / 38.7
+//     with 5, 44.7 / 39.0 with 9; per-ray absorption: 96^2 x 90 49.6 / 62.7 with 11, 67.9 / 64.8 with 15
+// Few strips (bins times pairs of angles: w) leave each waiting for its rows while the generic kernel spreads a bin over
+// a warp: 32^2 x 90 (w 1440) 8.9 / 10.7 with 32 slices, 13.0 / 11.6 with 36; 64^2 x 30 (w 960) 14.1 / 17.8 with 36, single
+// slices 23.3 / 22.4 with 33; 96^2 x 8 (w 384) 45 single slices 16 / 22, 117 slices 27 / 24.  From 58 slices in float4 rows
+// on they are the faster ones at any w.
+int strips_from(const vam_parallel_plan& p, bool four) {
+    const bool ray = p.abs_mode == VAM_ABS_RAY, pairs = !ray && 4LL * p.n_tasks_paired <= 3LL * p.nA;
+    const long long w = (long long)p.nX * (ray ? p.nA : p.n_tasks_paired);
+    if (issue_bound(p)) return four ? 9 : 5;
+    if (four && ray) return w < 4000 ? 58 : 56;
+    if (four) return w < 1400 ? 58 : w < 2000 ? 36 : pairs && p.nX >= 96 && w >= 2900 ? 12 : 20;
+    if (ray) return w < 800 ? 129 : w < 1800 ? 100 : w < 2800 ? 45 : w < 4000 ? 20 : 15;
+    return w < 350 ? 129 : w < 800 ? 80 : w < 1400 ? 33 : w < 2000 ? 18 : pairs ? 5 : 9;
+}
+
+// The same for the transpose's blocks, whose generic kernel evaluates all samples near a pixel: faster only for the
+// smallest slices (32^2 x 90 angles, four: 12 slices 13.3 / 15.7, 16 slices 28.7 / 13.4; per-ray absorption 27.1 / 33.8
+// with 24, 59.6 / 33.0 with 28, single slices 25.4 / 35.4 with 6, 58.0 / 32.2 with 7; 54^2 x 12 33.1 / 16.2 and, per-ray
+// absorption, 39.0 / 33.2).
+int blocks_from(const vam_parallel_plan& p, bool four) {
+    const bool ray = p.abs_mode == VAM_ABS_RAY, few = p.nX < 48 && !issue_bound(p);
+    if (four) return !few ? 9 : ray ? 28 : 16;
+    return few && ray ? 7 : 5;
+}
+
 // ---------------------------------------------------------------------------
 // Dispatch.  describe() decides which kernel body serves a call (fast or
 // generic path, vector width, angle batch, weight table) and fills its
@@ -1981,19 +2020,19 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         }
         return VAM_OK;
     }
-    // detector strips: every volume (any slice count, any alignment) without occlusion unless the generic
-    // kernel is tuned (1).  Eight slices per lane where one 128-slice chunk does not hold the volume.
-    // 201^2 x 117 x 240 angles: 3.92 -> 0.38 ms against the generic kernel, which evaluates every sample's
-    // coordinates in float64 for one slice per lane.  With few slices the strips' weights are not shared
-    // enough: at 122^2 x 440 angles the generic kernel takes 59 / 88 / 164 us with 4 / 8 / 12 slices (float4
-    // rows) and 70 / 125 / 188 with 2 / 3 / 6 (single floats), the strips 86 / 88 / 88 and 98 / 99 / 102, and
-    // 1.6 times that where no angle has a partner 180 degrees away.
+    // detector strips and, for the transpose, pixel blocks: any slice count and any alignment without occlusion from the
+    // slice counts on at which they beat the generic kernel, unless a tuning says which (1 the generic one, others
+    // these).  Eight slices per lane where one 128-slice chunk does not hold the volume.  201^2 x 117 x 240 angles: 3.92
+    // -> 0.36 ms against the generic kernel, which evaluates every sample's coordinates in float64 for one slice per
+    // lane.
     // Sums: the lanes among which the generic kernel shares a bin's samples or a pixel's angles, and the groups among
     // which a strip or block does (four slices per lane).  Where it has more lanes, and no kernel but it served the call
     // before the strips and blocks, their sums are the exact ones (strip.cuh), so that no slice count is less exact.
     const int lanes = 32 / choose_layout(plan->nZ, aligned16).LZ;
     const int groups = plan->nZ <= 16 ? 8 : plan->nZ <= 32 ? 4 : plan->nZ <= 64 ? 2 : 1;
-    const bool strips = plan->nZ > 8 || (plan->nZ > 4 && plan->nZ % 4 != 0);
+    const bool four = aligned16 && plan->nZ % 4 == 0;  // (what the generic kernel would read: float4s or single slices)
+    const bool strips = want == 0 ? plan->nZ >= (op == Op::Forward ? strips_from(*plan, four) : blocks_from(*plan, four))
+                                  : plan->nZ > 8 || (plan->nZ > 4 && plan->nZ % 4 != 0);
     if (op == Op::Forward && !plan->has_occ && strips && want != 1 &&
         (long)plan->nY * plan->nX * plan->nZ < (1L << 31)) {
         FastArgs& a = it.f;

@@ -110,8 +110,10 @@ class ParallelPlan:
         # 62.5 / 74.7 against 72.8 / 82.0 at 100^2 x 33 x 180; backprojection 12.4 against 13.7 at 64^2 x 9 x 90,
         # 246.8 against 497.8 at 200^2 x 33 x 180).  Above 112 slices the float4s of one pixel take a warp's lanes,
         # which leaves its angles to one lane after the other: slices of few pixels then gain nothing (46 against
-        # 42 us at 40^2 x 117 x 90; 47 against 83 at 56^2)
-        self.pad_from, self.pad_backward_from = 25e6, 3e6 if n_y >= 48 or n_z <= 112 else 2e8
+        # 42 us at 40^2 x 117 x 90; 47 against 83 at 56^2).  Nor do few angles of up to 80 slices, which the generic
+        # kernel shares among lanes (1.4 times the time at 128^2 to 384^2 x 65 x 4).
+        gains = (n_y >= 48 or n_z <= 112) and (self.angles.size >= 8 or n_z > 80)
+        self.pad_from, self.pad_backward_from = 25e6, 3e6 if gains else 2e8
         self.has_backward_table = False
         self._key = _pool_key(self.shape_vol, self.angles, self.device)
         reused = _pool_take(self._key)
