@@ -3,13 +3,13 @@
 The fastest vector width (slices per lane) and backprojection angle batch
 depend on the slice count, the number of angles and the device, so a plan can
 time every candidate once on its own device and keep the winner.  Winners are
-cached in a JSON file keyed by device name and problem shape, so later plans of
-the same shape apply the cached shape without timing anything.
+cached in a JSON file keyed by kernel revision, device name and problem shape, so
+later plans of the same shape apply the cached shape without timing anything.
 
 The cache file is ``$VAMTOOLBOX_B200_TUNE_CACHE`` when set, else
-``~/.cache/vamtoolbox_b200/tuning.json``.  Tuning changes launch shapes only:
-every candidate computes the same sums in the same order per slice, and the
-tests check each candidate against the oracle.
+``~/.cache/vamtoolbox_b200/tuning.json``.  Tuning chooses among kernels that
+compute the same sums, in orders of their own: results of two candidates differ
+by float32 rounding, and the tests check each against the oracle.
 """
 from __future__ import annotations
 
@@ -21,13 +21,16 @@ import torch
 
 from . import _lib
 
-# slices per lane: 1 = the generic kernel, 4 / 8 = the fast kernels (nZ % 4 == 0), 6 / 5 = the fast forward
-# on 192- / 160-slice chunks (nZ % 192 == 0 / nZ % 160 == 0)
-FORWARD_VZ = (1, 4, 5, 6, 8)
+# What the launch shapes mean: part of the cache's keys, raised whenever a kernel behind one of them changes, so that a
+# winner timed on other kernels is not applied to these.
+KERNEL_REVISION = 2
+
+# slices per lane: 1 = the generic kernel, 4 / 8 = the strips of three / two bins
+FORWARD_VZ = (1, 4, 8)
 # (slices per lane, angles per batch, bin table): the block table serves four or eight slices per lane,
 # and 0 (automatic) adds six / five on 192- / 160-slice chunks
 BACKWARD = ((1, 1, 0), (4, 1, 0), (8, 1, 0), (4, 2, 0), (8, 2, 0), (4, 4, 0), (4, 2, 1), (8, 2, 1), (0, 2, 1))
-ADJOINT = ((1, 0), (4, 1), (8, 1), (4, 0), (8, 0))           # (slices per lane, weight table on)
+ADJOINT = (1, 4, 8)  # slices per lane: 1 = the generic kernel, 4 / 8 = the pixel blocks
 
 _lock = threading.Lock()
 
@@ -42,7 +45,7 @@ def cache_path():
 def problem_key(plan):
     name = torch.cuda.get_device_name(plan.device).replace(" ", "_")
     ny, nx, nz = plan.shape_vol
-    return f"{name}|{ny}x{nx}x{nz}|na{plan.angles.size}|abs={plan.absorption or 'none'}|occ={int(plan.has_occlusion)}"
+    return f"k{KERNEL_REVISION}|{name}|{ny}x{nx}x{nz}|na{plan.angles.size}|abs={plan.absorption or 'none'}|occ={int(plan.has_occlusion)}"
 
 
 def _load(path):
@@ -81,19 +84,16 @@ def _time(fn, reps, warm):
 
 def measure(plan, reps=3, warm=1, ops=("forward", "backward", "adjoint")):
     """Time every candidate of ``ops`` on the plan's device; returns (tuning dict, timings in ms).
-    Ops left out keep the plan's current shape (the adjoint's weight table is then not built)."""
+    Ops left out keep the plan's current shape."""
     dev = plan.device
     with torch.cuda.device(dev):
         g = torch.Generator(device=dev).manual_seed(0)
         x = torch.rand(plan.shape_vol, device=dev, generator=g)
         b = torch.rand(plan.shape_sino, device=dev, generator=g)
         ob, ox = torch.empty_like(b), torch.empty_like(x)
-        table = plan.prepare_adjoint() if "adjoint" in ops else False
         times = {"forward": {}, "backward": {}, "adjoint": {}}
         base = plan.get_tuning()
         for vz in FORWARD_VZ if "forward" in ops else ():
-            if (vz == 6 and plan.shape_vol[2] % 192) or (vz == 5 and plan.shape_vol[2] % 160):
-                continue
             plan.set_tuning(dict(base, forward_vz=vz))
             times["forward"][str(vz)] = _time(lambda: plan.forward(x, ob), reps, warm)
         for vz, bt, tb in BACKWARD if "backward" in ops else ():
@@ -101,11 +101,9 @@ def measure(plan, reps=3, warm=1, ops=("forward", "backward", "adjoint")):
                 continue
             plan.set_tuning(dict(base, backward_vz=vz, backward_batch=bt, backward_table=tb))
             times["backward"][f"{vz},{bt},{tb}"] = _time(lambda: plan.backward_ref(b, ox), reps, warm)
-        for vz, tb in ADJOINT if "adjoint" in ops else ():
-            if tb and not table:
-                continue
-            plan.set_tuning(dict(base, adjoint_vz=vz, adjoint_table=tb))
-            times["adjoint"][f"{vz},{tb}"] = _time(lambda: plan.adjoint(b, ox), reps, warm)
+        for vz in ADJOINT if "adjoint" in ops else ():
+            plan.set_tuning(dict(base, adjoint_vz=vz))
+            times["adjoint"][str(vz)] = _time(lambda: plan.adjoint(b, ox), reps, warm)
         plan.set_tuning(base)
     best = dict(base)
     if times["forward"]:
@@ -114,7 +112,7 @@ def measure(plan, reps=3, warm=1, ops=("forward", "backward", "adjoint")):
         best["backward_vz"], best["backward_batch"], best["backward_table"] = map(
             int, min(times["backward"], key=times["backward"].get).split(","))
     if times["adjoint"]:
-        best["adjoint_vz"], best["adjoint_table"] = map(int, min(times["adjoint"], key=times["adjoint"].get).split(","))
+        best["adjoint_vz"] = int(min(times["adjoint"], key=times["adjoint"].get))
     return best, times
 
 
