@@ -885,7 +885,7 @@ constexpr int k2J = 64;     // forward: detector bins per tile
 constexpr int k2K = 64;     // forward: samples per bin per tile
 constexpr int k2Box = 96;   // forward: staged box side >= sqrt(2) (k2J + k2K - 2) + 5
 constexpr int k2Stride = k2Box + 1;
-constexpr int k2Smem = (k2Box * k2Stride + 4 * k2J) * 4;  // box + the k-group partial sums
+constexpr int k2Smem = k2Box * k2Stride * 4 + 4 * k2J * 8;  // box + the k-group partial sums
 constexpr int kB2 = 16;     // backprojection with per-ray absorption: pixel tile side
 constexpr int kB2A = 32;    // backprojection: angles per staged block (one per lane when staging)
 constexpr int kB2W = 30;    // backprojection with per-ray absorption: window bins per angle >= sqrt(2) (kB2 - 1) + 6
@@ -963,26 +963,28 @@ __device__ __forceinline__ float resum_2d(const Args& a, int theta, int j, int k
     return sum;
 }
 
-// Lattice row j's bins from the sum of its samples.
+// Lattice row j's bins from the sum of its samples, which is rounded to float32 here and nowhere before: sums over a
+// tile's samples are float32, sums over tiles, groups of samples and the end sample float64 (at 160^2 x 180 angles
+// 4.6e-8 -> 3.2e-8 relative to float64, the generic kernel's being 4.2e-8).
 template <bool RAY>
-__device__ __forceinline__ void store_2d(const Args& a, const Slice2d& t, const double4& tr, int j, float sum) {
+__device__ __forceinline__ void store_2d(const Args& a, const Slice2d& t, const double4& tr, int j, double sum) {
     const int N = a.nX;
-    if (!(fabsf(sum) <= 3.402823466e38f)) sum = resum_2d<RAY>(a, t.theta, j, t.kfirst);
-    if (j < N) a.out[(size_t)j * a.nA + t.theta] = t.ext ? sum + sample_2d(a, tr, j, 0) : sum;
+    if (!(fabs(sum) <= 3.402823466e38)) sum = resum_2d<RAY>(a, t.theta, j, t.kfirst);
+    if (j < N) a.out[(size_t)j * a.nA + t.theta] = (float)(t.ext ? sum + sample_2d(a, tr, j, 0) : sum);
     const int jp = 2 * a.C - j;
     if (t.partner >= 0 && jp >= 0 && jp < N)
-        a.out[(size_t)jp * a.nA + t.partner] = t.ext ? sum + sample_2d(a, tr, j, N) : sum;
+        a.out[(size_t)jp * a.nA + t.partner] = (float)(t.ext ? sum + sample_2d(a, tr, j, N) : sum);
 }
 
 // A tile that holds lattice row N alone (N a multiple of k2J): the block's threads share its samples.
-__device__ __forceinline__ void last_row_2d(const Args& a, const Slice2d& t, const double4& tr, float* part) {
+__device__ __forceinline__ void last_row_2d(const Args& a, const Slice2d& t, const double4& tr, double* part) {
     float v = 0.f;
     for (int k = t.kfirst + (int)threadIdx.x; k < a.nX; k += kWarpsPerBlock * kWarp) v += sample_2d(a, tr, a.nX, k);
     for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFull, v, off);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
-        float sum = 0.f;
+        double sum = 0.0;
         for (int w = 0; w < kWarpsPerBlock; ++w) sum += part[w];
         store_2d<false>(a, t, tr, a.nX, sum);
     }
@@ -1002,7 +1004,7 @@ template <bool RAY>
 __device__ __forceinline__ void k_forward_2d_body(const TileArgs& a, unsigned bx, unsigned by) {
     extern __shared__ float s_f2[];
     float* box = s_f2;
-    float* part = s_f2 + k2Box * k2Stride;
+    double* part = reinterpret_cast<double*>(s_f2 + k2Box * k2Stride);
     const Slice2d t2 = slice_2d(a, by);
     const int tj = threadIdx.x % k2J, tk = threadIdx.x / k2J;
     const int j0 = bx * k2J, j = j0 + tj;
@@ -1023,7 +1025,7 @@ __device__ __forceinline__ void k_forward_2d_body(const TileArgs& a, unsigned bx
     const double rb0 = fma(-s, (double)j0, tr.w), rb1 = fma(-s, (double)j1, tr.w);
     const double cb0 = fma(c, (double)j0, tr.z), cb1 = fma(c, (double)j1, tr.z);
     auto to_int = [](double v) { return (int)fmax(fmin(floor(v), 1e9), -1e9); };
-    float acc = 0.f;
+    double acc = 0.0;
     for (int k0 = t2.kfirst; k0 < a.nY; k0 += k2K) {
         const int k1 = min(k0 + k2K, a.nY) - 1;
         double rmin = 1e300, rmax = -1e300, cmin = 1e300, cmax = -1e300;
@@ -1108,7 +1110,7 @@ constexpr int kTmaW = 100, kTmaH = 96;  // box: 100 columns (x, 400 B) x 96 rows
 constexpr long kTmaWaitLimit = 1L << 24;  // try_wait polls before a block gives up
 // dynamic shared memory of the TMA tile body: 128 B of alignment slack, the box, the k-group partial sums
 // and the mbarrier
-constexpr int k2SmemTma = 128 + kTmaH * kTmaW * 4 + 4 * k2J * 4 + 16;
+constexpr int k2SmemTma = 128 + kTmaH * kTmaW * 4 + 4 * k2J * 8 + 16;
 
 
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
@@ -1127,7 +1129,7 @@ __device__ __forceinline__ void k_forward_2d_tma_body(const TileArgs& a, const C
                                                       unsigned bx, unsigned by) {
     extern __shared__ float s_f2[];
     float* box = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(s_f2) + 127) & ~(uintptr_t)127);
-    float* part = box + kTmaH * kTmaW;
+    double* part = reinterpret_cast<double*>(box + kTmaH * kTmaW);
     unsigned long long* mbar = reinterpret_cast<unsigned long long*>(part + 4 * k2J);
     const unsigned bar = smem_addr(mbar);
     const Slice2d t2 = slice_2d(a, by);
@@ -1160,7 +1162,7 @@ __device__ __forceinline__ void k_forward_2d_tma_body(const TileArgs& a, const C
     __syncthreads();
     unsigned phase = 0;
     bool failed = false;
-    float acc = 0.f;
+    double acc = 0.0;
     for (int k0 = t2.kfirst; k0 < a.nY; k0 += k2K) {
         const int k1 = min(k0 + k2K, a.nY) - 1;
         double rmin = 1e300, rmax = -1e300, cmin = 1e300, cmax = -1e300;
@@ -1225,7 +1227,7 @@ __device__ __forceinline__ void k_forward_2d_tma_body(const TileArgs& a, const C
 }
 
 template <bool RAY>
-__global__ void __launch_bounds__(256) k_forward_2d_tma(TileArgs a, const __grid_constant__ CUtensorMap tmap,
+__global__ void __launch_bounds__(256, RAY ? 0 : 4) k_forward_2d_tma(TileArgs a, const __grid_constant__ CUtensorMap tmap,
                                                         int* __restrict__ status) {
     k_forward_2d_tma_body<RAY>(a, &tmap, status, blockIdx.x, blockIdx.y);
 }
@@ -1235,9 +1237,10 @@ __global__ void __launch_bounds__(256) k_forward_2d(TileArgs a) {
     k_forward_2d_body<RAY>(a, blockIdx.x, blockIdx.y);
 }
 
-// With per-ray absorption: grid (ceil(nX / 16) * ceil(nY / 16)); 256 threads = one 16 x 16 pixel tile
-__device__ __forceinline__ void backward_2d_ray_body(const Args& a, unsigned bx) {
-    constexpr bool RAY = true;
+// With per-ray absorption: grid (ceil(nX / 16) * ceil(nY / 16)); 256
+// threads = one 16 x 16 pixel tile, bins and weights in float64
+template <bool RAY>
+__device__ __forceinline__ void backward_2d_f64_body(const Args& a, unsigned bx) {
     extern __shared__ float s_b2[];
     float* win = s_b2;                                            // [kB2A][kB2W]
     int* wlo = reinterpret_cast<int*>(s_b2 + kB2A * kB2W);        // [kB2A] first staged detector row
@@ -1343,7 +1346,9 @@ __device__ __forceinline__ void backward_2d_body(const TileArgs& a, unsigned bx)
     const int oi = i0 + wp, oj = jx0 + lane;
     const bool inside = oi < a.nY && oj < a.nX;
     const bool on = inside && a.circle[(long)oi * a.nX + oj];
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    // sums of a block's 16 angles, and of the blocks: a running sum of all of a group's angles is less exact than the
+    // generic kernel's lanes (256^2 x 360, relative to float64: 7.5e-8, generic 4.2e-8, so 3.2e-8)
+    float tot[4] = {0.f, 0.f, 0.f, 0.f};
     const bool any = __syncthreads_or(on);
     for (int th0 = 0; any && th0 < a.nA; th0 += kP2A) {
         const int na = min(kP2A, a.nA - th0);
@@ -1370,6 +1375,7 @@ __device__ __forceinline__ void backward_2d_body(const TileArgs& a, unsigned bx)
             }
         }
         __syncthreads();
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
         for (int al = ag; al < na; al += 4) {
             const float4 t4 = cs[al];
             const int2 lm = lim[al];
@@ -1406,28 +1412,31 @@ __device__ __forceinline__ void backward_2d_body(const TileArgs& a, unsigned bx)
                 if ((unsigned)k[q] < (unsigned)lm.y) acc[q] += x;
             }
         }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) tot[q] += acc[q];
         __syncthreads();
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) part[ag][r0 + q][lane] = acc[q];
+    for (int q = 0; q < 4; ++q) part[ag][r0 + q][lane] = tot[q];
     __syncthreads();
     if (inside) {
-        const float x = on ? (part[0][wp][lane] + part[1][wp][lane]) + (part[2][wp][lane] + part[3][wp][lane]) : 0.f;
+        const float x = on ? (float)(((double)part[0][wp][lane] + part[1][wp][lane]) +
+                                     ((double)part[2][wp][lane] + part[3][wp][lane])) : 0.f;
         const long p = (long)oi * a.nX + oj;
         a.out[p] = a.mask ? __ldg(a.mask + p) * x : x;
     }
     __syncthreads();  // (a persistent block's next tile reuses the shared memory)
 }
 
-template <bool RAY>
+template <bool RAY, bool F64>
 __device__ __forceinline__ void k_backward_2d_body(const TileArgs& a, unsigned bx) {
-    if constexpr (RAY) backward_2d_ray_body(a, bx);
+    if constexpr (F64) backward_2d_f64_body<RAY>(a, bx);
     else backward_2d_body(a, bx);
 }
 
-template <bool RAY>
+template <bool RAY, bool F64>
 __global__ void __launch_bounds__(256) k_backward_2d(TileArgs a) {
-    k_backward_2d_body<RAY>(a, blockIdx.x);
+    k_backward_2d_body<RAY, F64>(a, blockIdx.x);
 }
 
 // out = mask (per pixel, broadcast over z) * x; with nZ % 4 == 0 and aligned buffers four
@@ -2014,9 +2023,10 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
             it.smem = it.tma ? k2SmemTma : k2Smem;
         } else {
             it.kind = KB_2D;
-            it.gx = ray ? (unsigned)(((plan->nX + kB2 - 1) / kB2) * ((plan->nY + kB2 - 1) / kB2))
+            const bool f64 = ray;
+            it.gx = f64 ? (unsigned)(((plan->nX + kB2 - 1) / kB2) * ((plan->nY + kB2 - 1) / kB2))
                         : (unsigned)(((plan->nX + kP2X - 1) / kP2X) * ((plan->nY + kP2Y - 1) / kP2Y));
-            it.smem = ray ? kB2Smem : 0;
+            it.smem = f64 ? kB2Smem : 0;
         }
         return VAM_OK;
     }
@@ -2234,7 +2244,7 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
     if constexpr (FAM == kBackHeavy || (FAM == kBackFast && !RAY)) {
         if (it.kind == KB_2D) {
             const TileArgs a = it.a;
-            k_backward_2d_body<RAY>(a, bx);
+            k_backward_2d_body<RAY, RAY>(a, bx);
         } else if (it.kind == KB_BATCHED) {
             const Args a = it.a;
             if (it.vz == 8) k_backward_batched_body<8, 2, RAY>(a, bx, by);
@@ -2334,7 +2344,9 @@ void launch_fast(const Item& it, dim3 grid, cudaStream_t st) {
             if (it.tma) k_forward_2d_tma<RAY><<<grid, block, it.smem, st>>>(it.a, it.tmap, it.status);
             else k_forward_2d<RAY><<<grid, block, it.smem, st>>>(it.a);
             break;
-        case KB_2D: k_backward_2d<RAY><<<grid, block, it.smem, st>>>(it.a); break;
+        case KB_2D:
+            k_backward_2d<RAY, RAY><<<grid, block, it.smem, st>>>(it.a);
+            break;
         case KF_FAST:
             if (it.exact) { if (it.vec) k_forward_strip<1, true, RAY, true><<<grid, block, 0, st>>>(it.f); else k_forward_strip<1, false, RAY, true><<<grid, block, 0, st>>>(it.f); }
             else if (it.vz == 8) { if (it.vec) k_forward_strip<2, true, RAY><<<grid, block, 0, st>>>(it.f); else k_forward_strip<2, false, RAY><<<grid, block, 0, st>>>(it.f); }
