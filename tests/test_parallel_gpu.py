@@ -823,3 +823,22 @@ def test_slice_tiles_as_exact_as_the_generic_kernels(n, absn):
         p.set_tuning({"forward_vz": vz, "backward_vz": 0 if absn == "ray" else vz})
         err.append((relL2(p.forward(dev(x)).cpu().numpy(), rf), relL2(p.backward_ref(dev(b)).cpu().numpy(), rb)))
     assert err[0][0] <= err[1][0] + 2.0 ** -27 and err[0][1] <= err[1][1] + 2.0 ** -27, err
+
+
+@pytest.mark.parametrize("n,deg,bound", [(2048, 111.7, 11 * 2.0 ** -26), (4090, 328.5, 3 * 2.0 ** -25)])
+def test_slice_backprojection_weights_of_wide_slices(n, deg, bound):
+    """One angle's backprojection of alternating -1 and 1: a weight w gives 1 - 2 w, so its error is seen twice, and
+    one rounding of the result adds 2^-25.  Up to 2048 pixels a weight carries its rounding (2^-25), that of the
+    fraction (2^-26) and three of the low part (2^-27 each): twice 9 2^-27 and 2^-25, 11 2^-26.  Above it is formed in
+    float64 and rounded once."""
+    p = plan_for((n, n, 1), np.array([deg]))
+    b = np.where(np.arange(n) % 2, 1.0, -1.0)
+    got = p.backward_ref(dev(b.reshape(n, 1, 1))).cpu().numpy()[:, :, 0].astype(np.float64)
+    r, C = deg * (np.pi / 180.0), n // 2
+    t = (np.arange(n) - C)[None, :] * np.cos(r) - (np.arange(n) - C)[:, None] * np.sin(r)
+    j, w = np.floor(t).astype(int) + C, t - np.floor(t)
+    lin = np.linspace(-1, 1, n)
+    inside = (lin[:, None] ** 2 + lin[None, :] ** 2 <= 1) & (j >= 0) & (j < n - 1)
+    ref = np.where(inside, (1 - w) * b[j.clip(0, n - 1)] + w * b[(j + 1).clip(0, n - 1)], 0.0)
+    safe = inside & (w > 1e-9) & (w < 1 - 1e-9)
+    assert np.abs(got - ref)[safe].max() <= bound

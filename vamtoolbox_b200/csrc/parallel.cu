@@ -892,6 +892,7 @@ constexpr int kB2W = 30;    // backprojection with per-ray absorption: window bi
 constexpr int kB2Smem = kB2A * kB2W * 4 + kB2A * 4 + kB2A * 16;
 constexpr int kP2X = 32, kP2Y = 8;  // backprojection: pixel tile, four pixels per thread, four groups of angles
 constexpr int kP2A = 64;    // backprojection: angles per staged block
+constexpr int kP2Max = 2048;  // backprojection: above, the low part of cos and sin leaves 2^-24.3 of a bin uncertain
 constexpr int kP2W = 39;    // backprojection: window bins per angle >= |(kP2X - 1, kP2Y - 1)| + 6, odd (banks)
 
 // An angle and the one 180 degrees from it share their samples (see the strips): a tile sums both angles'
@@ -1237,7 +1238,7 @@ __global__ void __launch_bounds__(256) k_forward_2d(TileArgs a) {
     k_forward_2d_body<RAY>(a, blockIdx.x, blockIdx.y);
 }
 
-// With per-ray absorption: grid (ceil(nX / 16) * ceil(nY / 16)); 256
+// With per-ray absorption, or more pixels than the split of cos and sin serves: grid (ceil(nX / 16) * ceil(nY / 16)); 256
 // threads = one 16 x 16 pixel tile, bins and weights in float64
 template <bool RAY>
 __device__ __forceinline__ void backward_2d_f64_body(const Args& a, unsigned bx) {
@@ -1327,8 +1328,8 @@ __device__ __noinline__ float2 interp_bin(const double4* tr, float X, float Y, i
 //
 // np.interp's bin and weight without float64 arithmetic in the loop (its conversions and floors are issued at
 // an eighth of the float32 rate and took most of the time): cos and sin are split into a high part of few
-// enough bits that X ch - Y sh is exact in float32 and a low part (the plan's table), so t = A + B with A exact and B below one
-// bin, good to 2^-25 of a bin at any position; the nearest integer comes from adding 1.5 * 2^23.  Fractions
+// enough bits that X ch - Y sh is exact in float32 and a low part (the plan's table), so t = A + B with A exact and B below
+// 1/16 of a bin, the fraction good to 2^-24.9 of a bin at any position (one rounding of it is 2^-25), up to kP2Max pixels; the nearest integer comes from adding 1.5 * 2^23.  Fractions
 // within 1e-5 of an integer (where t decides between bins, or whether it is on the detector at all) are
 // formed again in float64 as numpy does, but for an exact integer (the centre pixel's, at every angle).
 // 512^2 x 720: 369 -> 219 us, 600^2 x 800 529 -> 310, 256^2 x 360 95 -> 53; issue is 75 % busy, 34
@@ -2023,7 +2024,7 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
             it.smem = it.tma ? k2SmemTma : k2Smem;
         } else {
             it.kind = KB_2D;
-            const bool f64 = ray;
+            const bool f64 = ray || plan->nX > kP2Max;
             it.gx = f64 ? (unsigned)(((plan->nX + kB2 - 1) / kB2) * ((plan->nY + kB2 - 1) / kB2))
                         : (unsigned)(((plan->nX + kP2X - 1) / kP2X) * ((plan->nY + kP2Y - 1) / kP2Y));
             it.smem = f64 ? kB2Smem : 0;
@@ -2244,7 +2245,8 @@ __device__ __forceinline__ void fast_body(const Item& it, unsigned bx, unsigned 
     if constexpr (FAM == kBackHeavy || (FAM == kBackFast && !RAY)) {
         if (it.kind == KB_2D) {
             const TileArgs a = it.a;
-            k_backward_2d_body<RAY, RAY>(a, bx);
+            if (RAY || a.nX > kP2Max) k_backward_2d_body<RAY, true>(a, bx);
+            else k_backward_2d_body<RAY, false>(a, bx);
         } else if (it.kind == KB_BATCHED) {
             const Args a = it.a;
             if (it.vz == 8) k_backward_batched_body<8, 2, RAY>(a, bx, by);
@@ -2345,7 +2347,8 @@ void launch_fast(const Item& it, dim3 grid, cudaStream_t st) {
             else k_forward_2d<RAY><<<grid, block, it.smem, st>>>(it.a);
             break;
         case KB_2D:
-            k_backward_2d<RAY, RAY><<<grid, block, it.smem, st>>>(it.a);
+            if (RAY || it.a.nX > kP2Max) k_backward_2d<RAY, true><<<grid, block, it.smem, st>>>(it.a);
+            else k_backward_2d<RAY, false><<<grid, block, it.smem, st>>>(it.a);
             break;
         case KF_FAST:
             if (it.exact) { if (it.vec) k_forward_strip<1, true, RAY, true><<<grid, block, 0, st>>>(it.f); else k_forward_strip<1, false, RAY, true><<<grid, block, 0, st>>>(it.f); }
@@ -2617,9 +2620,10 @@ extern "C" int vam_parallel_plan_create(const vam_parallel_geom* geom, vam_paral
     if (e == cudaSuccess) e = cudaMalloc(&p->d_status, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(p->d_status, 0, sizeof(int));
     if (e == cudaSuccess && p->nZ == 1) {
-        // cos and sin as a high part whose products with a pixel coordinate (and their difference) are exact in
-        // float32 and the rest: multiples of 2^-bits for coordinates below 2^(22 - bits)
-        const double unit = std::ldexp(1.0, 22 - (ilog2_pow2(p->nX) + 1));
+        // cos and sin as a high part whose products with a pixel coordinate are exact in float32, and their difference
+        // too, and the rest: multiples of 2^-bits, 2^(bits - 24) pixels wide.  A coordinate is at most half of that, so
+        // a product has 23 bits and the difference of two, at most sqrt 2 times as large, 24.
+        const double unit = std::ldexp(1.0, 24 - ilog2_pow2(p->nX));
         std::vector<float4> split(p->nA);
         for (int i = 0; i < p->nA; ++i) {
             const double ch = std::rint(trig[i].x * unit) / unit, sh = std::rint(trig[i].y * unit) / unit;
