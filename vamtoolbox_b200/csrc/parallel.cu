@@ -2019,7 +2019,11 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
             it.tma = use_tma && image_tensor_map(a.in, a.nX, a.nY, it.pre_wp ? it.pre_wp : a.nX, it.tmap) ? 1 : 0;
             it.a.tasks = ray ? plan->d_tasks_single : plan->d_tasks_paired;
             a.zs = it.pre_wp ? it.pre_wp : a.nX;
-            it.gx = (unsigned)((plan->nX + (plan->nX % 2 == 0 && !ray) + k2J - 1) / k2J);
+            // (lattice row N is a tile of its own where N is a multiple of k2J, if any angle has a partner: without one,
+            // blocks that have nothing to do left SMs with four of the others beside SMs with two, 256^2 x 91 angles
+            // 18.6 -> 22.3 us)
+            const bool row_n = plan->nX % 2 == 0 && !ray && plan->n_tasks_paired < plan->nA;
+            it.gx = (unsigned)((plan->nX + row_n + k2J - 1) / k2J);
             it.gy = (unsigned)(ray ? plan->nA : plan->n_tasks_paired);
             it.smem = it.tma ? k2SmemTma : k2Smem;
         } else {
