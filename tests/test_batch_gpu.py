@@ -264,3 +264,22 @@ def test_batch_of_every_kernel_family_bitwise(mode):
     torch.cuda.synchronize()
     for (p, op, _, out), r in zip(work, ref):
         assert torch.equal(out, r), (p.shape_vol, op)
+
+
+def test_batch_prepare_copies_nothing(monkeypatch):
+    """Preparing a list launches no padding copy; a submit after it reads the inputs as they are then."""
+    p = ParallelPlan(40, 40, 67, np.linspace(0, 360, 20, endpoint=False))
+    p.pad_from = p.pad_backward_from = 0
+    p.set_tuning({"forward_vz": 4})  # (the strips, which padded rows go to)
+    x, b = torch.rand(p.shape_vol, device="cuda"), torch.rand(p.shape_sino, device="cuda")
+    ob, ox = torch.empty_like(b), torch.empty_like(x)
+    batch, work = ProjectionBatch(), [(p, "forward", x, ob), (p, "backward_ref", b, ox)]
+    called, call = [], _lib.call
+    monkeypatch.setattr(_lib, "call", lambda name, *a: (called.append(name), call(name, *a))[1])
+    batch.prepare(work)
+    assert called == ["vam_batch_prepare"]
+    x.mul_(2.0)
+    batch.submit(work)
+    assert called.count("vam_pad_rows") == 2
+    monkeypatch.undo()
+    assert torch.equal(ob, p.forward(x)) and torch.equal(ox, p.backward_ref(b))

@@ -27,7 +27,8 @@ class ProjectionBatch:
 
     ``submit(work)`` runs the calls on the current stream (capturable in a
     CUDA graph: the call descriptions travel in the launch parameters);
-    ``prepare(work)`` only validates a list.  Calls of one batch run
+    ``prepare(work)`` only validates a list.  Inputs whose slice count is padded
+    to a multiple of four are copied by ``submit``, each time.  Calls of one batch run
     concurrently: no call may read another's output, and a single-slice plan
     whose forward stages its image appears at most once as a forward (the
     staged image is per plan).
@@ -56,7 +57,7 @@ class ProjectionBatch:
         except Exception:
             pass
 
-    def _works(self, work):
+    def _works(self, work, fill):
         items = []
         keep = []
         for plan, op, x, y in work:
@@ -73,7 +74,7 @@ class ProjectionBatch:
             code = OPS[op]
             if plan._pads(code):  # as the plan's own call (bit-identical to it)
                 with torch.cuda.device(self.device):
-                    x = plan._padded(x)
+                    x = plan._padded(x, fill)
                 code |= _lib.OP_PADDED
             items.append(_lib.Work(plan.handle.value, code, x.data_ptr(), y.data_ptr()))
             keep.append((plan, x, y))
@@ -81,13 +82,13 @@ class ProjectionBatch:
         return arr, keep
 
     def prepare(self, work):
-        arr, keep = self._works(work)
+        arr, keep = self._works(work, fill=False)
         with torch.cuda.device(self.device):
             _lib.call("vam_batch_prepare", self._h, arr, len(keep), _lib.stream_ptr(torch.cuda.current_stream(self.device)))
         self._arr, self._keep = arr, keep
 
     def submit(self, work):
-        arr, keep = self._works(work)
+        arr, keep = self._works(work, fill=True)
         with torch.cuda.device(self.device):
             _lib.call("vam_batch_submit", self._h, arr, len(keep), _lib.stream_ptr(torch.cuda.current_stream(self.device)))
         self._arr, self._keep = arr, keep

@@ -214,10 +214,13 @@ class ParallelPlan:
             return False
         return bool(_lib.load().vam_parallel_serves_padded(self._h, op))
 
-    def _padded(self, t):
-        """t ([a, b, nz]) with zero slices up to a multiple of four: a workspace of the current stream."""
+    def _padded(self, t, fill=True):
+        """t ([a, b, nz]) with zero slices up to a multiple of four: a workspace of the current stream (fill False:
+        the workspace alone)."""
         a, b, nz = t.shape
         out = torch.empty((a, b, (nz + 3) // 4 * 4), dtype=torch.float32, device=self.device)
+        if not fill:
+            return out
         _lib.call("vam_pad_rows", _lib.ptr(t), a * b, nz, _lib.ptr(out), self._stream())
         return out
 
