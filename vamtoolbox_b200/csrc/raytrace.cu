@@ -1109,10 +1109,11 @@ bool grid_symplectic(const RayArgs& a) {
 int64_t padded_voxels(const vam_ray_geom& g) { return (int64_t)(g.n_x + 2) * (g.n_y + 2) * (g.n_z + 2); }
 
 // the padded 3-D path serves the grid / symplectic configuration once its padded fields exist
-// (32-bit element offsets: fewer than 2^31 padded voxels; floor_near: axes below 2^22)
+// (32-bit element offsets: fewer than 2^31 padded voxels; axes below 10^6, beyond which corners_at decides every
+// neighbour in float64 and cell_corners would not)
 bool padded_path(const vam_ray_plan* p, const RayArgs& a) {
     return grid_symplectic(a) && !a.twod && p->d_npad && p->d_apad && p->d_spad &&
-           padded_voxels(p->g) < ((int64_t)1 << 31) && std::max(p->g.n_x, std::max(p->g.n_y, p->g.n_z)) < (1 << 22);
+           padded_voxels(p->g) < ((int64_t)1 << 31) && std::max(p->g.n_x, std::max(p->g.n_y, p->g.n_z)) < 1000000;
 }
 
 PadArgs make_pad_args(const vam_ray_plan* p) {
