@@ -41,9 +41,9 @@ constexpr int kStripRing = 128;  // ring entries per warp (the whole groups of t
 struct StripGeo {
     float4 coef;   // J and K per step of main and other
     float4 res;    // what the fixed-point coefficients leave out
-    int4 fix;      // the coefficients times 2^32, modulo 2^32
+    uint4 fix;     // the coefficients times 2^32, modulo 2^32 (unsigned: the sums wrap)
     float4 org;    // J and K at the origin; least other of the strip = slope * main + base
-    int2 fixorg;   // the origin in fixed point
+    uint2 fixorg;  // the origin in fixed point
     float4 cs;     // cos and sin, and what their float32 values leave out
 };
 
@@ -310,10 +310,10 @@ __device__ __forceinline__ void forward_strip_body(const FastArgs& a, const Fast
                          qw = rint(w * two32);
             q.coef = make_float4((float)x, (float)y, (float)z, (float)w);
             q.res = make_float4((float)(x - qx / two32), (float)(y - qy / two32), (float)(z - qz / two32), (float)(w - qw / two32));
-            q.fix = make_int4((int)(long long)qx, (int)(long long)qy, (int)(long long)qz, (int)(long long)qw);
+            q.fix = make_uint4((unsigned)(long long)qx, (unsigned)(long long)qy, (unsigned)(long long)qz, (unsigned)(long long)qw);
             q.org = make_float4((float)jo, (float)ko, (float)((rmain ? s : c) * inv),
                                 (float)((rmain ? (jlo - s * tr.w) * inv + tr.z : tr.w - (c * tr.z + jlo) * inv) - slack));
-            q.fixorg = make_int2((int)(long long)rint(jo * two32), (int)(long long)rint(ko * two32));
+            q.fixorg = make_uint2((unsigned)(long long)rint(jo * two32), (unsigned)(long long)rint(ko * two32));
             q.cs = make_float4((float)c, (float)s, (float)(c - (double)(float)c), (float)(s - (double)(float)s));
         }
         __syncwarp();
@@ -358,9 +358,10 @@ __device__ __forceinline__ void forward_strip_body(const FastArgs& a, const Fast
                 const float fo = (float)ot;
                 // nearest lattice point (Jn, Kn) and the pixel's offset from it
                 const float4 co = q.coef, re = q.res;
-                const int4 fx = q.fix;
-                const float dj = fmaf((float)(fx.x * mi + fx.y * ot + q.fixorg.x), 2.3283064e-10f, fmaf(re.x, fm, re.y * fo));
-                const float dk = fmaf((float)(fx.z * mi + fx.w * ot + q.fixorg.y), 2.3283064e-10f, fmaf(re.z, fm, re.w * fo));
+                const uint4 fx = q.fix;
+                const unsigned um = (unsigned)mi, uo = (unsigned)ot;
+                const float dj = fmaf((float)(int)(fx.x * um + fx.y * uo + q.fixorg.x), 2.3283064e-10f, fmaf(re.x, fm, re.y * fo));
+                const float dk = fmaf((float)(int)(fx.z * um + fx.w * uo + q.fixorg.y), 2.3283064e-10f, fmaf(re.z, fm, re.w * fo));
                 const float Jn = rintf(fmaf(co.x, fm, fmaf(co.y, fo, q.org.x)) - dj);
                 const float Kn = rintf(fmaf(co.z, fm, fmaf(co.w, fo, q.org.y)) - dk);
                 // cos and sin to more than float32: their rounding would scale every weight of the angle
