@@ -174,9 +174,10 @@ int vam_parallel_apply_padded(vam_parallel_plan* plan, int32_t op, const float* 
  * autotuner (vamtoolbox_b200/autotune.py times the candidates on the device
  * and caches the winner per device and problem shape).  Vector widths are the
  * slices each lane of a fast kernel carries (4 or 8; 1 = the generic kernel;
- * 0 = automatic; the fast kernels need nZ % 4 == 0; for a single slice any
- * value but 0 and 1 selects the shared-memory tile kernels, which 0 picks from
- * 192 (forward) and 320 (backprojection) pixels up); backward_batch is the
+ * 0 = automatic; the backprojection's fast kernels need nZ % 4 == 0, or padded
+ * rows; for a single slice any value but 0 and 1 selects the shared-memory
+ * tile kernels, which 0 picks from 192 pixels up: forward from 112 where the
+ * image needs no staging, backprojection from 320 with per-ray absorption); backward_batch is the
  * number of angles whose detector rows one warp loads together (1, 2 or 4);
  * adjoint_table is accepted and has no effect.
  * No counterpart in the reference. */

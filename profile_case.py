@@ -47,7 +47,6 @@ def run_parallel(n, na, calls, tuning, nz=None):
     x = torch.rand((n, n, nz), device="cuda", generator=g)
     b = torch.rand((n, na, nz), device="cuda", generator=g)
     ob, ox = torch.empty_like(b), torch.empty_like(x)
-    p.prepare_adjoint()
     for _ in range(calls):
         p.forward(x, ob)
         p.backward_ref(b, ox)

@@ -69,8 +69,6 @@ class ProjectionBatch:
             plan._check(y, shape_out, f"batch {op} output")
             if plan.device != self.device:
                 raise ValueError(f"plan on {plan.device}, batch on {self.device}")
-            if OPS[op] == _lib.OP_ADJOINT and not plan._adj_ready and not torch.cuda.is_current_stream_capturing():
-                plan.prepare_adjoint()
             code = OPS[op]
             if plan._pads(code):  # as the plan's own call (bit-identical to it)
                 with torch.cuda.device(self.device):

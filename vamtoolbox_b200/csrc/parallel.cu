@@ -9,13 +9,16 @@
 //                  (vamtoolbox/projector/Projector3DParallel.py:113-156)
 //   k_backward_ref R2, pixel-driven np.interp backprojection + circle clip
 //                  (Projector3DParallel.py:158-207)
-//   k_adjoint      exact transpose of k_forward, gather form, no atomics
+//   k_adjoint_block (strip.cuh), k_adjoint
+//                  transpose of the forward, gather form, no atomics
 //   k_occ_*        occlusion sinogram (Projector3DParallel.py:77-111)
 //
 // Sample coordinates are evaluated in float64 with the same expressions in
 // k_forward and k_adjoint (fma(c, k, fma(-s, j, m12)) etc.), so both see
 // bit-identical tap weights and the adjoint is the transpose of the forward
-// up to float32 summation order.  Weights and data are float32.
+// up to float32 summation order.  The strips and blocks, which most volumes
+// take, form the same weights from float32 offsets to the nearest sample, each
+// in its own way, good to about 2^-24.  Weights and data are float32.
 #include <float.h>
 #include <math.h>
 
@@ -268,26 +271,12 @@ __global__ void __launch_bounds__(256) k_forward(Args a) {
     k_forward_body<VZ, OCC, ABS>(a, blockIdx.x, blockIdx.y);
 }
 
-// Lane-interleaved z vectors of the fast kernels: with Q = VZ / 4, lane l of
+// Lane-interleaved z vectors of the computed-bin backprojections: with Q = VZ / 4, lane l of
 // a warp owns slices zbase + 4l + 128q + (0..3), q < Q, so every float4 load
 // of the warp covers 512 contiguous bytes (four 128-byte lines).  p points at
 // the lane's first slice; qn is the number of its vectors inside the volume.
-// Six / five slices per lane (192- / 160-slice chunks, full chunks only): a
-// float4 at zbase + 4l and a float2 at zbase + 128 + 2l or a float at
-// zbase + 128 + l (a 256- / 128-byte run per warp).
 template <int VZ>
-__device__ __forceinline__ void load_vz(const float* __restrict__ p, float* d, int qn = VZ / 4) {
-    if constexpr (VZ == 6 || VZ == 5) {
-        const float4 t = __ldg(reinterpret_cast<const float4*>(p));
-        d[0] = t.x; d[1] = t.y; d[2] = t.z; d[3] = t.w;
-        if constexpr (VZ == 6) {
-            const float2 u = __ldg(reinterpret_cast<const float2*>(p + 128 - 2 * (int)(threadIdx.x & 31)));
-            d[4] = u.x; d[5] = u.y;
-        } else {
-            d[4] = __ldg(p + 128 - 3 * (int)(threadIdx.x & 31));
-        }
-        return;
-    }
+__device__ __forceinline__ void load_vz(const float* __restrict__ p, float* d, int qn) {
 #pragma unroll
     for (int q = 0; q < VZ / 4; ++q) {
         float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -298,27 +287,15 @@ __device__ __forceinline__ void load_vz(const float* __restrict__ p, float* d, i
 
 template <int VZ>
 __device__ __forceinline__ void store_vz(float* __restrict__ p, const float* d, int qn) {
-    if constexpr (VZ == 6 || VZ == 5) {
-        *reinterpret_cast<float4*>(p) = make_float4(d[0], d[1], d[2], d[3]);
-        if constexpr (VZ == 6) *reinterpret_cast<float2*>(p + 128 - 2 * (int)(threadIdx.x & 31)) = make_float2(d[4], d[5]);
-        else p[128 - 3 * (int)(threadIdx.x & 31)] = d[4];
-        return;
-    }
 #pragma unroll
     for (int q = 0; q < VZ / 4; ++q)
         if (q < qn) *reinterpret_cast<float4*>(p + 128 * q) = make_float4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
 }
 
-// First slice and number of in-range vectors of a lane in z-chunk zc (six / five slices per lane: full
-// chunks, qn = 2 vectors).
+// First slice and number of in-range vectors of a lane in z-chunk zc.
 template <int VZ>
 __device__ __forceinline__ void lane_z(int zc, int lane, int nZ, int& z0, int& qn) {
     const int base = zc * 32 * VZ + 4 * lane;
-    if constexpr (VZ == 6 || VZ == 5) {
-        z0 = base;
-        qn = 2;
-        return;
-    }
     qn = 0;
 #pragma unroll
     for (int q = 0; q < VZ / 4; ++q) qn += (base + 128 * q < nZ) ? 1 : 0;
@@ -876,10 +853,11 @@ __global__ void __launch_bounds__(256, MINB) k_backward_blk(Args a, const int4* 
 // land in up to 32 different cache lines.  These kernels stage, per tile, the
 // region of the image (forward) or of the sinogram (backprojection) the tile's
 // samples touch, with coalesced row loads, and gather from shared memory.
-// The per-sample arithmetic is the generic kernels' (float64 coordinates and
-// np.interp bin, float32 weights); taps that fall outside the staged region
-// (not expected: the region is the tile's exact footprint plus a margin) are
-// read from global memory with the same bounds checks.
+// A tile's coordinates start from the generic kernels' float64 values and go on
+// in fixed point (forward) or come from cos and sin in two float32 parts
+// (backprojection; float64 with per-ray absorption); weights are float32.  The
+// staged region is the tile's exact footprint plus a margin, so no tap lies
+// outside it.
 // ---------------------------------------------------------------------------
 constexpr int k2J = 64;     // forward: detector bins per tile
 constexpr int k2K = 64;     // forward: samples per bin per tile
@@ -1836,11 +1814,9 @@ __global__ void k_occ2d_assign(const unsigned long long* __restrict__ slots, dou
 
 enum class Op { Forward, BackwardRef, Adjoint };
 
-// Slices per lane of the fast kernels for nZ slices (0 = use the generic
-// kernel): the widest vector whose lanes are at least min_eff busy.  The fast
-// forward gathers about four times as many samples per second as the generic
-// one, so it pays even with half of its lanes idle; the backprojectors' fast
-// and generic kernels are closer, so they ask for busier lanes.
+// Slices per lane of the computed-bin backprojections for nZ slices (0 = use the generic kernel): the widest vector
+// whose lanes are at least min_eff busy, 0.74 here.  (A forward and a transpose of this kind, the forward from 0.45 on,
+// served volumes before the strips and blocks: describe() compares with them.)
 int fast_vz(int nZ, bool aligned, double min_eff) {
     if (!aligned || nZ % 4) return 0;
     auto eff = [&](int vz) {
@@ -1893,7 +1869,7 @@ int blocks_from(const vam_parallel_plan& p, bool four) {
 
 // ---------------------------------------------------------------------------
 // Dispatch.  describe() decides which kernel body serves a call (fast or
-// generic path, vector width, angle batch, weight table) and fills its
+// generic path, vector width, angle batch, bin table) and fills its
 // arguments and grid; a direct call launches that one kernel, a batch runs the
 // same body for many calls inside one persistent launch.  Both paths therefore
 // compute bit-identical results.
@@ -1975,7 +1951,7 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     int vzf = 0;
     if (fast_ok && !padded) {
         if (want == 4 || want == 8) vzf = want;
-        else if (want == 0) vzf = fast_vz(plan->nZ, true, op == Op::Forward ? 0.45 : 0.74);
+        else if (want == 0) vzf = fast_vz(plan->nZ, true, 0.74);
     }
     const bool ray = plan->abs_mode == VAM_ABS_RAY;
     // 2-D slice: shared-memory tiles when tuned to them (any width but 1), or automatically for

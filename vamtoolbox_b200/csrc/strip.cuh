@@ -6,17 +6,17 @@
 //     W(j, p) = sum over samples k of hat(row(j, k) - row_p) hat(col(j, k) - col_p),  hat(d) = max(0, 1 - |d|),
 // the bilinear weights of all samples of the bin that touch the pixel (Projector3DParallel.py:137-156 via
 // skimage.warp).  Going through the pixels under the strip instead of through its samples loads every
-// pixel's row of slices once for all M bins and all their samples: 1.33 rows per sample for M = 4 (3.26 / 2
-// for two bins, 2.26 for one), against four taps per sample.  The rows' loads are what bounds the forward
-// (L1 data path), so this is where its time goes down.
+// pixel's row of slices once for all M bins and all their samples: 1.63 rows per sample for two bins, 1.42 for
+// three, against four taps per sample.  The rows' loads are what bounds the forward (L1 data path), so this is
+// where its time goes down.
 //
 // The warp lists the pixels in batches: the 32 lanes take R rows (or columns, whichever the rays run across)
 // of S candidate pixels, form each pixel's position in the rotated lattice and, from its fractions, its M
 // weights; pixels with any nonzero weight go through a ring in shared memory (pixel, M weights) that the same
 // warp then works off, U pixels at a time, the next U pixels' rows in flight meanwhile.
 //
-// Measured (B200): 256^3 x 360 angles 1.39 -> 0.84 ms, 512^2 x 128 x 720 7.30 -> 4.49 ms, 192^3 x 720 1.34 ->
-// 0.89 ms, 201^2 x 117 x 240 3.92 -> 0.37 ms against the sample kernels before.  At 256^3 the L1 data path is
+// Measured (B200): 256^3 x 360 angles 1.39 -> 0.83 ms, 512^2 x 128 x 720 7.30 -> 4.37 ms, 201^2 x 117 x 240 3.92 ->
+// 0.25 ms against the sample kernels before.  At 256^3 the L1 data path is
 // 68 % busy (a pixel is eight cycles of row and three or four of weights, which are written to every lane's
 // registers), issue 54 %, FP32 50 %; the rest is what 16 warps leave uncovered.
 #pragma once

@@ -129,7 +129,7 @@ def capture(fn, device):
     s = _capture_stream(device)
     # capture_begin / capture_end directly: the torch.cuda.graph context manager also runs a Python
     # garbage collection and empties the allocator cache on entry (tens of ms per capture), which the
-    # captured launches here do not need (they allocate nothing)
+    # captured launches here do not need (they allocate nothing but padded rows, from the graph's own pool)
     s.wait_stream(torch.cuda.current_stream(device))
     # no garbage collection while capturing: a collected object that owns device memory (a plan released
     # earlier) would free it inside the capture, which invalidates the graph

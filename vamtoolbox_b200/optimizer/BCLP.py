@@ -421,8 +421,9 @@ class DeviceIteration:
     ``step()`` issues, on the current stream: the backprojection of g into
     the dose, the fused dose pass (response, band error, operand and the 9
     loss / norm sums), the log append, the forward projection of the operand
-    and the clamped sinogram update.  Nothing is allocated and nothing syncs,
-    so ``capture()`` records it once as a CUDA graph.  ``reduce_stats`` (a
+    and the clamped sinogram update.  Nothing syncs, and nothing is allocated
+    but padded rows (see ``device_ops``), so ``capture()`` records it once as a
+    CUDA graph.  ``reduce_stats`` (a
     callable on the 9-float stats tensor) is the hook where a z-sharded run
     all-reduces the loss sums before the update.
     """

@@ -80,8 +80,8 @@ class CALDevice:
     sigmoid threshold of x / max(x) against the target, the forward
     projection of the residual, the (momentum) sinogram update clipped at
     zero, the backprojection, its maximum, VER and the log append.  Nothing
-    is allocated and nothing syncs, so a step is captured once as a CUDA
-    graph when the momentum is zero.
+    syncs, and nothing is allocated but padded rows (see ``device_ops``), so a
+    step is captured once as a CUDA graph when the momentum is zero.
     """
 
     def __init__(self, target_geo, proj_geo, options, A, ops=None):

@@ -66,8 +66,8 @@ class OSMODevice:
     device-side maximum and the normalisation floored at the inhibition
     level, the backprojection, its maximum and the normalisation floored at
     zero.  ``step()`` is one OSMO iteration (void half, gel half, VER, log
-    append).  Nothing is allocated and nothing syncs, so ``capture()``
-    records a step once as a CUDA graph.
+    append).  Nothing syncs, and nothing is allocated but padded rows
+    (see ``device_ops``), so ``capture()`` records a step once as a CUDA graph.
     """
 
     def __init__(self, target_geo, proj_geo, options, A, ops=None):

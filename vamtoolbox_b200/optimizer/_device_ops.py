@@ -5,7 +5,9 @@ device) for a projector of this package -- the parallel-beam plan (with the refe
 step before every backprojection), the ray tracer (deposit / integrate, its trajectory cache filled
 once for runs of several iterations), the vector-geometry projector, the algebraic propagator -- or
 None when the projector has no device entry points.  Each call writes into ``out`` on the current
-stream and allocates nothing, so an engine captures its iteration as one CUDA graph.
+stream, so an engine captures its iteration as one CUDA graph.  Nothing is allocated, but for a copy of the
+input where a parallel-beam plan pads its slice count to a multiple of four: torch's allocator gives it, while
+capturing from the graph's own pool, which lives as long as the graph.
 """
 from __future__ import annotations
 

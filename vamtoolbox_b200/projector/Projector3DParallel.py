@@ -99,7 +99,7 @@ class ParallelPlan:
         self.absorption = None
         self.has_occlusion = False
         self._adj_ready = False
-        # matched-transpose weight table: 16 B per pixel and angle (skipped above this size)
+        # what prepare_adjoint measures a weight table of 16 B per pixel and angle against (none is built any more)
         self.adj_table_limit_bytes = 8 << 30
         # backprojection bin table (32 B per 2 x 2 pixel block inside the circle and angle, about 8 B per
         # pixel), built here for volumes of 64 slices and more, so it exists before any capture of a
@@ -250,8 +250,8 @@ class ParallelPlan:
 
     def set_tuning(self, tuning):
         """Set launch shapes: dict with any of forward_vz / backward_vz / adjoint_vz (0 auto, 1 generic,
-        4, 8), backward_batch (1, 2, 4), adjoint_table, backward_table and forward_tma (0, 1); missing keys
-        keep their value."""
+        4, 8), backward_batch (1, 2, 4), adjoint_table (no effect), backward_table and forward_tma (0, 1);
+        missing keys keep their value."""
         cur = self.get_tuning()
         unknown = set(tuning) - set(self._TUNING_FIELDS)
         if unknown:
@@ -354,8 +354,6 @@ class ParallelPlan:
 
     def adjoint(self, sino, out=None):
         self._check(sino, self.shape_sino, "adjoint input")
-        if not self._adj_ready and not torch.cuda.is_current_stream_capturing():
-            self.prepare_adjoint()
         if out is None:
             out = torch.empty(self.shape_vol, dtype=torch.float32, device=self.device)
         self._check(out, self.shape_vol, "adjoint output")
