@@ -610,11 +610,18 @@ __device__ __forceinline__ void add_row(unsigned long long (&acc)[(VZ + 1) / 2],
     }
 }
 
+// eight slice pairs of each thread, a thread's 256 apart
+__device__ __forceinline__ unsigned long long* uneven_sums() {
+    __shared__ unsigned long long s[8 * kWarpsPerBlock * kWarp];
+    return s;
+}
+
 // sum += acc; with rest, what the rounding drops stays in acc for the next time
 __device__ __forceinline__ void carry_pair(unsigned long long& sum, unsigned long long& acc, bool rest) {
+    const unsigned long long was = sum;
     unsigned long long t, d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(sum), "l"(acc));
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(t), "l"(sum));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(was), "l"(acc));
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(t), "l"(was));
     asm("sub.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(d));
     if (!rest) acc = 0ull;
     sum = t;
@@ -661,9 +668,22 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
     // UNEVEN: the runs of angles summed up so far, acc being the current run.  The generic kernel, which these slice
     // counts took before, spreads a pixel's angles over up to four lanes (two above 128 slices); a running sum over
     // all angles is less exact (128^2 x 65 x 180 angles, relative to float64: 2.5e-7 against 5.9e-8; 201^2 x 117 x
-    // 240: 2.9e-7 against 2.1e-7).  Runs this long are at or below it (5.8e-8 and 5.6e-8) and cost a fifth of the
-    // time (335 -> 391 us at 201^2 x 117 x 240, 93 -> 113 at 128^2 x 65 x 180; generic 1951 and 364).
-    unsigned long long sum[4][UNEVEN ? NP : 1] = {};
+    // 240: 2.9e-7 against 2.1e-7).  Runs this long are at or below it (5.8e-8 and 5.6e-8) and cost 7 to 13 % of
+    // the time (335 -> 359 us at 201^2 x 117 x 240, 93 -> 105 at 128^2 x 65 x 180; generic 1951 and 364).
+    // in shared memory, as far as it goes (of eight slices per lane two pixels'): the registers are what rows in flight need
+    // (four slices per lane 391 -> 359 us at 201^2 x 117 x 240, eight 304 -> 270 at 201^3 x 120)
+    constexpr int INSMEM = UNEVEN ? 8 / NP : 0;
+    unsigned long long sum[4 - INSMEM > 0 ? 4 - INSMEM : 1][UNEVEN ? NP : 1] = {};
+    auto kept = [&](int q, int e) -> unsigned long long& {
+        if (q < INSMEM) return uneven_sums()[(q * NP + e) * (kWarpsPerBlock * kWarp) + threadIdx.x];
+        return sum[INSMEM < 4 ? q - INSMEM : 0][UNEVEN ? e : 0];
+    };
+    if constexpr (UNEVEN) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int e = 0; e < NP; ++e) kept(q, e) = 0ull;
+    }
     const int run = UNEVEN ? min(max(a.nA / (VZ == 8 ? 4 : 6), 4), 32) : 32;
     bool rest = true;
     auto carry = [&] {
@@ -671,7 +691,7 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
 #pragma unroll
             for (int q = 0; q < 4; ++q)
 #pragma unroll
-                for (int e = 0; e < NP; ++e) carry_pair(sum[q][e], acc[q][e], rest);
+                for (int e = 0; e < NP; ++e) carry_pair(kept(q, e), acc[q][e], rest);
         }
     };
     const int pc = bcidx[blk];
@@ -794,7 +814,7 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
 #pragma unroll
             for (int e2 = 0; e2 < NP; ++e2) {
                 float lo, hi;
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(sum[q][UNEVEN ? e2 : 0]));
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(kept(q, e2)));
                 bad = fmaf(hi, 0.f, fmaf(lo, 0.f, bad));
             }
         if (!__any_sync(0xffffffffu, bad != 0.f)) break;
@@ -802,7 +822,7 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
-            for (int e2 = 0; e2 < NP; ++e2) sum[q][UNEVEN ? e2 : 0] = acc[q][e2] = 0ull;
+            for (int e2 = 0; e2 < NP; ++e2) kept(q, e2) = acc[q][e2] = 0ull;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -812,7 +832,7 @@ __device__ __forceinline__ void k_backward_blk_body(const Args& a, const int4* _
         float v[2 * NP];
 #pragma unroll
         for (int e2 = 0; e2 < NP; ++e2)
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2 * e2]), "=f"(v[2 * e2 + 1]) : "l"(UNEVEN ? sum[q][UNEVEN ? e2 : 0] : acc[q][e2]));
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2 * e2]), "=f"(v[2 * e2 + 1]) : "l"(UNEVEN ? kept(q, e2) : acc[q][e2]));
         if (a.mask) {
             const float m = __ldg(a.mask + p);
 #pragma unroll
