@@ -8,7 +8,7 @@
     python profile_case.py batch --calls 1 --direct
 
 ``parallel`` runs forward, reference-parity backprojection and the matched
-adjoint (after building its weight table) on a random N x N x N volume with
+adjoint on a random N x N x N volume with
 ``angles`` equally spaced over 360 degrees; ``ray`` runs integrate and deposit
 of the curved-ray tracer through a graded-index, attenuating N^3 medium
 (physical path length, forward symplectic Euler), ``angles`` angles (with

@@ -17,8 +17,8 @@
 //
 // Measured (B200): 256^3 x 360 angles 1.39 -> 0.83 ms, 512^2 x 128 x 720 7.30 -> 4.37 ms, 201^2 x 117 x 240 3.92 ->
 // 0.25 ms against the sample kernels before.  At 256^3 the L1 data path is
-// 68 % busy (a pixel is eight cycles of row and three or four of weights, which are written to every lane's
-// registers), issue 54 %, FP32 50 %; the rest is what 16 warps leave uncovered.
+// 79 % busy (a pixel is eight cycles of row and three or four of weights, which are written to every lane's
+// registers), issue 50 %; the rest is what 16 warps leave uncovered.
 #pragma once
 
 #include "vam_internal.cuh"
