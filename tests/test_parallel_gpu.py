@@ -842,3 +842,23 @@ def test_slice_backprojection_weights_of_wide_slices(n, deg, bound):
     ref = np.where(inside, (1 - w) * b[j.clip(0, n - 1)] + w * b[(j + 1).clip(0, n - 1)], 0.0)
     safe = inside & (w > 1e-9) & (w < 1 - 1e-9)
     assert np.abs(got - ref)[safe].max() <= bound
+
+
+@pytest.mark.parametrize("nz", [5, 13, 25, 26, 27, 53, 55, 109, 111])
+@pytest.mark.parametrize("absn", [None, "mask", "ray"])
+def test_padded_generic_backprojection_shares_angles_as_before(nz, absn):
+    """The generic kernel on padded rows spreads a pixel's angles over as many lanes as on unpadded ones: where the
+    float4s of a row would take twice the lanes, the results are the unpadded call's bits."""
+    from vamtoolbox_b200 import _lib
+
+    rng = np.random.default_rng(nz)
+    p = plan_for((50, 50, nz), np.linspace(0, 360, 45, endpoint=False))
+    p.pad_backward_from = 0
+    assert p._pads(_lib.OP_BACKWARD_REF) and not p.has_backward_table
+    if absn == "mask":
+        p.set_absorption("mask", mask=rng.uniform(0.2, 1.0, (50, 50)))
+    elif absn == "ray":
+        p.set_absorption("ray", alpha_per_px=0.03, radius_px=23.5)
+    b, plain = dev(rng.uniform(-0.2, 1, p.shape_sino)), torch.empty(p.shape_vol, device="cuda")
+    _lib.call("vam_parallel_backward_ref", p.handle, _lib.ptr(b), _lib.ptr(plain), p._stream())
+    assert torch.equal(p.backward_ref(b), plain)

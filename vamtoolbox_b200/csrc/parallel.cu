@@ -2140,6 +2140,16 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         return VAM_OK;
     }
     Layout L = choose_layout(zs, padded || aligned16);
+    if (padded) {
+        // at least as many lanes for a pixel's angles as on unpadded rows, so that the sums are as exact (25 slices: seven
+        // float4s would take eight lanes and leave four, single slices four and leave eight; as many lanes are idle)
+        const int lz = choose_layout(plan->nZ, false).LZ;
+        if (lz < L.LZ) {
+            L.LZ = lz;
+            L.lz_shift = ilog2_pow2(lz);
+            L.zchunks = (L.zvec + lz - 1) / lz;
+        }
+    }
     Args& a = it.a;
     a.in = in; a.out = out; a.trig = plan->d_trig; a.circle = noclip ? plan->d_ones : plan->d_circle;
     a.mask = plan->d_mask; a.occ = plan->d_occ; a.occ_flag = plan->d_occ_flag;
