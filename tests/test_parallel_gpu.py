@@ -862,3 +862,23 @@ def test_padded_generic_backprojection_shares_angles_as_before(nz, absn):
     b, plain = dev(rng.uniform(-0.2, 1, p.shape_sino)), torch.empty(p.shape_vol, device="cuda")
     _lib.call("vam_parallel_backward_ref", p.handle, _lib.ptr(b), _lib.ptr(plain), p._stream())
     assert torch.equal(p.backward_ref(b), plain)
+
+
+@pytest.mark.parametrize("n,nz,na", [(48, 36, 61), (64, 9, 120), (64, 20, 90), (64, 40, 90), (40, 57, 60), (50, 63, 100),
+                                     (96, 33, 60), (96, 16, 90)])
+@pytest.mark.parametrize("value", [1.0, 0.3337])
+def test_strips_as_exact_as_the_generic_kernel_on_solid_parts(n, nz, na, value):
+    """Inside a solid part every sample is the part's value, which the generic kernel's few-lane sums add (nearly)
+    without rounding.  The strips' sums carry what their rounding drops to the end, so their error's norm is no larger
+    there either."""
+    ang = np.linspace(0, 360, na, endpoint=False)
+    p = plan_for((n, n, nz), ang)
+    i, j, k = np.ogrid[:n, :n, :nz]
+    r = np.hypot(i - n / 2.0 + 0.5, j - n / 2.0 + 0.5)
+    x = np.where((r < 0.42 * n) & (r > 0.1 * n + 0.1 * k * n / nz), np.float32(value), np.float32(0))
+    ref = O.parallel_forward(x.astype(np.float64), ang)
+    err = []
+    for vz in (4, 1):
+        p.set_tuning({"forward_vz": vz})
+        err.append(relL2(p.forward(dev(x)).cpu().numpy(), ref))
+    assert err[0] <= err[1], err

@@ -1856,25 +1856,33 @@ bool issue_bound(const vam_parallel_plan& p) {
 
 // The least slice count at which the strips take an automatic forward; below, their weights are shared by too few
 // slices.  Generic / strips in us (four: the generic kernel reads float4s):
-//   four, angles in pairs 180 degrees apart (one strip sums both): 54^2 x 90 angles 10.9 / 12.3 with 16 slices, 20.0 /
-//     13.6 with 20; 96^2 x 90 27.1 / 22.0 with 12
-//   four, no pairs: 96^2 x 91 23.7 / 30.4 with 16 slices, 43.4 / 36.3 with 20
-//   four, per-ray absorption (no pairs, and a factor per weight): 256^2 x 360 454 / 894 with 16 slices, 854 / 971 with
-//     32, 1665 / 1142 with 56
-//   single slices, pairs: 54^2 x 90 15.4 / 14.4 with 5 slices, 96^2 x 90 30.7 / 25.8; no pairs: 96^2 x 91 31.2 / 38.7
-//     with 5, 44.7 / 39.0 with 9; per-ray absorption: 96^2 x 90 49.6 / 62.7 with 11, 67.9 / 64.8 with 15
+//   four, angles in pairs 180 degrees apart (one strip sums both): 54^2 x 90 angles 11.8 / 13.6 with 16 slices, 21.1 /
+//     14.6 with 20; 96^2 x 90 28.5 / 23.1 with 12
+//   four, no pairs: 96^2 x 91 25.2 / 33.3 with 16 slices, 45.0 / 39.1 with 20
+//   four, per-ray absorption (no pairs, and a factor per weight): 160^2 x 180 102 / 204 with 16 slices, 187 / 225 with
+//     32, 357 / 270 with 56
+//   single slices, pairs: 64^2 x 90 19.3 / 16.7 with 5 slices, 96^2 x 90 32.3 / 27.0; no pairs: 96^2 x 91 32.9 / 39.2
+//     with 5, 46.3 / 40.5 with 9; per-ray absorption: 96^2 x 90 51.7 / 65.6 with 11, 69.2 / 69.0 with 15
 // Few strips (bins times pairs of angles: w) leave each waiting for its rows while the generic kernel spreads a bin over
-// a warp: 32^2 x 90 (w 1440) 8.9 / 10.7 with 32 slices, 13.0 / 11.6 with 36; 64^2 x 30 (w 960) 14.1 / 17.8 with 36, single
-// slices 23.3 / 22.4 with 33; 96^2 x 8 (w 384) 45 single slices 16 / 22, 117 slices 27 / 24.  From 58 slices in float4 rows
-// on they are the faster ones at any w.
+// a warp: 32^2 x 90 (w 1440) 9.8 / 12.1 with 32 slices, 14.2 / 13.2 with 36; per-ray absorption, 40^2 x 24 (w 960) 14.2 /
+// 22.8 with 100; single slices, 64^2 x 24 (w 768) 16.9 / 20.4 with 26, 26.5 / 20.8 with 30; small slices (below 48 pixels)
+// a little longer, 24^2 x 180 (w 2160) 8.8 / 10.8 with 28.
 int strips_from(const vam_parallel_plan& p, bool four) {
     const bool ray = p.abs_mode == VAM_ABS_RAY, pairs = !ray && 4LL * p.n_tasks_paired <= 3LL * p.nA;
     const long long w = (long long)p.nX * (ray ? p.nA : p.n_tasks_paired);
     if (issue_bound(p)) return four ? 9 : 5;
-    if (four && ray) return w < 4000 ? 58 : 56;
-    if (four) return w < 1400 ? 58 : w < 2000 ? 36 : pairs && p.nX >= 96 && w >= 2900 ? 12 : 20;
-    if (ray) return w < 800 ? 129 : w < 1800 ? 100 : w < 2800 ? 45 : w < 4000 ? 20 : 15;
-    return w < 350 ? 129 : w < 800 ? 80 : w < 1400 ? 33 : w < 2000 ? 18 : pairs ? 5 : 9;
+    const bool small = p.nX < 48;
+    if (four && ray) return w < 1500 ? 129 : w < 3000 ? 100 : w < 4000 ? 80 : 56;
+    if (four) {
+        if (w < 1400) return w < 760 ? 129 : 56;
+        if (w < 2000 || (small && w < 2600) || (!pairs && w < 4400)) return 36;
+        return pairs && p.nX >= 96 && w >= 2900 ? 12 : 20;
+    }
+    if (ray) return w < 1100 ? 129 : w < 1500 ? 90 : w < 2000 ? 50 : w < 2900 ? 33 : w < 4300 ? 24 : small ? 18 : 15;
+    if (w < 1400) return w < 550 ? 129 : w < 700 ? 90 : w < 900 ? 50 : 30;
+    if (w < 2000) return pairs ? 18 : 26;
+    if (w < 2600 && (small || !pairs)) return 13;
+    return pairs && !small && w >= 2800 ? 5 : 9;
 }
 
 // The same for the transpose's blocks, whose generic kernel evaluates all samples near a pixel: faster only for the
@@ -2037,8 +2045,9 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
     // -> 0.36 ms against the generic kernel, which evaluates every sample's coordinates in float64 for one slice per
     // lane.
     // Sums: the lanes among which the generic kernel shares a bin's samples or a pixel's angles, and the groups among
-    // which a strip or block does (four slices per lane).  Where it has more lanes, and no kernel but it served the call
-    // before the strips and blocks, their sums are the exact ones (strip.cuh), so that no slice count is less exact.
+    // which a strip or block does (four slices per lane).  Where it has more lanes (or, of the forward, several, or the
+    // strip several groups), and no kernel but it served the call before the strips and blocks, their sums are the exact
+    // ones (strip.cuh), so that no slice count is less exact.
     const int lanes = 32 / choose_layout(plan->nZ, aligned16).LZ;
     const int groups = plan->nZ <= 16 ? 8 : plan->nZ <= 32 ? 4 : plan->nZ <= 64 ? 2 : 1;
     const bool four = aligned16 && plan->nZ % 4 == 0;  // (what the generic kernel would read: float4s or single slices)
@@ -2058,9 +2067,11 @@ int describe(vam_parallel_plan* plan, Op op, const float* in, float* out, Item& 
         it.kind = KF_FAST; it.ray = ray;
         it.vec = rows4 && (padded || aligned16);
         it.vz = want == 4 || (want != 8 && plan->nZ <= 128) ? 4 : 8;
-        // (a strip's batches are sums of their own already: as exact as two lanes per bin.  From 58 slices in float4
-        // rows the less exact k_forward_fast served before.)
-        it.exact = it.vz == 4 && lanes >= std::max(4, 2 * groups) && !(aligned16 && fast_vz(plan->nZ, true, 0.45));
+        // From 58 slices in float4 rows the less exact k_forward_fast served before.  From 65 single slices on a strip is
+        // one group with more exact sums than the generic kernel's one lane per bin, except on volumes of zeros and ones,
+        // whose samples the latter adds without rounding (201^2 x 117 x 240: 9.8e-8 against 2.2e-7; of zeros and ones
+        // 6.5e-8 against 4.4e-8).
+        it.exact = it.vz == 4 && (lanes >= 2 || groups >= 2) && !(aligned16 && fast_vz(plan->nZ, true, 0.45));
         a.lz_shift = 5;
         if (it.vz == 4)  // lanes to spare take other pixels
             while (a.lz_shift > 2 && (4 << (a.lz_shift - 1)) >= plan->nZ) --a.lz_shift;

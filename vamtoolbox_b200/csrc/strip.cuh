@@ -109,6 +109,31 @@ __device__ __forceinline__ unsigned long long dropped(unsigned long long s, unsi
     return d;
 }
 
+__device__ __forceinline__ unsigned long long add_pairs(unsigned long long s, unsigned long long x) {
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s) : "l"(x));
+    return s;
+}
+
+// s + x into s; what the rounding drops, whichever is larger
+__device__ __forceinline__ unsigned long long two_sum(unsigned long long& s, unsigned long long x) {
+    const unsigned long long t = add_pairs(s, x);
+    unsigned long long d, e;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(t), "l"(s));
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(e) : "l"(t), "l"(d));
+    asm("sub.rn.f32x2 %0, %1, %0;" : "+l"(e) : "l"(s));
+    asm("sub.rn.f32x2 %0, %1, %0;" : "+l"(d) : "l"(x));
+    s = t;
+    return add_pairs(e, d);
+}
+
+// s + x, but s where that is no number (s infinite: what its rounding dropped is none)
+__device__ __forceinline__ unsigned long long add_finite(unsigned long long s, unsigned long long x) {
+    float s0, s1, t0, t1;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(s));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(add_pairs(s, x)));
+    return pk_pair(t0 == t0 ? t0 : s0, t1 == t1 ? t1 : s1);
+}
+
 // whole: the float4s may be stored as such; otherwise (padded rows) slice by slice, the first `left` of them
 // (those the output has: a padded row holds up to three more)
 template <int Q, bool VEC>
@@ -220,9 +245,11 @@ __device__ __forceinline__ bool strip_place(const FastArgs& a, unsigned bx, unsi
 
 // (param: the arguments where the launch left them, for the call at the end; a copy's address would keep it in memory)
 //
-// EXACT: the running sum of the batches keeps what its rounding drops.  For slice counts that the generic kernel gives
-// more lanes per bin than the strips do (Sums in describe()): its lanes' partial sums are otherwise the more exact ones
-// (64^2 x 40 x 90 angles, relative to float64: generic 4.3e-8, strips 5.9e-8, so 4.4e-8; 17.4 -> 18.6 us).
+// EXACT: the running sum takes up the current one after every group of pixels and keeps what its rounding drops, to
+// the end.  For slice counts that the generic kernel gives more lanes per bin, or of which the strips have several
+// groups (Sums in describe()): its lanes' partial sums are otherwise the more exact ones, the more so for volumes of
+// zeros and ones, whose samples it adds without rounding (64^2 x 40 x 90 angles, relative to float64: generic 4.3e-8,
+// 3.2e-8 for zeros and ones; strips 5.9e-8 and 4.4e-8, so 3.1e-8 and 2.7e-8; 17.3 -> 18.1 us, generic 32).
 template <int Q, bool VEC, bool RAY, bool EXACT = false>
 __device__ __forceinline__ void forward_strip_body(const FastArgs& a, const FastArgs& param, unsigned bx, unsigned by) {
     constexpr int M = strip_bins(Q), U = Q == 2 ? 3 : 4, VZ = 4 * Q;
@@ -417,17 +444,21 @@ __device__ __forceinline__ void forward_strip_body(const FastArgs& a, const Fast
             __syncwarp();
             for (; wait >= round; wait -= round) {
                 step(first + head, t1, v1, t0, v0);
+                if (EXACT) carry();
                 step(first + head + U * G, t0, v0, t1, v1);
+                if (EXACT) carry();
                 head = head + round < size ? head + round : 0;
             }
-            carry();
+            if (!EXACT) carry();
             __syncwarp();  // the entries worked off are free again
         }
         if (wait > 0) {  // the rest, filled up with entries of no weight (and the first pixel's row)
             for (int k = wait + lane; k < round; k += 32) ring.e[wp][head + k] = make_float4(0.f, 0.f, 0.f, 0.f);
             __syncwarp();
             step(first + head, t1, v1, t0, v0);
+            if (EXACT) carry();
             step(first + head + U * G, t0, v0, t1, v1);
+            if (EXACT) carry();
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) add1(t0[u], v0[u]);
@@ -457,8 +488,18 @@ __device__ __forceinline__ void forward_strip_body(const FastArgs& a, const Fast
 #pragma unroll
                 for (int e = 0; e < VZ / 2; ++e) {
                     const unsigned long long t = __shfl_xor_sync(kFull, sum[m][e], off);
-                    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[m][e]) : "l"(t));
+                    if constexpr (EXACT) {
+                        acc[m][e] = add_pairs(acc[m][e], __shfl_xor_sync(kFull, acc[m][e], off));
+                        acc[m][e] = add_pairs(acc[m][e], two_sum(sum[m][e], t));
+                    } else {
+                        sum[m][e] = add_pairs(sum[m][e], t);
+                    }
                 }
+    if constexpr (EXACT)
+#pragma unroll
+        for (int m = 0; m < M; ++m)
+#pragma unroll
+            for (int e = 0; e < VZ / 2; ++e) sum[m][e] = add_finite(sum[m][e], acc[m][e]);
     if (n == 0 || g != 0) return;
 #pragma unroll
     for (int m = 0; m < M; ++m)
