@@ -1433,8 +1433,10 @@ __device__ __forceinline__ void k_backward_2d_body(const TileArgs& a, unsigned b
     else backward_2d_body(a, bx);
 }
 
+// per-ray absorption at four blocks an SM: without spills, and a fifth resident block only moves the sizes whose tiles fit
+// one wave badly (400^2 x 140 angles 99 us with five, 83 with four; 450^2 x 300 212 and 247; 512^2 x 720 663 and 671)
 template <bool RAY, bool F64>
-__global__ void __launch_bounds__(256) k_backward_2d(TileArgs a) {
+__global__ void __launch_bounds__(256, RAY && F64 ? 4 : 0) k_backward_2d(TileArgs a) {
     k_backward_2d_body<RAY, F64>(a, blockIdx.x);
 }
 
