@@ -1874,17 +1874,17 @@ int strips_from(const vam_parallel_plan& p, bool four) {
     const long long w = (long long)p.nX * (ray ? p.nA : p.n_tasks_paired);
     if (issue_bound(p)) return four ? 9 : 5;
     const bool small = p.nX < 48;
-    if (four && ray) return w < 1500 ? 129 : w < 3000 ? 100 : w < 4000 ? 80 : 56;
+    if (four && ray) return w < 1500 ? 120 : w < 2800 ? 100 : w < 4000 ? 58 : 56;
     if (four) {
-        if (w < 1400) return w < 760 ? 129 : 56;
+        if (w < 1400) return w < 760 ? 120 : 56;
         if (w < 2000 || (small && w < 2600) || (!pairs && w < 4400)) return 36;
         return pairs && p.nX >= 96 && w >= 2900 ? 12 : 20;
     }
     if (ray) return w < 1100 ? 129 : w < 1500 ? 90 : w < 2000 ? 50 : w < 2900 ? 33 : w < 4300 ? 24 : small ? 18 : 15;
-    if (w < 1400) return w < 550 ? 129 : w < 700 ? 90 : w < 900 ? 50 : 30;
+    if (w < 1400) return w < 550 ? (small ? 129 : 110) : w < 700 ? 90 : w < 900 ? 50 : 30;
     if (w < 2000) return pairs ? 18 : 26;
     if (w < 2600 && (small || !pairs)) return 13;
-    return pairs && !small && w >= 2800 ? 5 : 9;
+    return pairs && !small && w >= 2400 ? 5 : 9;
 }
 
 // The same for the transpose's blocks, whose generic kernel evaluates all samples near a pixel: faster only for the
